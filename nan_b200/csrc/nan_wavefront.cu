@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_extend(Src src, const uint32_t* 
                 tally.extend++;
                 HitInfo h;
                 if constexpr (kShared > 0 && kWidth == 2) {
-                    SplitStack<kShared, 128, kTraversalStack> stk;
+                    SplitStack<kShared, 128, kTraversalStack + 1> stk;
                     stk.top = stack_top + threadIdx.x;
                     h = trace_closest_binary_s<kTraversalStack>(s, stk, xyz(o), xyz(d), o.w, d.w);
                 } else if constexpr (kSpec && kWidth == 2) {
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_shadow(Src src, const float4* __
             const SceneView s = src.of(p);
             bool blocked;
             if constexpr (kShared > 0 && kWidth == 2) {
-                SplitStack<kShared, 128, kTraversalStack> stk;
+                SplitStack<kShared, 128, kTraversalStack + 1> stk;
                 stk.top = stack_top + threadIdx.x;
                 blocked = trace_any_binary_s<kTraversalStack>(s, stk, xyz(a), xyz(b), 0.0f, c.w > 0.0f ? c.w : t_max);
             } else if constexpr (kSpec && kWidth == 2) {
