@@ -273,6 +273,33 @@ __device__ __forceinline__ void add_sah(double* sah, double cost) {
     if ((threadIdx.x & 31u) == 0u && cost != 0.0) atomicAdd(sah, cost);
 }
 
+// Outward padding of the binary node boxes: 1.5 x 2^-18 of the scene's
+// largest coordinate M. The slab test (box2 in nan_scene.cuh) rounds
+// distances that reach |o| + M along an axis at most four times, 4 x 2^-24 of
+// them, so it never culls a box the exact ray crosses while the ray's origin
+// lies within about 20 M.
+__device__ __forceinline__ float node_pad(const Bounds* bounds) {
+    return ordered_to_float(bounds->max_abs) * 5.7220458984375e-6f + 1e-30f;
+}
+
+// Padded interval [lo - pad, hi + pad] as (centre, half extent), the half
+// extent rounded up so that the centre's rounding never shrinks the interval.
+__device__ __forceinline__ float2 centre_half(float lo, float hi, float pad) {
+    const float l = lo - pad, h = hi + pad;
+    const float c = 0.5f * l + 0.5f * h;
+    return make_float2(c, fmaxf(__fsub_ru(h, c), __fsub_ru(c, l)));
+}
+
+// The three box words of a binary node (layout: SceneView, nan_scene.cuh).
+__device__ __forceinline__ void store_node_boxes(float4* node, float4 al, float4 ah, float4 bl, float4 bh, float pad) {
+    const float2 ax = centre_half(al.x, ah.x, pad), bx = centre_half(bl.x, bh.x, pad);
+    const float2 ay = centre_half(al.y, ah.y, pad), by = centre_half(bl.y, bh.y, pad);
+    const float2 az = centre_half(al.z, ah.z, pad), bz = centre_half(bl.z, bh.z, pad);
+    node[0] = make_float4(ax.x, bx.x, ay.x, by.x);
+    node[1] = make_float4(az.x, bz.x, ax.y, bx.y);
+    node[2] = make_float4(ay.y, by.y, az.y, bz.y);
+}
+
 __global__ void k_emit(uint32_t interior, const int2* __restrict__ children, const float4* __restrict__ node_lo,
                        const float4* __restrict__ node_hi, const float4* __restrict__ leaf_lo,
                        const float4* __restrict__ leaf_hi, const Bounds* __restrict__ bounds,
@@ -280,14 +307,12 @@ __global__ void k_emit(uint32_t interior, const int2* __restrict__ children, con
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     double cost = 0.0;
     if (i < interior) {
-        const float pad = ordered_to_float(bounds->max_abs) * 3.814697265625e-6f + 1e-30f;  // 2^-18 relative
+        const float pad = node_pad(bounds);
         const int2 ch = children[i];
         float4 al, ah, bl, bh;
         child_box(ch.x, node_lo, node_hi, leaf_lo, leaf_hi, &al, &ah);
         child_box(ch.y, node_lo, node_hi, leaf_lo, leaf_hi, &bl, &bh);
-        nodes[4u * i + 0] = make_float4(al.x - pad, ah.x + pad, al.y - pad, ah.y + pad);
-        nodes[4u * i + 1] = make_float4(bl.x - pad, bh.x + pad, bl.y - pad, bh.y + pad);
-        nodes[4u * i + 2] = make_float4(al.z - pad, ah.z + pad, bl.z - pad, bh.z + pad);
+        store_node_boxes(nodes + 4u * i, al, ah, bl, bh, pad);
         // leaves (single triangles in LBVH) as ~(first << 3 | count - 1)
         const int rx = ch.x < 0 ? ~((~ch.x) << 3) : ch.x;
         const int ry = ch.y < 0 ? ~((~ch.y) << 3) : ch.y;
@@ -572,14 +597,12 @@ __global__ void k_emit_dfs(uint32_t interior, const int2* __restrict__ children,
     const int slot = x < interior ? dfs[x] : -1;
     double cost = 0.0;
     if (slot >= 0 && !info[x].collapsed) {
-        const float pad = ordered_to_float(bounds->max_abs) * 3.814697265625e-6f + 1e-30f;
+        const float pad = node_pad(bounds);
         const int2 ch = children[x];
         float4 al, ah, bl, bh;
         child_box(ch.x, node_lo, node_hi, leaf_lo, leaf_hi, &al, &ah);
         child_box(ch.y, node_lo, node_hi, leaf_lo, leaf_hi, &bl, &bh);
-        nodes[4u * slot + 0] = make_float4(al.x - pad, ah.x + pad, al.y - pad, ah.y + pad);
-        nodes[4u * slot + 1] = make_float4(bl.x - pad, bh.x + pad, bl.y - pad, bh.y + pad);
-        nodes[4u * slot + 2] = make_float4(al.z - pad, ah.z + pad, bl.z - pad, bh.z + pad);
+        store_node_boxes(nodes + 4u * slot, al, ah, bl, bh, pad);
         const int ra = child_ref(ch.x, dfs, tri_off, tri_pos, info);
         const int rb = child_ref(ch.y, dfs, tri_off, tri_pos, info);
         nodes[4u * slot + 3] = make_float4(__int_as_float(ra), __int_as_float(rb), 0.0f, 0.0f);

@@ -13,10 +13,10 @@ constexpr int kTraversalStack = 96;
 constexpr uint32_t kStatusStackOverflow = 1u;
 
 // Binary BVH node, 64 bytes: both children's boxes live in the parent so one
-// node fetch tests two boxes.
-//   a = (c0.lo.x, c0.hi.x, c0.lo.y, c0.hi.y)
-//   b = (c1.lo.x, c1.hi.x, c1.lo.y, c1.hi.y)
-//   c = (c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z)
+// node fetch tests two boxes, as centres c and half extents h.
+//   a = (c0.c.x, c1.c.x, c0.c.y, c1.c.y)
+//   b = (c0.c.z, c1.c.z, c0.h.x, c1.h.x)
+//   c = (c0.h.y, c1.h.y, c0.h.z, c1.h.z)
 //   d = (child0, child1, -, -): child >= 0 is an interior node; child < 0 a
 //       leaf of triangles [first, first + count) in leaf order, encoded as
 //       ~(first << 3 | (count - 1)) (1..8 triangles).
@@ -133,7 +133,13 @@ __device__ __forceinline__ void load_tri(const SceneView& s, int i, f3* v0, f3* 
 
 // Slab test of both children of a node. Node boxes are padded outward at
 // build time by more than the rounding of the fused slab arithmetic, so the
-// test never rejects a box the exact ray crosses.
+// test never rejects a box the exact ray crosses. A box as centre and half
+// extent gives the near and far distance of an axis as (c - o) / d -+
+// h / |d|: three FMAs, where two planes take two FMAs and a min and a max to
+// sort them. The FMAs run for both children at once (f32x2), and min and max,
+// which issue at half the FMA rate, drop from 20 to 8 a node. With 9 blocks a
+// SM: 200k-triangle texel iteration 20.8 -> 20.2 ms (scalar FMAs 20.3), probe
+// batch 15.6 -> 14.6 ms (14.8), 33.5 M visibility rays 6.37 -> 5.56 ms (5.84).
 struct BoxRay {
     float ix, iy, iz, ox, oy, oz;
 };
@@ -163,18 +169,31 @@ __device__ __forceinline__ float max3f(float a, float b, float c) {
     return d;
 }
 
+// Two FMAs in one instruction (PTX fma.rn.f32x2, sm_100 and later), each
+// rounded as __fmaf_rn rounds.
+__device__ __forceinline__ float2 fma2(float2 a, float2 m, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, m, c, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 m, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+        "fma.rn.f32x2 d, a, m, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(m.x), "f"(m.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
+
 __device__ __forceinline__ void box2(const BoxRay& r, float4 na, float4 nb, float4 nc, float tmin, float tmax,
                                      float* t0, float* t1, bool* h0, bool* h1) {
-    const float x0a = __fmaf_rn(na.x, r.ix, -r.ox), x0b = __fmaf_rn(na.y, r.ix, -r.ox);
-    const float y0a = __fmaf_rn(na.z, r.iy, -r.oy), y0b = __fmaf_rn(na.w, r.iy, -r.oy);
-    const float z0a = __fmaf_rn(nc.x, r.iz, -r.oz), z0b = __fmaf_rn(nc.y, r.iz, -r.oz);
-    const float x1a = __fmaf_rn(nb.x, r.ix, -r.ox), x1b = __fmaf_rn(nb.y, r.ix, -r.ox);
-    const float y1a = __fmaf_rn(nb.z, r.iy, -r.oy), y1b = __fmaf_rn(nb.w, r.iy, -r.oy);
-    const float z1a = __fmaf_rn(nc.z, r.iz, -r.oz), z1b = __fmaf_rn(nc.w, r.iz, -r.oz);
-    const float lo0 = max3f(fminf(x0a, x0b), fminf(y0a, y0b), fmaxf(fminf(z0a, z0b), tmin));
-    const float hi0 = min3f(fmaxf(x0a, x0b), fmaxf(y0a, y0b), fminf(fmaxf(z0a, z0b), tmax));
-    const float lo1 = max3f(fminf(x1a, x1b), fminf(y1a, y1b), fmaxf(fminf(z1a, z1b), tmin));
-    const float hi1 = min3f(fmaxf(x1a, x1b), fmaxf(y1a, y1b), fminf(fmaxf(z1a, z1b), tmax));
+    const float2 ax = dup(fabsf(r.ix)), ay = dup(fabsf(r.iy)), az = dup(fabsf(r.iz));
+    const float2 mx = dup(-fabsf(r.ix)), my = dup(-fabsf(r.iy)), mz = dup(-fabsf(r.iz));
+    const float2 x = fma2(make_float2(na.x, na.y), dup(r.ix), dup(-r.ox));
+    const float2 y = fma2(make_float2(na.z, na.w), dup(r.iy), dup(-r.oy));
+    const float2 z = fma2(make_float2(nb.x, nb.y), dup(r.iz), dup(-r.oz));
+    const float2 hx = make_float2(nb.z, nb.w), hy = make_float2(nc.x, nc.y), hz = make_float2(nc.z, nc.w);
+    const float2 xl = fma2(hx, mx, x), yl = fma2(hy, my, y), zl = fma2(hz, mz, z);
+    const float2 xh = fma2(hx, ax, x), yh = fma2(hy, ay, y), zh = fma2(hz, az, z);
+    const float lo0 = max3f(xl.x, yl.x, fmaxf(zl.x, tmin)), hi0 = min3f(xh.x, yh.x, fminf(zh.x, tmax));
+    const float lo1 = max3f(xl.y, yl.y, fmaxf(zl.y, tmin)), hi1 = min3f(xh.y, yh.y, fminf(zh.y, tmax));
     *t0 = lo0;
     *t1 = lo1;
     *h0 = lo0 <= hi0;

@@ -152,10 +152,10 @@ template <int kWidth, class Src, int kShared = 0, bool kSpec = false>
 // kShared > 0 (binary nodes): the first kShared traversal-stack entries of a
 // thread live in a shared-memory column, the rest in local memory. kSpec
 // (binary nodes): the speculative while-while walk.
-// 10 resident blocks of 128 per SM (48 registers a thread, -Xptxas -v): measured
-// 1,941 against 1,895 Mrays/s with the register count left free (9 blocks),
-// 1,916 at 11 and 12 blocks, 1,639 at 16 (spills).
-__global__ void __launch_bounds__(128, 10) k_wf_extend(Src src, const uint32_t* __restrict__ queue,
+// 9 resident blocks of 128 per SM (56 registers a thread): the 200k-triangle
+// texel iteration takes 20.2 ms, against 20.6 with 8 blocks and 20.7 with 10
+// (48 registers, spills); the 16-scene probe batch 14.6, 14.9 and 15.9 ms.
+__global__ void __launch_bounds__(128, 9) k_wf_extend(Src src, const uint32_t* __restrict__ queue,
                                                    uint32_t* ctl, const float4* __restrict__ ro,
                                                    const float4* __restrict__ rd, const uint32_t* __restrict__ flags,
                                                    float4* __restrict__ hit, unsigned long long* counters) {
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_extend(Src src, const uint32_t* 
 }
 
 template <int kWidth, class Src, int kShared = 0, bool kSpec = false>
-__global__ void __launch_bounds__(128, 10) k_wf_shadow(Src src, const float4* __restrict__ queue, uint32_t* ctl,
+__global__ void __launch_bounds__(128, 9) k_wf_shadow(Src src, const float4* __restrict__ queue, uint32_t* ctl,
                                                    float t_max, float4* __restrict__ rad, float4* __restrict__ si,
                                                    unsigned long long* counters) {
     const uint32_t count = *(volatile uint32_t*)(ctl + 2);
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_shadow(Src src, const float4* __
 // between two refill checks. Without refill, a warp that took 32 rays runs
 // until the slowest of them ends.
 template <int kRefill, int kBurst, class Src>
-__global__ void __launch_bounds__(128, 10) k_wf_extend_refill(Src src, const uint32_t* __restrict__ queue,
+__global__ void __launch_bounds__(128, 9) k_wf_extend_refill(Src src, const uint32_t* __restrict__ queue,
                                                           uint32_t* ctl, const float4* __restrict__ ro,
                                                           const float4* __restrict__ rd,
                                                           const uint32_t* __restrict__ flags,
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_extend_refill(Src src, const uin
 }
 
 template <int kRefill, int kBurst, class Src>
-__global__ void __launch_bounds__(128, 10) k_wf_shadow_refill(Src src, const float4* __restrict__ queue, uint32_t* ctl,
+__global__ void __launch_bounds__(128, 9) k_wf_shadow_refill(Src src, const float4* __restrict__ queue, uint32_t* ctl,
                                                           float t_max, float4* __restrict__ rad,
                                                           float4* __restrict__ si, unsigned long long* counters) {
     const uint32_t count = *(volatile uint32_t*)(ctl + 2);
