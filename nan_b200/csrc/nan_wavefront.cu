@@ -1,13 +1,18 @@
 // nan_wavefront.cu -- wavefront form of the integrators.
 //
-// A path lives in SoA state arrays between kernels. Each iteration runs:
-//   extend   persistent warps pull path ids from a compacted queue and trace
-//            the closest hit of each path's ray (all lanes do traversal);
-//   shade    per path: emission, sun NEE shadow ray (queued), next direction;
-//   shadow   persistent warps trace the queued any-hit rays and add the
-//            contributions of the visible ones;
-//   finalize per path: continue, or close the sample (and start the next
-//            sample, the back side, or retire the path).
+// A path lives in SoA state arrays between kernels. Each round runs:
+//   trace  persistent warps pull rays from two compacted queues: the closest
+//          hit of every walking path's ray, and any hit of the shadow rays
+//          that the last round's stage queued, adding the contributions of
+//          the visible ones;
+//   stage  per path: emission, sun NEE shadow ray (queued), next direction;
+//          a path that ended one round ago, or left the scene now, is closed
+//          (and starts the next sample or side, or retires).
+// A path that ends at a surface has its last shadow ray in flight while the
+// others trace on, and is closed a round later. Shadow and closest-hit rays
+// of neighbouring vertices thus share one launch: two launches and one wait
+// for the longest ray per round, where a launch each for extend, shade,
+// shadow and finalize took four and two.
 // The RNG of a path is the reference's per-thread stream, drawn in the same
 // order, and every radiance sum is formed in the same order as the
 // reference's loop, so the result equals the one-thread-per-unit kernels bit
@@ -27,7 +32,6 @@ using nan_host::cuda_fail;
 using nan_host::set_error;
 
 constexpr uint32_t kFlagBack = 1u << 0;
-constexpr uint32_t kFlagEnd = 1u << 1;
 constexpr uint32_t kFlagNoPath = 1u << 2;
 constexpr uint32_t kFlagTwoSided = 1u << 3;
 constexpr uint32_t kBounceShift = 4;
@@ -55,13 +59,22 @@ struct WfState {
     uint4* pc;        // probes: 2 per path, per-radial-texel sample counts (16 x u16)
 };
 
+// Queues of one chunk of paths. The paths that trace on fill a round's extend
+// queue from the front, those that wait to be closed from the back: each path
+// in flight is in it at most once.
 struct WfQueues {
     uint32_t* ext[2];
     uint32_t* ext_sorted;  // the extend queue regrouped by direction octant (NanTuning ray_order 1)
     float4* shd[2];        // 3 float4 per entry: (o, path bits), (d, kind bits), (c, 0)
-    uint32_t* ctl;         // per iteration k: [4k] ext count, [4k+1] ext fetch, [4k+2] shd count, [4k+3] shd fetch
-    uint32_t* oct;         // per iteration k: [16k..16k+7] paths per octant, [16k+8..16k+15] placement cursors
+    uint32_t* ctl;         // kCtlWords per round: kExt, kExtFetch, kShd, kShdFetch, kClose
+    uint32_t* oct;         // 8 paths per octant, 8 placement cursors
+    uint32_t cap;          // paths in flight: the length of an extend queue
 };
+
+// Words of a round's control block: walking paths, fetch counter of the trace
+// (or extend) launch, shadow rays queued by the round's stage, fetch counter
+// of a separate shadow launch, paths to close.
+constexpr uint32_t kCtlWords = 8u, kExt = 0u, kExtFetch = 1u, kShd = 2u, kShdFetch = 3u, kClose = 4u;
 
 constexpr size_t kBytesPerPath = 4 + 4 + 4 + 16 * 9 + 8 + 16 + 16 + 32 + 3 * 4 + 2 * 2 * 48;
 
@@ -77,10 +90,20 @@ __device__ __forceinline__ uint32_t queue_slot(uint32_t* count, bool want) {
     return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
 }
 
+// Into the queue of the round that ctl belongs to: a path that traces on, or
+// one that waits to be closed.
+__device__ __forceinline__ void push_path(const WfQueues& q, int buf, uint32_t* ctl, uint32_t p) {
+    q.ext[buf][queue_slot(ctl + kExt, true)] = p;
+}
+
+__device__ __forceinline__ void push_close(const WfQueues& q, int buf, uint32_t* ctl, uint32_t p) {
+    q.ext[buf][q.cap - 1u - queue_slot(ctl + kClose, true)] = p;
+}
+
 // tmax 0: the ray runs to the scene's t_max
-__device__ __forceinline__ void push_shadow(const WfQueues& q, int buf, uint32_t* count, uint32_t p, f3 o, f3 d,
+__device__ __forceinline__ void push_shadow(const WfQueues& q, int buf, uint32_t* ctl, uint32_t p, f3 o, f3 d,
                                             f3 c, uint32_t kind, float tmax = 0.0f) {
-    const uint32_t slot = queue_slot(count, true);
+    const uint32_t slot = queue_slot(ctl + kShd, true);
     float4* e = q.shd[buf] + 3u * slot;
     e[0] = make_float4(o.x, o.y, o.z, __uint_as_float(p));
     e[1] = make_float4(d.x, d.y, d.z, __uint_as_float(kind));
@@ -103,7 +126,7 @@ __device__ __forceinline__ uint32_t dir_octant(float4 d) {
 
 __global__ void __launch_bounds__(256) k_wf_octant_count(const uint32_t* __restrict__ queue, const uint32_t* ctl,
                                                          const float4* __restrict__ rd, uint32_t* oct) {
-    const uint32_t count = *(volatile const uint32_t*)(ctl + 0);
+    const uint32_t count = *(volatile const uint32_t*)(ctl + kExt);
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
         const uint32_t o = dir_octant(rd[queue[idx]]);
         const unsigned group = __match_any_sync(__activemask(), o);
@@ -114,7 +137,7 @@ __global__ void __launch_bounds__(256) k_wf_octant_count(const uint32_t* __restr
 __global__ void __launch_bounds__(256) k_wf_octant_place(const uint32_t* __restrict__ queue, const uint32_t* ctl,
                                                          const float4* __restrict__ rd, uint32_t* oct,
                                                          uint32_t* __restrict__ out) {
-    const uint32_t count = *(volatile const uint32_t*)(ctl + 0);
+    const uint32_t count = *(volatile const uint32_t*)(ctl + kExt);
     uint32_t base[8];
     uint32_t sum = 0u;
     for (int o = 0; o < 8; ++o) {
@@ -135,6 +158,14 @@ __global__ void __launch_bounds__(256) k_wf_octant_place(const uint32_t* __restr
     }
 }
 
+// The paths to close of a regrouped queue, at its back as before.
+__global__ void __launch_bounds__(256) k_wf_close_copy(const uint32_t* __restrict__ queue, const uint32_t* ctl,
+                                                       uint32_t cap, uint32_t* __restrict__ out) {
+    const uint32_t count = *(volatile const uint32_t*)(ctl + kClose);
+    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x)
+        out[cap - 1u - idx] = queue[cap - 1u - idx];
+}
+
 // Scene of a path: one scene for the per-scene passes, the path's probe set
 // for the multi-scene batch (set index per path).
 struct OneScene {
@@ -149,16 +180,14 @@ struct ManyScenes {
 };
 
 // Rays a warp takes from a queue at once: 32, or fewer where the queue would
-// leave most of the grid's warps without any: then the even share over half
-// of them. Few rays a warp end sooner (a warp runs as long as its longest
-// ray, and diverging lanes take turns), and idle warps cost nothing: probe
-// baker over 20,480 sites 9.1 -> 6.1 ms. An even share over all warps gives
-// 5.8 ms there, but 65,536 screen rays in the 36-triangle box then cost more
-// in warps than they gain (293 against 265 us a frame, 302 before). Warps take
+// leave warps of the grid without any: then the even share. Few rays a warp
+// end sooner: a warp runs as long as its longest ray, and its diverging lanes
+// take turns (probe baker over 20,480 sites: 9.1 ms with 32 rays a warp, 5.8
+// with the even share, extend and shadow in launches of their own). Warps take
 // their first rays by their number, without an atomic.
-__device__ __forceinline__ uint32_t rays_per_grab(uint32_t count) {
+__device__ __forceinline__ uint32_t rays_per_grab(unsigned long long count) {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    return (uint32_t)min((unsigned long long)32u, max(1ull, (2ull * count + warps - 1u) / warps));
+    return (uint32_t)min(32ull, max(1ull, (count + warps - 1u) / warps));
 }
 
 template <int kWidth, class Src, int kShared = 0, bool kSpec = false>
@@ -170,9 +199,9 @@ template <int kWidth, class Src, int kShared = 0, bool kSpec = false>
 // (48 registers, spills); the 16-scene probe batch 14.6, 14.9 and 15.9 ms.
 __global__ void __launch_bounds__(128, 9) k_wf_extend(Src src, const uint32_t* __restrict__ queue,
                                                    uint32_t* ctl, const float4* __restrict__ ro,
-                                                   const float4* __restrict__ rd, const uint32_t* __restrict__ flags,
-                                                   float4* __restrict__ hit, unsigned long long* counters) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
+                                                   const float4* __restrict__ rd, float4* __restrict__ hit,
+                                                   unsigned long long* counters) {
+    const uint32_t count = *(volatile uint32_t*)(ctl + kExt);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t grab = rays_per_grab(count);
     RayTally tally{0u, 0u};
@@ -182,27 +211,23 @@ __global__ void __launch_bounds__(128, 9) k_wf_extend(Src src, const uint32_t* _
         const uint32_t idx = base + lane;
         if (lane < grab && idx < count) {
             const uint32_t p = queue[idx];
-            if (flags[p] & kFlagNoPath) {
-                hit[p] = make_float4(__uint_as_float(0xffffffffu), 0.0f, 0.0f, 0.0f);
+            const SceneView s = src.of(p);
+            const float4 o = ro[p], d = rd[p];
+            tally.extend++;
+            HitInfo h;
+            if constexpr (kShared > 0 && kWidth == 2) {
+                SplitStack<kShared, 128, kTraversalStack + 1> stk;
+                stk.top = stack_top + threadIdx.x;
+                h = trace_closest_binary_s<kTraversalStack>(s, stk, xyz(o), xyz(d), o.w, d.w);
+            } else if constexpr (kSpec && kWidth == 2) {
+                h = trace_closest_binary_spec(s, xyz(o), xyz(d), o.w, d.w);
             } else {
-                const SceneView s = src.of(p);
-                const float4 o = ro[p], d = rd[p];
-                tally.extend++;
-                HitInfo h;
-                if constexpr (kShared > 0 && kWidth == 2) {
-                    SplitStack<kShared, 128, kTraversalStack + 1> stk;
-                    stk.top = stack_top + threadIdx.x;
-                    h = trace_closest_binary_s<kTraversalStack>(s, stk, xyz(o), xyz(d), o.w, d.w);
-                } else if constexpr (kSpec && kWidth == 2) {
-                    h = trace_closest_binary_spec(s, xyz(o), xyz(d), o.w, d.w);
-                } else {
-                    h = trace_closest_w<kWidth>(s, xyz(o), xyz(d), o.w, d.w);
-                }
-                hit[p] = make_float4(__uint_as_float(h.valid ? h.flat : 0xffffffffu), h.t, h.b1, h.b2);
+                h = trace_closest_w<kWidth>(s, xyz(o), xyz(d), o.w, d.w);
             }
+            hit[p] = make_float4(__uint_as_float(h.valid ? h.flat : 0xffffffffu), h.t, h.b1, h.b2);
         }
         if (first >= count) break;
-        if (lane == 0u) base = atomicAdd(ctl + 1, grab);
+        if (lane == 0u) base = atomicAdd(ctl + kExtFetch, grab);
         base = first + __shfl_sync(0xffffffffu, base, 0);
     }
     flush_tally(counters, tally, 0u, 0u);
@@ -212,7 +237,7 @@ template <int kWidth, class Src, int kShared = 0, bool kSpec = false>
 __global__ void __launch_bounds__(128, 9) k_wf_shadow(Src src, const float4* __restrict__ queue, uint32_t* ctl,
                                                    float t_max, float4* __restrict__ rad, float4* __restrict__ si,
                                                    unsigned long long* counters) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 2);
+    const uint32_t count = *(volatile uint32_t*)(ctl + kShd);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t grab = rays_per_grab(count);
     RayTally tally{0u, 0u};
@@ -242,8 +267,59 @@ __global__ void __launch_bounds__(128, 9) k_wf_shadow(Src src, const float4* __r
             }
         }
         if (first >= count) break;
-        if (lane == 0u) base = atomicAdd(ctl + 3, grab);
+        if (lane == 0u) base = atomicAdd(ctl + kShdFetch, grab);
         base = first + __shfl_sync(0xffffffffu, base, 0);
+    }
+    flush_tally(counters, tally, 0u, 0u);
+}
+
+// The trace launch of a round: the closest hits of the walking paths (ctl) and
+// the shadow rays of the round before (ctl_prev). Warps take chunks of up to
+// 32 rays of one kind, closest hits first. Against extend, shade, shadow and
+// finalize launches in turn: probe baker over 20,480 sites 6.14 -> 4.77 ms,
+// 256x256 box frame 267 -> 200 us, 1080p frame over 1M triangles
+// 2.71 -> 2.43 ms, 200k-triangle texel iteration 20.0 -> 19.6 ms.
+template <class Src>
+__global__ void __launch_bounds__(128, 9) k_wf_trace(Src src, const uint32_t* __restrict__ queue, uint32_t* ctl,
+                                                     const float4* __restrict__ ro, const float4* __restrict__ rd,
+                                                     float4* __restrict__ hit, const float4* __restrict__ shadows,
+                                                     const uint32_t* ctl_prev, float t_max, float4* __restrict__ rad,
+                                                     float4* __restrict__ si, unsigned long long* counters) {
+    const uint32_t rays = *(volatile uint32_t*)(ctl + kExt);
+    const uint32_t shadow_rays = *(const volatile uint32_t*)(ctl_prev + kShd);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t grab = rays_per_grab((unsigned long long)rays + shadow_rays);
+    const uint32_t ray_chunks = (rays + grab - 1u) / grab, chunks = ray_chunks + (shadow_rays + grab - 1u) / grab;
+    RayTally tally{0u, 0u};
+    for (uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < chunks;) {
+        if (c < ray_chunks) {
+            const uint32_t idx = c * grab + lane;
+            if (lane < grab && idx < rays) {
+                const uint32_t p = queue[idx];
+                const SceneView s = src.of(p);
+                const float4 o = ro[p], d = rd[p];
+                tally.extend++;
+                const HitInfo h = trace_closest_binary(s, xyz(o), xyz(d), o.w, d.w);
+                hit[p] = make_float4(__uint_as_float(h.valid ? h.flat : 0xffffffffu), h.t, h.b1, h.b2);
+            }
+        } else {
+            const uint32_t idx = (c - ray_chunks) * grab + lane;
+            if (lane < grab && idx < shadow_rays) {
+                const float4 a = shadows[3u * idx], b = shadows[3u * idx + 1u], e = shadows[3u * idx + 2u];
+                tally.shadow++;
+                const uint32_t p = __float_as_uint(a.w);
+                const SceneView s = src.of(p);
+                if (!trace_any_binary(s, xyz(a), xyz(b), 0.0f, e.w > 0.0f ? e.w : t_max)) {
+                    float4* target = (__float_as_uint(b.w) == kKindNee) ? rad : si;
+                    const float4 v = target[p];
+                    target[p] = make_float4(v.x + e.x, v.y + e.y, v.z + e.z, v.w);
+                }
+            }
+        }
+        if (chunks <= warps) break;
+        if (lane == 0u) c = atomicAdd(ctl + kExtFetch, 1u);
+        c = warps + __shfl_sync(0xffffffffu, c, 0);
     }
     flush_tally(counters, tally, 0u, 0u);
 }
@@ -259,10 +335,9 @@ __global__ void __launch_bounds__(128, 9) k_wf_shadow(Src src, const float4* __r
 template <int kRefill, int kBurst, class Src>
 __global__ void __launch_bounds__(128, 9) k_wf_extend_refill(Src src, const uint32_t* __restrict__ queue,
                                                           uint32_t* ctl, const float4* __restrict__ ro,
-                                                          const float4* __restrict__ rd,
-                                                          const uint32_t* __restrict__ flags,
-                                                          float4* __restrict__ hit, unsigned long long* counters) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
+                                                          const float4* __restrict__ rd, float4* __restrict__ hit,
+                                                          unsigned long long* counters) {
+    const uint32_t count = *(volatile uint32_t*)(ctl + kExt);
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
     RayTally tally{0u, 0u};
@@ -282,20 +357,16 @@ __global__ void __launch_bounds__(128, 9) k_wf_extend_refill(Src src, const uint
             }
             const uint32_t n = (uint32_t)__popc(idle);
             uint32_t base = 0u;
-            if (lane == 0u) base = atomicAdd(ctl + 1, n);
+            if (lane == 0u) base = atomicAdd(ctl + kExtFetch, n);
             base = __shfl_sync(0xffffffffu, base, 0);
             if (!alive) {
                 const uint32_t idx = base + (uint32_t)__popc(idle & below);
                 if (idx < count) {
                     p = queue[idx];
-                    if (flags[p] & kFlagNoPath) {
-                        hit[p] = make_float4(__uint_as_float(0xffffffffu), 0.0f, 0.0f, 0.0f);
-                    } else {
-                        const float4 o = ro[p], d = rd[p];
-                        tally.extend++;
-                        alive = closest_begin(src.of(p), w, xyz(o), xyz(d), o.w, d.w);
-                        pending = !alive;
-                    }
+                    const float4 o = ro[p], d = rd[p];
+                    tally.extend++;
+                    alive = closest_begin(src.of(p), w, xyz(o), xyz(d), o.w, d.w);
+                    pending = !alive;
                 }
             }
             if (base + n >= count) drained = true;
@@ -324,7 +395,7 @@ template <int kRefill, int kBurst, class Src>
 __global__ void __launch_bounds__(128, 9) k_wf_shadow_refill(Src src, const float4* __restrict__ queue, uint32_t* ctl,
                                                           float t_max, float4* __restrict__ rad,
                                                           float4* __restrict__ si, unsigned long long* counters) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 2);
+    const uint32_t count = *(volatile uint32_t*)(ctl + kShd);
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
     RayTally tally{0u, 0u};
@@ -346,7 +417,7 @@ __global__ void __launch_bounds__(128, 9) k_wf_shadow_refill(Src src, const floa
             }
             const uint32_t n = (uint32_t)__popc(idle);
             uint32_t base = 0u;
-            if (lane == 0u) base = atomicAdd(ctl + 3, n);
+            if (lane == 0u) base = atomicAdd(ctl + kShdFetch, n);
             base = __shfl_sync(0xffffffffu, base, 0);
             if (!alive) {
                 const uint32_t idx = base + (uint32_t)__popc(idle & below);
@@ -409,8 +480,9 @@ struct TexelArgs {
 
 // Start sample k of the current side: sun irradiance shadow ray, first
 // direction (estimate_surface_irradiance, texture_space_path_tracer.slang:95-113).
+// its shadow ray goes to the round of (buf, ctl), the path to the next one.
 __device__ __forceinline__ void texel_start_sample(const SceneView& s, const LightParams& L, const WfState& st,
-                                                   const WfQueues& q, int buf, uint32_t* ctl_next, uint32_t p,
+                                                   const WfQueues& q, int buf, uint32_t* ctl, uint32_t p,
                                                    uint32_t flags, Rng& rng, bool direct = true) {
     const float4 sf = st.surf[p];
     const uint32_t inst = __float_as_uint(sf.z), prim = __float_as_uint(sf.w);
@@ -421,24 +493,24 @@ __device__ __forceinline__ void texel_start_sample(const SceneView& s, const Lig
     const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
     const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
     // the two draws are taken either way, so the RNG streams stay aligned
-    if (direct) push_shadow(q, buf, ctl_next + 2, p, sd.origin_front, l, L.illum * ndl, kKindSun);
+    if (direct) push_shadow(q, buf, ctl, p, sd.origin_front, l, L.illum * ndl, kKindSun);
     st.si[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     st.rad[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     st.thp[p] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     const float e0 = rng.next_1d(), e1 = rng.next_1d();
     float pdf;
     const f3 dir = cosine_sample_hemisphere(e0, e1, &pdf);
-    flags &= ~(kFlagEnd | kFlagNoPath | kBounceMask);
+    flags &= ~(kFlagNoPath | kBounceMask);
     if (pdf > 1e-6f) {
         st.ro[p] = f4(sd.origin_front, 0.0f);
         st.rd[p] = f4(sd.frame.to_global(dir), L.t_max);
         st.zpdf[p] = make_float2(fabsf(dir.z), pdf);
+        push_path(q, buf ^ 1, ctl + kCtlWords, p);
     } else {
         flags |= kFlagNoPath;
+        push_close(q, buf ^ 1, ctl + kCtlWords, p);
     }
     st.flags[p] = flags;
-    const uint32_t slot = queue_slot(ctl_next + 0, true);
-    q.ext[buf][slot] = p;
 }
 
 __global__ void __launch_bounds__(128, 6) k_wf_texel_generate(SceneView s, LightingRaw lraw, TexelArgs a, WfState st,
@@ -454,7 +526,7 @@ __global__ void __launch_bounds__(128, 6) k_wf_texel_generate(SceneView s, Light
     st.surf[p] = make_float4(ts.b1, ts.b2, __uint_as_float(ts.inst), __uint_as_float(ts.prim));
     st.irr[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const uint32_t flags = (ts.side.y & 1u) ? kFlagTwoSided : 0u;
-    texel_start_sample(s, L, st, q, 0, q.ctl, p, flags, rng);
+    texel_start_sample(s, L, st, q, 1, q.ctl, p, flags, rng);
     st.rng[p] = rng.state;
     RayTally none{0u, 0u};
     flush_tally(counters, none, 1u, (ts.side.y & 1u) ? 2u * a.n : a.n);
@@ -482,93 +554,80 @@ __global__ void __launch_bounds__(128) k_wf_point_generate(SceneView s, Lighting
     st.unit[p] = u;
     st.surf[p] = make_float4(pt.x, pt.y, __uint_as_float(inst), __uint_as_float(prim));
     st.irr[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    texel_start_sample(s, L, st, q, 0, q.ctl, p, (primw >> 31) ? kFlagBack : 0u, rng, !a.indirect_only);
+    texel_start_sample(s, L, st, q, 1, q.ctl, p, (primw >> 31) ? kFlagBack : 0u, rng, !a.indirect_only);
     st.rng[p] = rng.state;
     RayTally none{0u, 0u};
     flush_tally(counters, none, 1u, a.n);
 }
 
-// One bounce of trace_radiance (texture_space_path_tracer.slang:60-83) after
-// the extend stage found the hit.
-__global__ void __launch_bounds__(128, 8) k_wf_texel_shade(SceneView s, LightingRaw lraw, TexelArgs a, WfState st,
+// One bounce of trace_radiance (texture_space_path_tracer.slang:60-83) for the
+// paths whose hit the trace found, and the closing of finished samples: si +=
+// L*|z|/pdf, irr += si, next sample / side, or the running-mean store
+// (texture_space_path_tracer.slang:111-138, 203-215).
+__global__ void __launch_bounds__(128, 8) k_wf_texel_stage(SceneView s, LightingRaw lraw, TexelArgs a, WfState st,
                                                         WfQueues q, int buf, uint32_t* ctl) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
-    const LightParams L = make_light(lraw);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx];
-        uint32_t flags = st.flags[p];
-        if (flags & kFlagNoPath) {
-            st.flags[p] = flags | kFlagEnd;
-            continue;
-        }
-        const float4 h = st.hit[p];
-        const f3 d = xyz(st.rd[p]);
-        f3 thp = xyz(st.thp[p]), rad = xyz(st.rad[p]);
-        const uint32_t flat = __float_as_uint(h.x);
-        if (flat == 0xffffffffu) {
-            rad = rad + thp * sky_radiance(L, d);
-            st.rad[p] = f4(rad, 0.0f);
-            st.flags[p] = flags | kFlagEnd;
-            continue;
-        }
-        Rng rng(0u, 0u, 0u);
-        rng.state = st.rng[p];
-        const uint2 ref = __ldg(s.tri_refs + flat);
-        const Shading sd = shading_data(s, ref.x, ref.y, h.z, h.w, -d);
-        rad = rad + thp * sd.emissive;
-        const float u0 = rng.next_1d(), u1 = rng.next_1d();
-        const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
-        const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
-        const f3 f = sd.diffuse * kInvPi;
-        push_shadow(q, buf, ctl + 2, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
-        const float e0 = rng.next_1d(), e1 = rng.next_1d();
-        float pdf;
-        const f3 sdir = cosine_sample_hemisphere(e0, e1, &pdf);
-        if (pdf <= 1e-6f) {
-            flags |= kFlagEnd;
-        } else {
-            thp = thp * ((f * fabsf(sdir.z)) / pdf);
-            st.ro[p] = f4(sd.origin_front, 0.0f);
-            st.rd[p] = f4(sd.frame.to_global(sdir), L.t_max);
-            const uint32_t bounce = ((flags & kBounceMask) >> kBounceShift) + 1u;
-            flags = (flags & ~kBounceMask) | (bounce << kBounceShift);
-            if (bounce >= a.max_bounces) flags |= kFlagEnd;
-        }
-        st.thp[p] = f4(thp, 0.0f);
-        st.rad[p] = f4(rad, 0.0f);
-        st.rng[p] = rng.state;
-        st.flags[p] = flags;
-    }
-}
-
-// Close finished samples: si += L*|z|/pdf, irr += si, next sample / side, or
-// the running-mean store (texture_space_path_tracer.slang:111-138, 203-215).
-__global__ void __launch_bounds__(128, 8) k_wf_texel_finalize(SceneView s, LightingRaw lraw, TexelArgs a, WfState st,
-                                                           WfQueues q, int buf, uint32_t* ctl, uint32_t* ctl_next) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
+    const uint32_t walking = *(volatile uint32_t*)(ctl + kExt);
+    const uint32_t count = walking + *(volatile uint32_t*)(ctl + kClose);
+    uint32_t* ctl_next = ctl + kCtlWords;
     const LightParams L = make_light(lraw);
     const int nbuf = buf ^ 1;
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx];
+        const uint32_t p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
         uint32_t flags = st.flags[p];
-        if (!(flags & kFlagEnd)) {
-            const uint32_t slot = queue_slot(ctl_next + 0, true);
-            q.ext[nbuf][slot] = p;
-            continue;
+        f3 rad = xyz(st.rad[p]);
+        if (idx < walking) {
+            const float4 h = st.hit[p];
+            const f3 d = xyz(st.rd[p]);
+            f3 thp = xyz(st.thp[p]);
+            const uint32_t flat = __float_as_uint(h.x);
+            if (flat != 0xffffffffu) {
+                Rng rng(0u, 0u, 0u);
+                rng.state = st.rng[p];
+                const uint2 ref = __ldg(s.tri_refs + flat);
+                const Shading sd = shading_data(s, ref.x, ref.y, h.z, h.w, -d);
+                rad = rad + thp * sd.emissive;
+                const float u0 = rng.next_1d(), u1 = rng.next_1d();
+                const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
+                const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
+                const f3 f = sd.diffuse * kInvPi;
+                push_shadow(q, buf, ctl, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
+                const float e0 = rng.next_1d(), e1 = rng.next_1d();
+                float pdf;
+                const f3 sdir = cosine_sample_hemisphere(e0, e1, &pdf);
+                bool ended = true;
+                if (pdf > 1e-6f) {
+                    const uint32_t bounce = ((flags & kBounceMask) >> kBounceShift) + 1u;
+                    flags = (flags & ~kBounceMask) | (bounce << kBounceShift);
+                    ended = bounce >= a.max_bounces;
+                    if (!ended) {
+                        thp = thp * ((f * fabsf(sdir.z)) / pdf);
+                        st.ro[p] = f4(sd.origin_front, 0.0f);
+                        st.rd[p] = f4(sd.frame.to_global(sdir), L.t_max);
+                        st.thp[p] = f4(thp, 0.0f);
+                    }
+                }
+                st.rad[p] = f4(rad, 0.0f);
+                st.rng[p] = rng.state;
+                st.flags[p] = flags;
+                if (ended) push_close(q, nbuf, ctl_next, p);
+                else push_path(q, nbuf, ctl_next, p);
+                continue;
+            }
+            rad = rad + thp * sky_radiance(L, d);
         }
         f3 si = xyz(st.si[p]);
         if (!(flags & kFlagNoPath)) {
             const float2 zp = st.zpdf[p];
-            si = si + ((xyz(st.rad[p]) * zp.x) / zp.y);
+            si = si + ((rad * zp.x) / zp.y);
         }
         f3 irr = xyz(st.irr[p]) + si;
         uint32_t k = (flags >> kSampleShift) + 1u;
         Rng rng(0u, 0u, 0u);
-        rng.state = st.rng[p];
         if (k < a.n) {
             flags = (flags & ((1u << kSampleShift) - 1u)) | (k << kSampleShift);
             st.irr[p] = f4(irr, 0.0f);
-            texel_start_sample(s, L, st, q, nbuf, ctl_next, p, flags, rng, !a.indirect_only);
+            rng.state = st.rng[p];
+            texel_start_sample(s, L, st, q, buf, ctl, p, flags, rng, !a.indirect_only);
             st.rng[p] = rng.state;
             continue;
         }
@@ -588,7 +647,8 @@ __global__ void __launch_bounds__(128, 8) k_wf_texel_finalize(SceneView s, Light
         if (!(flags & kFlagBack) && (flags & kFlagTwoSided)) {
             flags = (flags & ((1u << kSampleShift) - 1u)) | kFlagBack;
             st.irr[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            texel_start_sample(s, L, st, q, nbuf, ctl_next, p, flags, rng);
+            rng.state = st.rng[p];
+            texel_start_sample(s, L, st, q, buf, ctl, p, flags, rng);
             st.rng[p] = rng.state;
         }
     }
@@ -628,7 +688,6 @@ struct ScreenArgs {
     float4* out;
     uint32_t width, height, frame, max_vertices;
     int cached;
-    int area_nee;  // lighting flag bit 1 (the finalize stage has no lighting)
     CachedArgs cache;
 };
 
@@ -663,8 +722,7 @@ __global__ void __launch_bounds__(128) k_wf_screen_generate(SceneView s, Lightin
     st.rad[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     st.si[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     st.zpdf[p] = make_float2(0.0f, 1.0f);
-    const uint32_t slot = queue_slot(q.ctl + 0, true);
-    q.ext[0][slot] = p;
+    push_path(q, 0, q.ctl + kCtlWords, p);
     RayTally none{0u, 0u};
     flush_tally(counters, none, 1u, 1u);
 }
@@ -677,13 +735,22 @@ __device__ __forceinline__ f3 fold_area_term(const WfState& st, uint32_t p, f3 r
     return rad + xyz(a);
 }
 
-__global__ void __launch_bounds__(128, 6) k_wf_screen_shade(SceneView s, LightingRaw lraw, ScreenArgs a, WfState st,
+__global__ void __launch_bounds__(128, 6) k_wf_screen_stage(SceneView s, LightingRaw lraw, ScreenArgs a, WfState st,
                                                          WfQueues q, int buf, uint32_t* ctl) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
+    const uint32_t walking = *(volatile uint32_t*)(ctl + kExt);
+    const uint32_t count = walking + *(volatile uint32_t*)(ctl + kClose);
+    uint32_t* ctl_next = ctl + kCtlWords;
+    const int nbuf = buf ^ 1;
     const LightParams L = make_light(lraw);
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx];
-        uint32_t flags = st.flags[p];
+        const uint32_t p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
+        if (idx >= walking) {
+            f3 r = xyz(st.rad[p]);
+            if (L.area_nee) r = r + xyz(st.si[p]);
+            a.out[st.unit[p]] = f4(r, 1.0f);
+            continue;
+        }
+        const uint32_t flags = st.flags[p];
         const float4 h = st.hit[p];
         const f3 d = xyz(st.rd[p]);
         f3 thp = xyz(st.thp[p]), rad = xyz(st.rad[p]);
@@ -694,8 +761,9 @@ __global__ void __launch_bounds__(128, 6) k_wf_screen_shade(SceneView s, Lightin
             f3 sky = sky_radiance(L, d);
             if (vertex == 0u && L.sun_disk) sky = sky + sun_disk(L, d);
             rad = rad + thp * sky;
-            st.rad[p] = f4(rad, 0.0f);
-            st.flags[p] = flags | kFlagEnd;
+            // (an area-light term of zero: the last vertex's is in rad)
+            if (L.area_nee) rad = rad + mk3(0.0f, 0.0f, 0.0f);
+            a.out[st.unit[p]] = f4(rad, 1.0f);
             continue;
         }
         Rng rng(0u, 0u, 0u);
@@ -715,7 +783,7 @@ __global__ void __launch_bounds__(128, 6) k_wf_screen_shade(SceneView s, Lightin
                 const float u0 = rng.next_1d(), u1 = rng.next_1d();
                 const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
                 const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
-                push_shadow(q, buf, ctl + 2, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
+                push_shadow(q, buf, ctl, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
             }
             const uint32_t pixel = st.unit[p];
             const uint32_t qi = queue_slot(a.cache.query_count, true);
@@ -737,20 +805,25 @@ __global__ void __launch_bounds__(128, 6) k_wf_screen_shade(SceneView s, Lightin
                 a.cache.train_queries[2u * ti] = q0;
                 a.cache.train_queries[2u * ti + 1u] = q1;
             }
-            st.rad[p] = f4(rad, 0.0f);
-            st.flags[p] = flags | kFlagEnd;
+            if (vertex == 0u) {
+                st.rad[p] = f4(rad, 0.0f);
+                push_close(q, nbuf, ctl_next, p);  // its sun ray is in flight
+            } else {
+                if (L.area_nee) rad = rad + mk3(0.0f, 0.0f, 0.0f);
+                a.out[pixel] = f4(rad, 1.0f);
+            }
             continue;
         }
         const float u0 = rng.next_1d(), u1 = rng.next_1d();
         const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
         const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
-        push_shadow(q, buf, ctl + 2, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
+        push_shadow(q, buf, ctl, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
         // light reached from this vertex lies on the next one: sampled only
         // where that vertex exists, so both strategies cover the same paths
         if (L.area_nee && vertex + 1u < a.max_vertices) {
             const float us = rng.next_1d(), a0 = rng.next_1d(), a1 = rng.next_1d();
             const AreaSample as = area_nee_sample(s, sd, us, a0, a1);
-            if (as.valid) push_shadow(q, buf, ctl + 2, p, sd.origin_front, as.dir, thp * as.contrib, kKindSun, as.tmax);
+            if (as.valid) push_shadow(q, buf, ctl, p, sd.origin_front, as.dir, thp * as.contrib, kKindSun, as.tmax);
         }
         const float e0 = rng.next_1d(), e1 = rng.next_1d();
         float pdf;
@@ -761,31 +834,12 @@ __global__ void __launch_bounds__(128, 6) k_wf_screen_shade(SceneView s, Lightin
         st.ro[p] = f4(sd.origin_front, 0.0f);
         st.rd[p] = f4(sd.frame.to_global(wo), L.t_max);
         const uint32_t next = vertex + 1u;
-        flags = (flags & ~kBounceMask) | (next << kBounceShift);
-        if (next >= a.max_vertices) flags |= kFlagEnd;
         st.thp[p] = f4(thp, 0.0f);
         st.rad[p] = f4(rad, 0.0f);
         st.rng[p] = rng.state;
-        st.flags[p] = flags;
-    }
-}
-
-__global__ void __launch_bounds__(128) k_wf_screen_finalize(ScreenArgs a, WfState st, WfQueues q, int buf,
-                                                            uint32_t* ctl, uint32_t* ctl_next) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx];
-        if (!(st.flags[p] & kFlagEnd)) {
-            const uint32_t slot = queue_slot(ctl_next + 0, true);
-            q.ext[buf ^ 1][slot] = p;
-            continue;
-        }
-        float4 r = st.rad[p];
-        if (a.area_nee) {
-            const float4 t = st.si[p];
-            r = make_float4(r.x + t.x, r.y + t.y, r.z + t.z, r.w);
-        }
-        a.out[st.unit[p]] = make_float4(r.x, r.y, r.z, 1.0f);
+        st.flags[p] = (flags & ~kBounceMask) | (next << kBounceShift);
+        if (next >= a.max_vertices) push_close(q, nbuf, ctl_next, p);
+        else push_path(q, nbuf, ctl_next, p);
     }
 }
 
@@ -809,9 +863,10 @@ __device__ __forceinline__ Shading probe_surface(const SceneView& s, const Probe
     return shading_data(s, __float_as_uint(surf.z), __float_as_uint(surf.w), surf.x, surf.y, view);
 }
 
-// One cosine sample around the face normal (no sun at the probe itself).
+// One cosine sample around the face normal (no sun at the probe itself); the
+// path goes to the queue of the round of (buf, ctl).
 __device__ __forceinline__ void probe_start_sample(const SceneView& s, const LightParams& L, const ProbeArgs& a,
-                                                   const WfState& st, const WfQueues& q, int buf, uint32_t* ctl_next,
+                                                   const WfState& st, const WfQueues& q, int buf, uint32_t* ctl,
                                                    uint32_t p, uint32_t flags, Rng& rng) {
     const float4 surf = st.surf[p];
     const Shading sd = probe_surface(s, a, st.unit[p], surf);
@@ -819,7 +874,7 @@ __device__ __forceinline__ void probe_start_sample(const SceneView& s, const Lig
     const float e0 = rng.next_1d(), e1 = rng.next_1d();
     float pdf;
     const f3 dir = cosine_sample_hemisphere(e0, e1, &pdf);
-    flags &= ~(kFlagEnd | kFlagNoPath | kBounceMask);
+    flags &= ~(kFlagNoPath | kBounceMask);
     if (pdf > 1e-6f) {
         const f3 o = sd.origin_front;
         st.ro[p] = f4(o, 0.0f);
@@ -832,12 +887,12 @@ __device__ __forceinline__ void probe_start_sample(const SceneView& s, const Lig
         b.x = 0u;
         b.w = radial_texel(dir);
         st.pb[p] = b;
+        push_path(q, buf, ctl, p);
     } else {
         flags |= kFlagNoPath;
+        push_close(q, buf, ctl, p);
     }
     st.flags[p] = flags;
-    const uint32_t slot = queue_slot(ctl_next + 0, true);
-    q.ext[buf][slot] = p;
 }
 
 // Per-path bodies of the probe stages, shared by the one-scene kernels and the
@@ -863,19 +918,17 @@ __device__ __forceinline__ bool probe_generate_path(const SceneView& s, const Li
     if (a.reset)
         for (int t = 0; t < 16; ++t) a.out.radial[16u * probe + (uint32_t)t] = 0u;
     Rng rng(probe, inst, a.iteration * a.n);
-    probe_start_sample(s, L, a, st, q, 0, q.ctl, p, 0u, rng);
+    probe_start_sample(s, L, a, st, q, 0, q.ctl + kCtlWords, p, 0u, rng);
     st.rng[p] = rng.state;
     return true;
 }
 
-__device__ __forceinline__ void probe_shade_path(const SceneView& s, const LightParams& L, const ProbeArgs& a,
+// Shades the path's hit. False when the path has left the scene: its sample
+// has no shadow ray in flight and can be closed.
+__device__ __forceinline__ bool probe_shade_path(const SceneView& s, const LightParams& L, const ProbeArgs& a,
                                                  const WfState& st, const WfQueues& q, int buf, uint32_t* ctl,
                                                  uint32_t p) {
     uint32_t flags = st.flags[p];
-    if (flags & kFlagNoPath) {
-        st.flags[p] = flags | kFlagEnd;
-        return;
-    }
     const float4 h = st.hit[p];
     const f3 d = xyz(st.rd[p]);
     f3 thp = xyz(st.thp[p]), rad = xyz(st.rad[p]);
@@ -888,8 +941,7 @@ __device__ __forceinline__ void probe_shade_path(const SceneView& s, const Light
         rad = rad + thp * sky_radiance(L, d);
         st.pa[p] = pa;
         st.rad[p] = f4(rad, 0.0f);
-        st.flags[p] = flags | kFlagEnd;
-        return;
+        return false;
     }
     if (bounce == 0u) pa.w = minf(h.y, radial_max);
     const uint2 ref = __ldg(s.tri_refs + flat);
@@ -911,13 +963,12 @@ __device__ __forceinline__ void probe_shade_path(const SceneView& s, const Light
     const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
     const f3 f = sd.diffuse * kInvPi;
     // the set's own t_max travels with the shadow ray (the batch mixes scenes)
-    push_shadow(q, buf, ctl + 2, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee, L.t_max);
+    push_shadow(q, buf, ctl, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee, L.t_max);
     const float e0 = rng.next_1d(), e1 = rng.next_1d();
     float pdf;
     const f3 sdir = cosine_sample_hemisphere(e0, e1, &pdf);
-    if (pdf <= 1e-6f) {
-        flags |= kFlagEnd;
-    } else {
+    bool ended = true;
+    if (pdf > 1e-6f) {
         thp = thp * ((f * fabsf(sdir.z)) / pdf);
         const f3 next_origin = sd.origin_front;
         st.ro[p] = f4(next_origin, 0.0f);
@@ -927,25 +978,24 @@ __device__ __forceinline__ void probe_shade_path(const SceneView& s, const Light
         pa.z = len3(next_origin - sd.position);
         const uint32_t next = bounce + 1u;
         flags = (flags & ~kBounceMask) | (next << kBounceShift);
-        if (next >= a.max_bounces) flags |= kFlagEnd;
+        ended = next >= a.max_bounces;
     }
     st.pa[p] = pa;
     st.thp[p] = f4(thp, 0.0f);
     st.rad[p] = f4(rad, 0.0f);
     st.rng[p] = rng.state;
     st.flags[p] = flags;
+    if (ended) push_close(q, buf ^ 1, ctl + kCtlWords, p);
+    else push_path(q, buf ^ 1, ctl + kCtlWords, p);
+    return true;
 }
 
-__device__ __forceinline__ void probe_finalize_path(const SceneView& s, const LightParams& L, const ProbeArgs& a,
-                                                    const WfState& st, const WfQueues& q, int buf,
-                                                    uint32_t* ctl_next, uint32_t p) {
-    const int nbuf = buf ^ 1;
-    uint32_t flags = st.flags[p];
-    if (!(flags & kFlagEnd)) {
-        const uint32_t slot = queue_slot(ctl_next + 0, true);
-        q.ext[nbuf][slot] = p;
-        return;
-    }
+// Closes the path's sample: the next one starts in the next round, or the
+// probe's running mean is stored.
+__device__ __forceinline__ void probe_close_path(const SceneView& s, const LightParams& L, const ProbeArgs& a,
+                                                 const WfState& st, const WfQueues& q, int buf, uint32_t* ctl,
+                                                 uint32_t p) {
+    const uint32_t flags = st.flags[p];
     const uint32_t probe = st.unit[p];
     f3 irr = xyz(st.irr[p]);
     uint4 b = st.pb[p];
@@ -969,7 +1019,7 @@ __device__ __forceinline__ void probe_finalize_path(const SceneView& s, const Li
         st.irr[p] = f4(irr, 0.0f);
         Rng rng(0u, 0u, 0u);
         rng.state = st.rng[p];
-        probe_start_sample(s, L, a, st, q, nbuf, ctl_next, p,
+        probe_start_sample(s, L, a, st, q, buf ^ 1, ctl + kCtlWords, p,
                            (flags & ((1u << kSampleShift) - 1u)) | (k << kSampleShift), rng);
         st.rng[p] = rng.state;
         return;
@@ -1000,20 +1050,16 @@ __global__ void __launch_bounds__(128) k_wf_probe_generate(SceneView s, Lighting
     flush_tally(counters, none, 1u, a.n);
 }
 
-__global__ void __launch_bounds__(128, 6) k_wf_probe_shade(SceneView s, LightingRaw lraw, ProbeArgs a, WfState st,
+__global__ void __launch_bounds__(128, 6) k_wf_probe_stage(SceneView s, LightingRaw lraw, ProbeArgs a, WfState st,
                                                         WfQueues q, int buf, uint32_t* ctl) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
+    const uint32_t walking = *(volatile uint32_t*)(ctl + kExt);
+    const uint32_t count = walking + *(volatile uint32_t*)(ctl + kClose);
     const LightParams L = make_light(lraw);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x)
-        probe_shade_path(s, L, a, st, q, buf, ctl, q.ext[buf][idx]);
-}
-
-__global__ void __launch_bounds__(128, 6) k_wf_probe_finalize(SceneView s, LightingRaw lraw, ProbeArgs a, WfState st,
-                                                           WfQueues q, int buf, uint32_t* ctl, uint32_t* ctl_next) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
-    const LightParams L = make_light(lraw);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x)
-        probe_finalize_path(s, L, a, st, q, buf, ctl_next, q.ext[buf][idx]);
+    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
+        const uint32_t p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
+        if (idx >= walking || !probe_shade_path(s, L, a, st, q, buf, ctl, p))
+            probe_close_path(s, L, a, st, q, buf, ctl, p);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1111,27 +1157,26 @@ __global__ void __launch_bounds__(128) k_wfi_probe_generate(BatchWfArgs m, WfSta
     st.si[p] = make_float4(0.0f, 0.0f, 0.0f, maxf(params.x, 1e-6f));
     st.pb[p] = make_uint4(0u, 0u, 0u, 0u);
     Rng rng(probe, inst, a.iteration * m.n + k);
-    probe_start_sample(b.s, make_light(b.light), a, st, q, 0, q.ctl, p, 0u, rng);
+    probe_start_sample(b.s, make_light(b.light), a, st, q, 0, q.ctl + kCtlWords, p, 0u, rng);
     st.rng[p] = rng.state;
 }
 
-__global__ void __launch_bounds__(128) k_wfi_probe_finalize(BatchWfArgs m, WfState st, WfQueues q, int buf,
-                                                            uint32_t* ctl, uint32_t* ctl_next) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
+__global__ void __launch_bounds__(128, 6) k_wfi_probe_stage(BatchWfArgs m, WfState st, WfQueues q, int buf,
+                                                            uint32_t* ctl) {
+    const uint32_t walking = *(volatile uint32_t*)(ctl + kExt);
+    const uint32_t count = walking + *(volatile uint32_t*)(ctl + kClose);
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx];
-        const uint32_t flags = st.flags[p];
-        if (!(flags & kFlagEnd)) {
-            const uint32_t slot = queue_slot(ctl_next + 0, true);
-            q.ext[buf ^ 1][slot] = p;
-            continue;
+        const uint32_t p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
+        if (idx < walking) {
+            const BatchSet& b = m.sets[m.set_of[p]];
+            if (probe_shade_path(b.s, make_light(b.light), batch_probe_args(m, b), st, q, buf, ctl, p)) continue;
         }
         ProbeSample r;
         r.si = mk3(0.0f, 0.0f, 0.0f);
         r.self_hits = 0u;
         r.texel = 0u;
         r.nd = 0.0f;
-        r.has_path = !(flags & kFlagNoPath);
+        r.has_path = !(st.flags[p] & kFlagNoPath);
         if (r.has_path) {
             const uint4 b = st.pb[p];
             const float2 zp = st.zpdf[p];
@@ -1166,23 +1211,17 @@ __global__ void __launch_bounds__(128) k_wfi_probe_fold(BatchWfArgs m, unsigned 
     flush_tally(counters, none, 1u, m.n);
 }
 
-__global__ void __launch_bounds__(128, 6) k_wfb_probe_shade(BatchWfArgs m, WfState st, WfQueues q, int buf,
+__global__ void __launch_bounds__(128, 6) k_wfb_probe_stage(BatchWfArgs m, WfState st, WfQueues q, int buf,
                                                          uint32_t* ctl) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
+    const uint32_t walking = *(volatile uint32_t*)(ctl + kExt);
+    const uint32_t count = walking + *(volatile uint32_t*)(ctl + kClose);
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx];
+        const uint32_t p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
         const BatchSet& b = m.sets[m.set_of[p]];
-        probe_shade_path(b.s, make_light(b.light), batch_probe_args(m, b), st, q, buf, ctl, p);
-    }
-}
-
-__global__ void __launch_bounds__(128, 6) k_wfb_probe_finalize(BatchWfArgs m, WfState st, WfQueues q, int buf,
-                                                            uint32_t* ctl, uint32_t* ctl_next) {
-    const uint32_t count = *(volatile uint32_t*)(ctl + 0);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx];
-        const BatchSet& b = m.sets[m.set_of[p]];
-        probe_finalize_path(b.s, make_light(b.light), batch_probe_args(m, b), st, q, buf, ctl_next, p);
+        const LightParams L = make_light(b.light);
+        const ProbeArgs a = batch_probe_args(m, b);
+        if (idx >= walking || !probe_shade_path(b.s, L, a, st, q, buf, ctl, p))
+            probe_close_path(b.s, L, a, st, q, buf, ctl, p);
     }
 }
 
@@ -1228,7 +1267,7 @@ template <class T> T* carve(unsigned char*& cur, size_t count) {
 template <class Src>
 void launch_extend(const NanContext* ctx, int blocks, cudaStream_t st, bool wide, Src src, const uint32_t* queue,
                    uint32_t* ctl, const WfState& S) {
-#define NAN_EXT_ARGS src, queue, ctl, S.ro, S.rd, S.flags, S.hit, ctx->d_counters
+#define NAN_EXT_ARGS src, queue, ctl, S.ro, S.rd, S.hit, ctx->d_counters
     if (wide) k_wf_extend<8><<<blocks, 128, 0, st>>>(NAN_EXT_ARGS);
     else switch (ctx->tuning.traversal) {
         case 1: k_wf_extend_refill<8, 1, Src><<<blocks, 128, 0, st>>>(NAN_EXT_ARGS); break;
@@ -1264,16 +1303,41 @@ struct Grid {
     int stream_blocks;
 };
 
-Grid grid_for(const NanContext* ctx) {
+// Launch shapes for up to `paths` paths in flight: no more blocks than they
+// can fill (a warp takes at least one ray of the at most three per path).
+Grid grid_for(const NanContext* ctx, uint64_t paths) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wf_extend<2, OneScene>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wf_trace<OneScene>, 128, 0);
     Grid g;
     const int per_sm = ctx->tuning.trace_blocks_per_sm ? (int)ctx->tuning.trace_blocks_per_sm : std::max(occ, 1);
-    g.persistent_blocks = sms * per_sm;
-    g.stream_blocks = sms * 16;
+    g.persistent_blocks = (int)std::min<uint64_t>((uint64_t)sms * per_sm, std::max<uint64_t>((3 * paths + 3) / 4, 1));
+    g.stream_blocks = (int)std::min<uint64_t>((uint64_t)sms * 16, std::max<uint64_t>((paths + 127) / 128, 1));
     return g;
+}
+
+// The traversal of round `it`: the closest hits of its walking paths and the
+// shadow rays that the round before queued, in one launch; in two (extend, then
+// shadow) for the wide nodes, the other traversal forms and stage timing.
+template <class Src>
+void launch_trace(NanContext* ctx, int blocks, cudaStream_t st, bool wide, Src src, const WfQueues& q, uint32_t it,
+                  float t_max, const WfState& S) {
+    const int buf = (int)(it & 1u);
+    uint32_t* ctl = q.ctl + kCtlWords * (it + 1u);
+    if (!wide && ctx->tuning.traversal == 0u && !ctx->tuning.kernel_timing) {
+        k_wf_trace<Src><<<blocks, 128, 0, st>>>(src, q.ext[buf], ctl, S.ro, S.rd, S.hit, q.shd[buf ^ 1],
+                                                ctl - kCtlWords, t_max, S.rad, S.si, ctx->d_counters);
+        ctx->launches++;
+        return;
+    }
+    cudaEvent_t ev = nan_host::timing_begin(ctx, st);
+    launch_extend(ctx, blocks, st, wide, src, q.ext[buf], ctl, S);
+    nan_host::timing_end(ctx, 0, ev, st);
+    ev = nan_host::timing_begin(ctx, st);
+    launch_shadow(ctx, blocks, st, wide, src, q.shd[buf ^ 1], ctl - kCtlWords, t_max, S);
+    nan_host::timing_end(ctx, 1, ev, st);
+    ctx->launches += 2;
 }
 
 }  // namespace
@@ -1359,15 +1423,20 @@ void release_timing(NanContext* ctx) {
     ctx->event_pool.clear();
 }
 
-// Scratch plan shared by the integrators: control words for `iters`
-// iterations plus as many paths as the arena holds (or the tuning cap).
-int wf_plan(NanContext* ctx, uint64_t iters64, uint32_t* iters, uint64_t* cap) {
+// Scratch plan shared by the integrators: `samples` samples of up to `bounces`
+// traced vertices each take bounces + 1 rounds (the last one closes); control
+// words for them plus as many paths as the arena holds (or the tuning cap).
+// 8 words a round, at most 2 rounds per bounce, fit the 20 words a bounce
+// set aside.
+int wf_plan(NanContext* ctx, uint64_t samples, uint32_t bounces, uint32_t* rounds, uint64_t* cap) {
+    const uint64_t iters64 = samples * bounces;
     if (iters64 > (1u << 20)) {
         set_error("samples * bounces too large for the wavefront schedule");
         return NAN_ERR_INVALID_ARGUMENT;
     }
-    *iters = (uint32_t)iters64;
-    const size_t ctl_bytes = ((size_t)(*iters + 2) * 20 * sizeof(uint32_t) + 255u) / 256u * 256u;
+    *rounds = (uint32_t)(samples * (bounces + 1u));
+    const size_t ctl_bytes = ((size_t)(iters64 + 2) * 20 * sizeof(uint32_t) + 255u) / 256u * 256u;
+    static_assert(20 >= 2 * kCtlWords, "control words");
     if (ctx->scratch_bytes <= ctl_bytes + 8192) {
         set_error("no wavefront scratch reserved on this context (nan_ctx_reserve)");
         return NAN_ERR_INVALID_ARGUMENT;
@@ -1381,10 +1450,13 @@ int wf_plan(NanContext* ctx, uint64_t iters64, uint32_t* iters, uint64_t* cap) {
     return NAN_OK;
 }
 
-void wf_carve(NanContext* ctx, uint32_t count, uint32_t iters, WfState& S, WfQueues& q) {
+size_t ctl_words(uint32_t rounds) { return (size_t)(rounds + 2) * kCtlWords + 16; }
+
+void wf_carve(NanContext* ctx, uint32_t count, uint32_t rounds, WfState& S, WfQueues& q) {
     unsigned char* cur = static_cast<unsigned char*>(ctx->scratch);
-    q.ctl = carve<uint32_t>(cur, (size_t)(iters + 2) * 20);
-    q.oct = q.ctl + (size_t)(iters + 2) * 4;
+    q.ctl = carve<uint32_t>(cur, ctl_words(rounds));
+    q.oct = q.ctl + (size_t)(rounds + 2) * kCtlWords;
+    q.cap = count;
     S.unit = carve<uint32_t>(cur, count);
     S.rng = carve<uint32_t>(cur, count);
     S.flags = carve<uint32_t>(cur, count);
@@ -1407,51 +1479,45 @@ void wf_carve(NanContext* ctx, uint32_t count, uint32_t iters, WfState& S, WfQue
     q.shd[1] = carve<float4>(cur, 3ull * 2 * count);
 }
 
-// Runs units [begin, end) in chunks: generate, then `iters` rounds of
-// extend / shade / shadow / finalize. gen(S, q, first_unit, count),
-// shade(S, q, buf, ctl) and fin(S, q, buf, ctl, ctl_next) launch the
-// integrator's own stages.
-template <class Gen, class Shade, class Fin>
-int wf_run(NanContext* ctx, cudaStream_t st, uint64_t begin, uint64_t end, uint32_t iters, uint64_t cap, float t_max,
-           Gen gen, Shade shade, Fin fin) {
+// Runs units [begin, end) in chunks: generate, then `rounds` rounds of trace
+// and stage. gen(S, q, first_unit, count) and stage(S, q, buf, ctl, blocks)
+// launch the integrator's own stages. The control block of round k is block
+// k + 1: the generated paths' shadow rays belong to block 0.
+template <class Gen, class Stage>
+int wf_run(NanContext* ctx, cudaStream_t st, uint64_t begin, uint64_t end, uint32_t rounds, uint64_t cap, float t_max,
+           Gen gen, Stage stage) {
     const SceneView s = scene_view(ctx);
-    const Grid g = grid_for(ctx);
+    const Grid g = grid_for(ctx, std::min<uint64_t>(cap, end - begin));
     for (uint64_t cb = begin; cb < end; cb += cap) {
         const uint32_t count = (uint32_t)std::min<uint64_t>(cap, end - cb);
         WfState S;
         WfQueues q;
-        wf_carve(ctx, count, iters, S, q);
-        cudaError_t err = cudaMemsetAsync(q.ctl, 0, (size_t)(iters + 2) * 20 * sizeof(uint32_t), st);
+        wf_carve(ctx, count, rounds, S, q);
+        cudaError_t err = cudaMemsetAsync(q.ctl, 0, ctl_words(rounds) * sizeof(uint32_t), st);
         if (err != cudaSuccess) return cuda_fail(err, "wavefront control reset");
         cudaEvent_t ev = timing_begin(ctx, st);
         gen(S, q, (uint32_t)cb, count);
         timing_end(ctx, 2, ev, st);
         ctx->launches++;
-        for (uint32_t it = 0; it < iters; ++it) {
+        for (uint32_t it = 0; it < rounds; ++it) {
             const int buf = (int)(it & 1u);
-            uint32_t* ctl = q.ctl + 4u * it;
+            uint32_t* ctl = q.ctl + kCtlWords * (it + 1u);
             if (ctx->tuning.ray_order == 1u) {
                 ev = timing_begin(ctx, st);
-                uint32_t* oct = q.oct + 16u * it;
-                k_wf_octant_count<<<g.stream_blocks, 256, 0, st>>>(q.ext[buf], ctl, S.rd, oct);
-                k_wf_octant_place<<<g.stream_blocks, 256, 0, st>>>(q.ext[buf], ctl, S.rd, oct, q.ext_sorted);
+                err = cudaMemsetAsync(q.oct, 0, 16 * sizeof(uint32_t), st);
+                if (err != cudaSuccess) return cuda_fail(err, "ray order reset");
+                k_wf_octant_count<<<g.stream_blocks, 256, 0, st>>>(q.ext[buf], ctl, S.rd, q.oct);
+                k_wf_octant_place<<<g.stream_blocks, 256, 0, st>>>(q.ext[buf], ctl, S.rd, q.oct, q.ext_sorted);
+                k_wf_close_copy<<<g.stream_blocks, 256, 0, st>>>(q.ext[buf], ctl, q.cap, q.ext_sorted);
                 timing_end(ctx, 2, ev, st);
                 std::swap(q.ext[buf], q.ext_sorted);
-                ctx->launches += 2;
+                ctx->launches += 3;
             }
+            launch_trace(ctx, g.persistent_blocks, st, s.wnodes != nullptr, OneScene{s}, q, it, t_max, S);
             ev = timing_begin(ctx, st);
-            launch_extend(ctx, g.persistent_blocks, st, s.wnodes != nullptr, OneScene{s}, q.ext[buf], ctl, S);
-            timing_end(ctx, 0, ev, st);
-            ev = timing_begin(ctx, st);
-            shade(S, q, buf, ctl);
+            stage(S, q, buf, ctl, g.stream_blocks);
             timing_end(ctx, 2, ev, st);
-            ev = timing_begin(ctx, st);
-            launch_shadow(ctx, g.persistent_blocks, st, s.wnodes != nullptr, OneScene{s}, q.shd[buf], ctl, t_max, S);
-            timing_end(ctx, 1, ev, st);
-            ev = timing_begin(ctx, st);
-            fin(S, q, buf, ctl, ctl + 4);
-            timing_end(ctx, 2, ev, st);
-            ctx->launches += 4;
+            ctx->launches++;
         }
         err = cudaGetLastError();
         if (err != cudaSuccess) return cuda_fail(err, "wavefront launch");
@@ -1464,10 +1530,10 @@ int launch_trace_texels_wavefront(NanContext* ctx, const NanMeshColorsDesc* lay,
                                   const NanLighting* light, uint32_t begin, uint32_t end, cudaStream_t st) {
     if (end <= begin) return NAN_OK;
     const uint32_t n = std::max(spt, 1u);
-    uint32_t iters = 0;
+    uint32_t rounds = 0;
     uint64_t cap = 0;
-    // a path may run its back side after its front: 2 sides x n samples x bounces
-    int rc = wf_plan(ctx, 2ull * n * std::max(max_bounces, 1u), &iters, &cap);
+    // a path may run its back side after its front: 2 sides x n samples
+    int rc = wf_plan(ctx, 2ull * n, std::max(max_bounces, 1u), &rounds, &cap);
     if (rc) return rc;
     const SceneView s = scene_view(ctx);
     const LightingRaw lr = to_raw(light);
@@ -1485,18 +1551,14 @@ int launch_trace_texels_wavefront(NanContext* ctx, const NanMeshColorsDesc* lay,
     a.n = n;
     a.max_bounces = std::max(max_bounces, 1u);
     a.reset = reset;
-    const Grid g = grid_for(ctx);
     unsigned long long* counters = ctx->d_counters;
     return wf_run(
-        ctx, st, begin, end, iters, cap, lr.ray_t_max,
+        ctx, st, begin, end, rounds, cap, lr.ray_t_max,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t count) {
             k_wf_texel_generate<<<(count + 127) / 128, 128, 0, st>>>(s, lr, a, S, q, first, count, counters);
         },
-        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl) {
-            k_wf_texel_shade<<<g.stream_blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
-        },
-        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, uint32_t* ctl_next) {
-            k_wf_texel_finalize<<<g.stream_blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl, ctl_next);
+        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, int blocks) {
+            k_wf_texel_stage<<<blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
         });
 }
 
@@ -1538,9 +1600,9 @@ int launch_trace_points_wavefront(NanContext* ctx, const float* points, uint32_t
                                   const NanLighting* light, cudaStream_t st) {
     if (count == 0) return NAN_OK;
     const uint32_t n = std::max(samples, 1u);
-    uint32_t iters = 0;
+    uint32_t rounds = 0;
     uint64_t cap = 0;
-    int rc = wf_plan(ctx, (uint64_t)n * std::max(max_bounces, 1u), &iters, &cap);
+    int rc = wf_plan(ctx, n, std::max(max_bounces, 1u), &rounds, &cap);
     if (rc) return rc;
     const SceneView s = scene_view(ctx);
     const LightingRaw lr = to_raw(light);
@@ -1552,18 +1614,14 @@ int launch_trace_points_wavefront(NanContext* ctx, const float* points, uint32_t
     a.points = reinterpret_cast<const float4*>(points);
     a.point_out = reinterpret_cast<float4*>(out);
     a.indirect_only = (flags & NAN_POINTS_INDIRECT_ONLY) != 0u;
-    const Grid g = grid_for(ctx);
     unsigned long long* counters = ctx->d_counters;
     return wf_run(
-        ctx, st, 0, count, iters, cap, lr.ray_t_max,
+        ctx, st, 0, count, rounds, cap, lr.ray_t_max,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t cnt) {
             k_wf_point_generate<<<(cnt + 127) / 128, 128, 0, st>>>(s, lr, a, S, q, first, cnt, counters);
         },
-        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl) {
-            k_wf_texel_shade<<<g.stream_blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
-        },
-        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, uint32_t* ctl_next) {
-            k_wf_texel_finalize<<<g.stream_blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl, ctl_next);
+        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, int blocks) {
+            k_wf_texel_stage<<<blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
         });
 }
 
@@ -1572,9 +1630,9 @@ int screen_wavefront(NanContext* ctx, float* out, uint32_t w, uint32_t h, uint32
                      const NanCamera* cam, const NanLighting* light, const CachedArgs* cached, cudaStream_t st) {
     const uint64_t pixels = (uint64_t)w * h;
     if (pixels == 0 || max_vertices == 0) return NAN_OK;
-    uint32_t iters = 0;
+    uint32_t rounds = 0;
     uint64_t cap = 0;
-    int rc = wf_plan(ctx, max_vertices, &iters, &cap);
+    int rc = wf_plan(ctx, 1u, max_vertices, &rounds, &cap);
     if (rc) return rc;
     const SceneView s = scene_view(ctx);
     const LightingRaw lr = to_raw(light);
@@ -1586,28 +1644,23 @@ int screen_wavefront(NanContext* ctx, float* out, uint32_t w, uint32_t h, uint32
     a.frame = frame;
     a.max_vertices = max_vertices;
     a.cached = cached != nullptr;
-    a.area_nee = (light->flags & 2u) != 0u;
     if (cached) a.cache = *cached;
     else memset(&a.cache, 0, sizeof(a.cache));
-    const Grid g = grid_for(ctx);
     unsigned long long* counters = ctx->d_counters;
     return wf_run(
-        ctx, st, 0, pixels, iters, cap, lr.ray_t_max,
+        ctx, st, 0, pixels, rounds, cap, lr.ray_t_max,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t count) {
             k_wf_screen_generate<<<(count + 127) / 128, 128, 0, st>>>(s, lr, a, S, q, first, count, counters);
         },
-        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl) {
-            k_wf_screen_shade<<<g.stream_blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
-        },
-        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, uint32_t* ctl_next) {
-            k_wf_screen_finalize<<<g.stream_blocks, 128, 0, st>>>(a, S, q, buf, ctl, ctl_next);
+        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, int blocks) {
+            k_wf_screen_stage<<<blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
         });
 }
 }  // namespace
 
 size_t probe_sample_bytes() { return sizeof(ProbeSample); }
 
-const void* wavefront_extend_kernel() { return reinterpret_cast<const void*>(&k_wf_extend<2, ManyScenes>); }
+const void* wavefront_extend_kernel() { return reinterpret_cast<const void*>(&k_wf_trace<ManyScenes>); }
 
 // The multi-scene probe batch on the wavefront: generate every (set, probe)
 // unit as one path, then n * max_bounces rounds of extend / shade / shadow /
@@ -1618,9 +1671,9 @@ int launch_batch_wavefront(NanContext* ctx, const void* sets, const uint32_t* pr
                            float t_max, cudaStream_t st) {
     if (total == 0) return NAN_OK;
     const uint32_t n = std::max(spp, 1u);
-    uint32_t iters = 0;
+    uint32_t rounds = 0;
     uint64_t cap = 0;
-    int rc = wf_plan(ctx, (uint64_t)n * std::max(max_bounces, 1u), &iters, &cap);
+    int rc = wf_plan(ctx, n, std::max(max_bounces, 1u), &rounds, &cap);
     if (rc) return rc;
     if (cap < total) {
         set_error("batch wavefront scratch holds fewer paths than the batch has probes");
@@ -1640,22 +1693,18 @@ int launch_batch_wavefront(NanContext* ctx, const void* sets, const uint32_t* pr
     m.units = total;
     m.samples = nullptr;
     const ManyScenes src{m.sets, set_of};
-    const Grid g = grid_for(ctx);
+    const Grid g = grid_for(ctx, total);
     WfState S;
     WfQueues q;
-    wf_carve(ctx, total, iters, S, q);
-    cudaError_t err = cudaMemsetAsync(q.ctl, 0, (size_t)(iters + 2) * 20 * sizeof(uint32_t), st);
+    wf_carve(ctx, total, rounds, S, q);
+    cudaError_t err = cudaMemsetAsync(q.ctl, 0, ctl_words(rounds) * sizeof(uint32_t), st);
     if (err != cudaSuccess) return cuda_fail(err, "batch wavefront control reset");
     k_wfb_probe_generate<<<(total + 127) / 128, 128, 0, st>>>(m, S, q, ctx->d_counters);
     ctx->launches++;
-    for (uint32_t it = 0; it < iters; ++it) {
-        const int buf = (int)(it & 1u);
-        uint32_t* ctl = q.ctl + 4u * it;
-        launch_extend(ctx, g.persistent_blocks, st, false, src, q.ext[buf], ctl, S);
-        k_wfb_probe_shade<<<g.stream_blocks, 128, 0, st>>>(m, S, q, buf, ctl);
-        launch_shadow(ctx, g.persistent_blocks, st, false, src, q.shd[buf], ctl, t_max, S);
-        k_wfb_probe_finalize<<<g.stream_blocks, 128, 0, st>>>(m, S, q, buf, ctl, ctl + 4);
-        ctx->launches += 4;
+    for (uint32_t it = 0; it < rounds; ++it) {
+        launch_trace(ctx, g.persistent_blocks, st, false, src, q, it, t_max, S);
+        k_wfb_probe_stage<<<g.stream_blocks, 128, 0, st>>>(m, S, q, (int)(it & 1u), q.ctl + kCtlWords * (it + 1u));
+        ctx->launches++;
     }
     return cuda_fail(cudaGetLastError(), "batch wavefront launch");
 }
@@ -1666,9 +1715,9 @@ int launch_batch_wavefront_independent(NanContext* ctx, const void* sets, const 
                                        float t_max, cudaStream_t st) {
     if (total == 0) return NAN_OK;
     const uint32_t n = std::max(spp, 1u);
-    uint32_t iters = 0;
+    uint32_t rounds = 0;
     uint64_t cap = 0;
-    int rc = wf_plan(ctx, std::max(max_bounces, 1u), &iters, &cap);
+    int rc = wf_plan(ctx, 1u, std::max(max_bounces, 1u), &rounds, &cap);
     if (rc) return rc;
     cap = std::min(cap, path_capacity);
     const uint64_t chunk_units = cap / n;
@@ -1688,27 +1737,23 @@ int launch_batch_wavefront_independent(NanContext* ctx, const void* sets, const 
     m.max_bounces = std::max(max_bounces, 1u);
     m.samples = static_cast<ProbeSample*>(samples);
     const ManyScenes src{m.sets, set_of};
-    const Grid g = grid_for(ctx);
+    const Grid g = grid_for(ctx, std::min<uint64_t>(chunk_units, total) * n);
     for (uint64_t ub = 0; ub < total; ub += chunk_units) {
         m.unit_begin = (uint32_t)ub;
         m.units = (uint32_t)std::min<uint64_t>(chunk_units, total - ub);
         const uint32_t paths = m.units * n;
         WfState S;
         WfQueues q;
-        wf_carve(ctx, paths, iters, S, q);
-        cudaError_t err = cudaMemsetAsync(q.ctl, 0, (size_t)(iters + 2) * 20 * sizeof(uint32_t), st);
+        wf_carve(ctx, paths, rounds, S, q);
+        cudaError_t err = cudaMemsetAsync(q.ctl, 0, ctl_words(rounds) * sizeof(uint32_t), st);
         if (err != cudaSuccess) return cuda_fail(err, "batch wavefront control reset");
         k_wfi_probe_generate<<<(paths + 127) / 128, 128, 0, st>>>(m, S, q);
-        for (uint32_t it = 0; it < iters; ++it) {
-            const int buf = (int)(it & 1u);
-            uint32_t* ctl = q.ctl + 4u * it;
-            launch_extend(ctx, g.persistent_blocks, st, false, src, q.ext[buf], ctl, S);
-            k_wfb_probe_shade<<<g.stream_blocks, 128, 0, st>>>(m, S, q, buf, ctl);
-            launch_shadow(ctx, g.persistent_blocks, st, false, src, q.shd[buf], ctl, t_max, S);
-            k_wfi_probe_finalize<<<g.stream_blocks, 128, 0, st>>>(m, S, q, buf, ctl, ctl + 4);
+        for (uint32_t it = 0; it < rounds; ++it) {
+            launch_trace(ctx, g.persistent_blocks, st, false, src, q, it, t_max, S);
+            k_wfi_probe_stage<<<g.stream_blocks, 128, 0, st>>>(m, S, q, (int)(it & 1u), q.ctl + kCtlWords * (it + 1u));
         }
         k_wfi_probe_fold<<<(m.units + 127) / 128, 128, 0, st>>>(m, ctx->d_counters);
-        ctx->launches += 2 + 4ull * iters;
+        ctx->launches += 2 + rounds;
     }
     return cuda_fail(cudaGetLastError(), "batch wavefront launch");
 }
@@ -1721,9 +1766,9 @@ int launch_trace_probes_wavefront(NanContext* ctx, float* values, uint32_t* coun
     end = std::min(end, probe_count);
     if (end <= begin) return NAN_OK;
     const uint32_t n = std::max(spp, 1u);
-    uint32_t iters = 0;
+    uint32_t rounds = 0;
     uint64_t cap = 0;
-    int rc = wf_plan(ctx, (uint64_t)n * std::max(max_bounces, 1u), &iters, &cap);
+    int rc = wf_plan(ctx, n, std::max(max_bounces, 1u), &rounds, &cap);
     if (rc) return rc;
     const SceneView s = scene_view(ctx);
     const LightingRaw lr = to_raw(light);
@@ -1737,18 +1782,14 @@ int launch_trace_probes_wavefront(NanContext* ctx, float* values, uint32_t* coun
     a.spp = spp;
     a.max_bounces = std::max(max_bounces, 1u);
     a.reset = reset;
-    const Grid g = grid_for(ctx);
     unsigned long long* counters = ctx->d_counters;
     return wf_run(
-        ctx, st, begin, end, iters, cap, lr.ray_t_max,
+        ctx, st, begin, end, rounds, cap, lr.ray_t_max,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t count) {
             k_wf_probe_generate<<<(count + 127) / 128, 128, 0, st>>>(s, lr, a, S, q, first, count, counters);
         },
-        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl) {
-            k_wf_probe_shade<<<g.stream_blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
-        },
-        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, uint32_t* ctl_next) {
-            k_wf_probe_finalize<<<g.stream_blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl, ctl_next);
+        [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, int blocks) {
+            k_wf_probe_stage<<<blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
         });
 }
 
