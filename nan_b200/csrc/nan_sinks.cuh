@@ -21,10 +21,10 @@ __device__ __forceinline__ void flush_tally(unsigned long long* counters, const 
     const uint32_t u = __reduce_add_sync(mask, units);
     const uint32_t p = __reduce_add_sync(mask, paths);
     if ((threadIdx.x & 31u) == (uint32_t)(__ffs(mask) - 1)) {
-        atomicAdd(counters + 0, (unsigned long long)e);
-        atomicAdd(counters + 1, (unsigned long long)s);
-        atomicAdd(counters + 2, (unsigned long long)u);
-        atomicAdd(counters + 3, (unsigned long long)p);
+        if (e) atomicAdd(counters + 0, (unsigned long long)e);
+        if (s) atomicAdd(counters + 1, (unsigned long long)s);
+        if (u) atomicAdd(counters + 2, (unsigned long long)u);
+        if (p) atomicAdd(counters + 3, (unsigned long long)p);
     }
 }
 

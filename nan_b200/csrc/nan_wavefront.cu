@@ -90,20 +90,85 @@ __device__ __forceinline__ uint32_t queue_slot(uint32_t* count, bool want) {
     return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
 }
 
-// Into the queue of the round that ctl belongs to: a path that traces on, or
-// one that waits to be closed.
-__device__ __forceinline__ void push_path(const WfQueues& q, int buf, uint32_t* ctl, uint32_t p) {
-    q.ext[buf][queue_slot(ctl + kExt, true)] = p;
+// Appends of a whole block to up to two queues: counts per warp, one atomic
+// per queue and block, then every thread its slot. Every thread of the block
+// calls it; two blocks of shared memory taken in turn need no further barrier
+// between calls. Appending by warp left the queues a patchwork of part warps
+// and made every warp wait for its turn at one address. By block, neighbouring
+// paths stay together in the queues (trace launches of the 200k-triangle texel
+// iteration 15.2 -> 14.3 ms, all of it 19.65 -> 18.78 ms) and a chunk of 2 M
+// screen paths is generated in 31 us (177 us; its queue needs no atomics at
+// all). Blocks of 128 threads; 256 take 18.87 ms.
+constexpr int kStageThreads = 128;
+
+struct BlockAppend {
+    uint32_t n[2][kStageThreads / 32];
+    uint32_t base[2];
+};
+
+__device__ __forceinline__ uint2 block_slots(BlockAppend& sh, uint32_t* count0, bool want0, uint32_t* count1,
+                                             bool want1) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const unsigned m0 = __ballot_sync(0xffffffffu, want0), m1 = __ballot_sync(0xffffffffu, want1);
+    if (lane == 0u) {
+        sh.n[0][warp] = (uint32_t)__popc(m0);
+        sh.n[1][warp] = (uint32_t)__popc(m1);
+    }
+    __syncthreads();
+    if (lane == 0u && warp < 2u) {
+        uint32_t sum = 0u;
+#pragma unroll
+        for (int w = 0; w < kStageThreads / 32; ++w) sum += sh.n[warp][w];
+        if (sum) sh.base[warp] = atomicAdd(warp ? count1 : count0, sum);
+    }
+    __syncthreads();
+    uint2 slot = make_uint2(sh.base[0], sh.base[1]);
+    for (uint32_t w = 0; w < warp; ++w) {
+        slot.x += sh.n[0][w];
+        slot.y += sh.n[1][w];
+    }
+    const unsigned below = (1u << lane) - 1u;
+    slot.x += (uint32_t)__popc(m0 & below);
+    slot.y += (uint32_t)__popc(m1 & below);
+    return slot;
 }
 
-__device__ __forceinline__ void push_close(const WfQueues& q, int buf, uint32_t* ctl, uint32_t p) {
-    q.ext[buf][q.cap - 1u - queue_slot(ctl + kClose, true)] = p;
+// What becomes of a path after a stage: it retires, traces on in the next
+// round, or waits there to be closed.
+enum PathNext { kRetire = 0, kWalk = 1, kAwaitClose = 2 };
+
+// The block's paths into the queue of the round that (buf, ctl) belong to:
+// the walking ones from the front, those to close from the back.
+__device__ __forceinline__ void push_paths(BlockAppend& sh, const WfQueues& q, int buf, uint32_t* ctl, uint32_t p,
+                                           PathNext next) {
+    const uint2 slot = block_slots(sh, ctl + kExt, next == kWalk, ctl + kClose, next == kAwaitClose);
+    if (next == kWalk) q.ext[buf][slot.x] = p;
+    if (next == kAwaitClose) q.ext[buf][q.cap - 1u - slot.y] = p;
 }
 
-// tmax 0: the ray runs to the scene's t_max
-__device__ __forceinline__ void push_shadow(const WfQueues& q, int buf, uint32_t* ctl, uint32_t p, f3 o, f3 d,
-                                            f3 c, uint32_t kind, float tmax = 0.0f) {
-    const uint32_t slot = queue_slot(ctl + kShd, true);
+// Slots in the shadow queue of the round that ctl belongs to.
+__device__ __forceinline__ uint32_t shadow_slots(BlockAppend& sh, uint32_t* ctl, bool want) {
+    return block_slots(sh, ctl + kShd, want, nullptr, false).x;
+}
+
+// Counters of the generated units (context counters 2 and 3), by block.
+__device__ __forceinline__ void count_units(unsigned long long* counters, bool unit, uint32_t paths) {
+    __shared__ uint32_t s_paths;
+    const int units = __syncthreads_count(unit);
+    if (threadIdx.x == 0u) s_paths = 0u;
+    __syncthreads();
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, unit ? paths : 0u);
+    if ((threadIdx.x & 31u) == 0u && sum) atomicAdd(&s_paths, sum);
+    __syncthreads();
+    if (threadIdx.x == 0u && units) {
+        atomicAdd(counters + 2, (unsigned long long)units);
+        atomicAdd(counters + 3, (unsigned long long)s_paths);
+    }
+}
+
+// A shadow ray at its slot; tmax 0: the ray runs to the scene's t_max.
+__device__ __forceinline__ void store_shadow(const WfQueues& q, int buf, uint32_t slot, uint32_t p, f3 o, f3 d, f3 c,
+                                             uint32_t kind, float tmax = 0.0f) {
     float4* e = q.shd[buf] + 3u * slot;
     e[0] = make_float4(o.x, o.y, o.z, __uint_as_float(p));
     e[1] = make_float4(d.x, d.y, d.z, __uint_as_float(kind));
@@ -455,13 +520,11 @@ __global__ void __launch_bounds__(128, 9) k_wf_shadow_refill(Src src, const floa
     flush_tally(counters, tally, 0u, 0u);
 }
 
-// The path-state stages (generate / shade / finalize) are bound by the
-// latency of their gathers (scene records, path state) more than by
-// bandwidth: their launch bound of 6 blocks of 128 per SM (at most 80
-// registers, no spills in the texel stages; they used 111-128) doubles the
-// resident warps. Measured on the 200k texel iteration: 5.54 -> 5.03 ms of
-// stage time per step. Shade and finalize take 8 blocks (64 registers, about
-// 112 B of spills each): 5.04 -> 4.92 ms; generate stays at 6.
+// The path-state stages are bound by the latency of their gathers (scene
+// records, path state) more than by bandwidth (10 long-scoreboard stalls an
+// issue, 2.3 to 2.5 TB/s of DRAM traffic): 6 blocks of 128 per SM (80
+// registers), the texel stage 8 (64 registers, 212 B of spills; 18.8 ms for
+// the 200k texel iteration against 19.3 with 6).
 // ---------------------------------------------------------------------------
 // Texture-space integrator stages (texture_space_path_tracer.slang:57-216).
 // ---------------------------------------------------------------------------
@@ -478,12 +541,12 @@ struct TexelArgs {
     int indirect_only;     // points mode: leave out the direct sun irradiance term
 };
 
-// Start sample k of the current side: sun irradiance shadow ray, first
-// direction (estimate_surface_irradiance, texture_space_path_tracer.slang:95-113).
-// its shadow ray goes to the round of (buf, ctl), the path to the next one.
-__device__ __forceinline__ void texel_start_sample(const SceneView& s, const LightParams& L, const WfState& st,
-                                                   const WfQueues& q, int buf, uint32_t* ctl, uint32_t p,
-                                                   uint32_t flags, Rng& rng, bool direct = true) {
+// Start sample k of the current side: sun irradiance shadow ray (at its slot
+// of the round's queue), first direction (estimate_surface_irradiance,
+// texture_space_path_tracer.slang:95-113).
+__device__ __forceinline__ PathNext texel_start_sample(const SceneView& s, const LightParams& L, const WfState& st,
+                                                       const WfQueues& q, int buf, uint32_t shadow_slot, uint32_t p,
+                                                       uint32_t flags, Rng& rng, bool direct) {
     const float4 sf = st.surf[p];
     const uint32_t inst = __float_as_uint(sf.z), prim = __float_as_uint(sf.w);
     f3 view = world_flat_normal(s, inst, prim);
@@ -493,7 +556,7 @@ __device__ __forceinline__ void texel_start_sample(const SceneView& s, const Lig
     const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
     const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
     // the two draws are taken either way, so the RNG streams stay aligned
-    if (direct) push_shadow(q, buf, ctl, p, sd.origin_front, l, L.illum * ndl, kKindSun);
+    if (direct) store_shadow(q, buf, shadow_slot, p, sd.origin_front, l, L.illum * ndl, kKindSun);
     st.si[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     st.rad[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     st.thp[p] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
@@ -501,156 +564,177 @@ __device__ __forceinline__ void texel_start_sample(const SceneView& s, const Lig
     float pdf;
     const f3 dir = cosine_sample_hemisphere(e0, e1, &pdf);
     flags &= ~(kFlagNoPath | kBounceMask);
-    if (pdf > 1e-6f) {
+    const bool path = pdf > 1e-6f;
+    if (path) {
         st.ro[p] = f4(sd.origin_front, 0.0f);
         st.rd[p] = f4(sd.frame.to_global(dir), L.t_max);
         st.zpdf[p] = make_float2(fabsf(dir.z), pdf);
-        push_path(q, buf ^ 1, ctl + kCtlWords, p);
     } else {
         flags |= kFlagNoPath;
-        push_close(q, buf ^ 1, ctl + kCtlWords, p);
     }
     st.flags[p] = flags;
+    return path ? kWalk : kAwaitClose;
 }
 
-__global__ void __launch_bounds__(128, 6) k_wf_texel_generate(SceneView s, LightingRaw lraw, TexelArgs a, WfState st,
-                                                           WfQueues q, uint32_t begin, uint32_t count,
-                                                           unsigned long long* counters) {
+__global__ void __launch_bounds__(kStageThreads, 6) k_wf_texel_generate(SceneView s, LightingRaw lraw, TexelArgs a,
+                                                                     WfState st, WfQueues q, uint32_t begin,
+                                                                     uint32_t count, unsigned long long* counters) {
+    __shared__ BlockAppend sh[2];
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= count) return;
     TexelSurface ts;
     Rng rng(0u, 0u, 0u);
-    if (!texel_surface(s, a.mc, begin + p, a.iteration, a.n, &ts, &rng)) return;
-    const LightParams L = make_light(lraw);
-    st.unit[p] = begin + p;
-    st.surf[p] = make_float4(ts.b1, ts.b2, __uint_as_float(ts.inst), __uint_as_float(ts.prim));
-    st.irr[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const uint32_t flags = (ts.side.y & 1u) ? kFlagTwoSided : 0u;
-    texel_start_sample(s, L, st, q, 1, q.ctl, p, flags, rng);
-    st.rng[p] = rng.state;
-    RayTally none{0u, 0u};
-    flush_tally(counters, none, 1u, (ts.side.y & 1u) ? 2u * a.n : a.n);
+    const bool unit = p < count && texel_surface(s, a.mc, begin + p, a.iteration, a.n, &ts, &rng);
+    const bool two_sided = unit && (ts.side.y & 1u);
+    const uint32_t slot = shadow_slots(sh[0], q.ctl, unit);
+    PathNext next = kRetire;
+    if (unit) {
+        const LightParams L = make_light(lraw);
+        st.unit[p] = begin + p;
+        st.surf[p] = make_float4(ts.b1, ts.b2, __uint_as_float(ts.inst), __uint_as_float(ts.prim));
+        st.irr[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        next = texel_start_sample(s, L, st, q, 1, slot, p, two_sided ? kFlagTwoSided : 0u, rng, true);
+        st.rng[p] = rng.state;
+    }
+    push_paths(sh[1], q, 0, q.ctl + kCtlWords, p, next);
+    count_units(counters, unit, two_sided ? 2u * a.n : a.n);
 }
 
 // Surface points instead of texels: the same estimator at the listed points,
 // with RNG(index, 0xFFFFFFFF, iteration * n) and view = the flat normal,
 // negated for the back side.
-__global__ void __launch_bounds__(128) k_wf_point_generate(SceneView s, LightingRaw lraw, TexelArgs a, WfState st,
-                                                           WfQueues q, uint32_t begin, uint32_t count,
-                                                           unsigned long long* counters) {
+__global__ void __launch_bounds__(kStageThreads) k_wf_point_generate(SceneView s, LightingRaw lraw, TexelArgs a,
+                                                                  WfState st, WfQueues q, uint32_t begin,
+                                                                  uint32_t count, unsigned long long* counters) {
+    __shared__ BlockAppend sh[2];
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= count) return;
     const uint32_t u = begin + p;
-    const float4 pt = a.points[u];
-    const uint32_t inst = __float_as_uint(pt.z), primw = __float_as_uint(pt.w);
-    const uint32_t prim = primw & 0x7fffffffu;
-    if (inst == 0xffffffffu || !valid_prim(s, inst, prim)) {
-        if (inst != 0xffffffffu) atomicOr(s.status, kStatusBadRecord);
-        a.point_out[u] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-        return;
+    float4 pt = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    bool unit = p < count;
+    uint32_t inst = 0u, primw = 0u;
+    if (unit) {
+        pt = a.points[u];
+        inst = __float_as_uint(pt.z);
+        primw = __float_as_uint(pt.w);
+        if (inst == 0xffffffffu || !valid_prim(s, inst, primw & 0x7fffffffu)) {
+            if (inst != 0xffffffffu) atomicOr(s.status, kStatusBadRecord);
+            a.point_out[u] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+            unit = false;
+        }
     }
-    const LightParams L = make_light(lraw);
-    Rng rng(u, 0xffffffffu, a.iteration * a.n);
-    st.unit[p] = u;
-    st.surf[p] = make_float4(pt.x, pt.y, __uint_as_float(inst), __uint_as_float(prim));
-    st.irr[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    texel_start_sample(s, L, st, q, 1, q.ctl, p, (primw >> 31) ? kFlagBack : 0u, rng, !a.indirect_only);
-    st.rng[p] = rng.state;
-    RayTally none{0u, 0u};
-    flush_tally(counters, none, 1u, a.n);
+    const uint32_t slot = shadow_slots(sh[0], q.ctl, unit && !a.indirect_only);
+    PathNext next = kRetire;
+    if (unit) {
+        const LightParams L = make_light(lraw);
+        Rng rng(u, 0xffffffffu, a.iteration * a.n);
+        st.unit[p] = u;
+        st.surf[p] = make_float4(pt.x, pt.y, __uint_as_float(inst), __uint_as_float(primw & 0x7fffffffu));
+        st.irr[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        next = texel_start_sample(s, L, st, q, 1, slot, p, (primw >> 31) ? kFlagBack : 0u, rng, !a.indirect_only);
+        st.rng[p] = rng.state;
+    }
+    push_paths(sh[1], q, 0, q.ctl + kCtlWords, p, next);
+    count_units(counters, unit, a.n);
 }
 
 // One bounce of trace_radiance (texture_space_path_tracer.slang:60-83) for the
 // paths whose hit the trace found, and the closing of finished samples: si +=
 // L*|z|/pdf, irr += si, next sample / side, or the running-mean store
 // (texture_space_path_tracer.slang:111-138, 203-215).
-__global__ void __launch_bounds__(128, 8) k_wf_texel_stage(SceneView s, LightingRaw lraw, TexelArgs a, WfState st,
-                                                        WfQueues q, int buf, uint32_t* ctl) {
+__global__ void __launch_bounds__(kStageThreads, 8) k_wf_texel_stage(SceneView s, LightingRaw lraw, TexelArgs a,
+                                                                  WfState st, WfQueues q, int buf, uint32_t* ctl) {
+    __shared__ BlockAppend sh[2];
     const uint32_t walking = *(volatile uint32_t*)(ctl + kExt);
     const uint32_t count = walking + *(volatile uint32_t*)(ctl + kClose);
-    uint32_t* ctl_next = ctl + kCtlWords;
     const LightParams L = make_light(lraw);
-    const int nbuf = buf ^ 1;
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
-        uint32_t flags = st.flags[p];
-        f3 rad = xyz(st.rad[p]);
-        if (idx < walking) {
-            const float4 h = st.hit[p];
+    for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
+        const uint32_t idx = base + threadIdx.x;
+        const bool live = idx < count;
+        uint32_t p = 0u, flags = 0u, flat = 0xffffffffu;
+        float4 h = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (live) {
+            p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
+            flags = st.flags[p];
+            if (idx < walking) {
+                h = st.hit[p];
+                flat = __float_as_uint(h.x);
+            }
+        }
+        const bool at_hit = flat != 0xffffffffu;
+        const bool more_samples = (flags >> kSampleShift) + 1u < a.n;
+        const bool to_back = !more_samples && !a.point_out && !(flags & kFlagBack) && (flags & kFlagTwoSided);
+        const bool starts = live && !at_hit && (more_samples || to_back);
+        const uint32_t slot = shadow_slots(sh[0], ctl, at_hit || (starts && (to_back || !a.indirect_only)));
+        PathNext next = kRetire;
+        if (at_hit) {
             const f3 d = xyz(st.rd[p]);
-            f3 thp = xyz(st.thp[p]);
-            const uint32_t flat = __float_as_uint(h.x);
-            if (flat != 0xffffffffu) {
+            f3 thp = xyz(st.thp[p]), rad = xyz(st.rad[p]);
+            Rng rng(0u, 0u, 0u);
+            rng.state = st.rng[p];
+            const uint2 ref = __ldg(s.tri_refs + flat);
+            const Shading sd = shading_data(s, ref.x, ref.y, h.z, h.w, -d);
+            rad = rad + thp * sd.emissive;
+            const float u0 = rng.next_1d(), u1 = rng.next_1d();
+            const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
+            const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
+            const f3 f = sd.diffuse * kInvPi;
+            store_shadow(q, buf, slot, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
+            const float e0 = rng.next_1d(), e1 = rng.next_1d();
+            float pdf;
+            const f3 sdir = cosine_sample_hemisphere(e0, e1, &pdf);
+            next = kAwaitClose;
+            if (pdf > 1e-6f) {
+                const uint32_t bounce = ((flags & kBounceMask) >> kBounceShift) + 1u;
+                flags = (flags & ~kBounceMask) | (bounce << kBounceShift);
+                if (bounce < a.max_bounces) {
+                    next = kWalk;
+                    thp = thp * ((f * fabsf(sdir.z)) / pdf);
+                    st.ro[p] = f4(sd.origin_front, 0.0f);
+                    st.rd[p] = f4(sd.frame.to_global(sdir), L.t_max);
+                    st.thp[p] = f4(thp, 0.0f);
+                }
+            }
+            st.rad[p] = f4(rad, 0.0f);
+            st.rng[p] = rng.state;
+            st.flags[p] = flags;
+        } else if (live) {
+            f3 si = xyz(st.si[p]);
+            if (!(flags & kFlagNoPath)) {
+                f3 rad = xyz(st.rad[p]);
+                if (idx < walking) rad = rad + xyz(st.thp[p]) * sky_radiance(L, xyz(st.rd[p]));
+                const float2 zp = st.zpdf[p];
+                si = si + ((rad * zp.x) / zp.y);
+            }
+            f3 irr = xyz(st.irr[p]) + si;
+            if (!more_samples) {
+                const uint32_t u = st.unit[p];
+                if (a.point_out) {
+                    a.point_out[u] = f4(irr / (float)a.n, 0.0f);
+                } else {
+                    // side complete: running mean into its slot
+                    const uint32_t inst = __float_as_uint(st.surf[p].z);
+                    const uint4 info = __ldg(a.mc.instance_infos + inst);
+                    const uint2 side = __ldg(a.mc.side_infos + inst);
+                    const uint32_t global_texel = info.z + (u - __ldg(a.mc.surface_prefix + inst));
+                    const uint32_t to = (flags & kFlagBack) ? side.x + (global_texel - info.z) : global_texel;
+                    if (to < a.mc.payload_count)
+                        store_running_mean(a.slots, to, irr / (float)a.n, a.reset, a.mc.compensation);
+                    else
+                        atomicOr(s.status, 2u);
+                }
+                irr = mk3(0.0f, 0.0f, 0.0f);
+            }
+            if (starts) {
+                const uint32_t low = flags & ((1u << kSampleShift) - 1u);
+                const uint32_t k = (flags >> kSampleShift) + 1u;
+                st.irr[p] = f4(irr, 0.0f);
                 Rng rng(0u, 0u, 0u);
                 rng.state = st.rng[p];
-                const uint2 ref = __ldg(s.tri_refs + flat);
-                const Shading sd = shading_data(s, ref.x, ref.y, h.z, h.w, -d);
-                rad = rad + thp * sd.emissive;
-                const float u0 = rng.next_1d(), u1 = rng.next_1d();
-                const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
-                const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
-                const f3 f = sd.diffuse * kInvPi;
-                push_shadow(q, buf, ctl, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
-                const float e0 = rng.next_1d(), e1 = rng.next_1d();
-                float pdf;
-                const f3 sdir = cosine_sample_hemisphere(e0, e1, &pdf);
-                bool ended = true;
-                if (pdf > 1e-6f) {
-                    const uint32_t bounce = ((flags & kBounceMask) >> kBounceShift) + 1u;
-                    flags = (flags & ~kBounceMask) | (bounce << kBounceShift);
-                    ended = bounce >= a.max_bounces;
-                    if (!ended) {
-                        thp = thp * ((f * fabsf(sdir.z)) / pdf);
-                        st.ro[p] = f4(sd.origin_front, 0.0f);
-                        st.rd[p] = f4(sd.frame.to_global(sdir), L.t_max);
-                        st.thp[p] = f4(thp, 0.0f);
-                    }
-                }
-                st.rad[p] = f4(rad, 0.0f);
+                next = texel_start_sample(s, L, st, q, buf, slot, p, to_back ? (low | kFlagBack) : (low | (k << kSampleShift)),
+                                          rng, to_back || !a.indirect_only);
                 st.rng[p] = rng.state;
-                st.flags[p] = flags;
-                if (ended) push_close(q, nbuf, ctl_next, p);
-                else push_path(q, nbuf, ctl_next, p);
-                continue;
             }
-            rad = rad + thp * sky_radiance(L, d);
         }
-        f3 si = xyz(st.si[p]);
-        if (!(flags & kFlagNoPath)) {
-            const float2 zp = st.zpdf[p];
-            si = si + ((rad * zp.x) / zp.y);
-        }
-        f3 irr = xyz(st.irr[p]) + si;
-        uint32_t k = (flags >> kSampleShift) + 1u;
-        Rng rng(0u, 0u, 0u);
-        if (k < a.n) {
-            flags = (flags & ((1u << kSampleShift) - 1u)) | (k << kSampleShift);
-            st.irr[p] = f4(irr, 0.0f);
-            rng.state = st.rng[p];
-            texel_start_sample(s, L, st, q, buf, ctl, p, flags, rng, !a.indirect_only);
-            st.rng[p] = rng.state;
-            continue;
-        }
-        const uint32_t u = st.unit[p];
-        if (a.point_out) {
-            a.point_out[u] = f4(irr / (float)a.n, 0.0f);
-            continue;
-        }
-        // side complete: running mean into its slot
-        const uint32_t inst = __float_as_uint(st.surf[p].z);
-        const uint4 info = __ldg(a.mc.instance_infos + inst);
-        const uint2 side = __ldg(a.mc.side_infos + inst);
-        const uint32_t global_texel = info.z + (u - __ldg(a.mc.surface_prefix + inst));
-        const uint32_t slot = (flags & kFlagBack) ? side.x + (global_texel - info.z) : global_texel;
-        if (slot < a.mc.payload_count) store_running_mean(a.slots, slot, irr / (float)a.n, a.reset, a.mc.compensation);
-        else atomicOr(s.status, 2u);
-        if (!(flags & kFlagBack) && (flags & kFlagTwoSided)) {
-            flags = (flags & ((1u << kSampleShift) - 1u)) | kFlagBack;
-            st.irr[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            rng.state = st.rng[p];
-            texel_start_sample(s, L, st, q, buf, ctl, p, flags, rng);
-            st.rng[p] = rng.state;
-        }
+        push_paths(sh[1], q, buf ^ 1, ctl + kCtlWords, p, next);
     }
 }
 
@@ -691,7 +775,7 @@ struct ScreenArgs {
     CachedArgs cache;
 };
 
-__global__ void __launch_bounds__(128) k_wf_screen_generate(SceneView s, LightingRaw lraw, ScreenArgs a, WfState st,
+__global__ void __launch_bounds__(kStageThreads) k_wf_screen_generate(SceneView s, LightingRaw lraw, ScreenArgs a, WfState st,
                                                             WfQueues q, uint32_t begin, uint32_t count,
                                                             unsigned long long* counters) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -722,9 +806,13 @@ __global__ void __launch_bounds__(128) k_wf_screen_generate(SceneView s, Lightin
     st.rad[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     st.si[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     st.zpdf[p] = make_float2(0.0f, 1.0f);
-    push_path(q, 0, q.ctl + kCtlWords, p);
-    RayTally none{0u, 0u};
-    flush_tally(counters, none, 1u, 1u);
+    // every pixel of the chunk is a path: queue and counters need no appends
+    q.ext[0][p] = p;
+    if (p == 0u) {
+        q.ctl[kCtlWords + kExt] = count;
+        atomicAdd(counters + 2, (unsigned long long)count);
+        atomicAdd(counters + 3, (unsigned long long)count);
+    }
 }
 
 // The area-light term of the previous vertex (kept apart by the shadow stage)
@@ -735,111 +823,130 @@ __device__ __forceinline__ f3 fold_area_term(const WfState& st, uint32_t p, f3 r
     return rad + xyz(a);
 }
 
-__global__ void __launch_bounds__(128, 6) k_wf_screen_stage(SceneView s, LightingRaw lraw, ScreenArgs a, WfState st,
-                                                         WfQueues q, int buf, uint32_t* ctl) {
+// Shades the hit of path p (path_tracer.slang:54-82); its sun ray goes to
+// `slot` of the round's shadow queue.
+__device__ __forceinline__ PathNext screen_shade_path(const SceneView& s, const LightParams& L, const ScreenArgs& a,
+                                                      const WfState& st, const WfQueues& q, int buf, uint32_t* ctl,
+                                                      uint32_t p, uint32_t flags, uint32_t vertex, float4 h,
+                                                      bool at_cache, uint32_t slot) {
+    const f3 d = xyz(st.rd[p]);
+    f3 thp = xyz(st.thp[p]), rad = xyz(st.rad[p]);
+    if (L.area_nee) rad = fold_area_term(st, p, rad);
+    const uint32_t flat = __float_as_uint(h.x);
+    Rng rng(0u, 0u, 0u);
+    rng.state = st.rng[p];
+    const uint2 ref = __ldg(s.tri_refs + flat);
+    const Shading sd = shading_data(s, ref.x, ref.y, h.z, h.w, -d);
+    if (L.area_nee && vertex > 0u)
+        rad = rad + thp * (sd.emissive * area_mis_weight(s, sd.emissive, sd.face_normal, d, h.y, st.zpdf[p].y));
+    else
+        rad = rad + thp * sd.emissive;
+    const f3 f = sd.diffuse * kInvPi;
+    if (at_cache) {
+        // the rest of the path is the cache's irradiance at this point;
+        // at vertex 0 the sun is still sampled (NEE) and the cache holds
+        // the indirect irradiance only
+        if (vertex == 0u) {
+            const float u0 = rng.next_1d(), u1 = rng.next_1d();
+            const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
+            const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
+            store_shadow(q, buf, slot, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
+        }
+        const uint32_t pixel = st.unit[p];
+        const uint32_t qi = queue_slot(a.cache.query_count, true);
+        const float4 q0 = make_float4(sd.position.x, sd.position.y, sd.position.z, __uint_as_float(pixel));
+        const float4 q1 = f4(sd.frame.n, 0.0f);
+        a.cache.queries[2u * qi] = q0;
+        a.cache.queries[2u * qi + 1u] = q1;
+        a.cache.weights[qi] = f4(thp * f, 0.0f);
+        const uint32_t P = a.width * a.height;
+        const uint32_t rel = pixel >= a.cache.train_offset ? pixel - a.cache.train_offset
+                                                           : pixel + (P - a.cache.train_offset);
+        const uint32_t ti = (uint32_t)(((uint64_t)rel * a.cache.train_inverse) % P);
+        if (ti < a.cache.train_count) {
+            // a back side exists for double-sided materials only (as texel back slots)
+            const bool two = (__float_as_uint(__ldg(tri_refs(s, ref.x, ref.y).mat + 3)) & 1u) != 0u;
+            const bool back = two && dot3(world_flat_normal(s, ref.x, ref.y), -d) < 0.0f;
+            a.cache.train_points[ti] = make_float4(h.z, h.w, __uint_as_float(ref.x),
+                                                   __uint_as_float(ref.y | (back ? 0x80000000u : 0u)));
+            a.cache.train_queries[2u * ti] = q0;
+            a.cache.train_queries[2u * ti + 1u] = q1;
+        }
+        if (vertex == 0u) {
+            st.rad[p] = f4(rad, 0.0f);
+            return kAwaitClose;  // its sun ray is in flight
+        }
+        if (L.area_nee) rad = rad + mk3(0.0f, 0.0f, 0.0f);
+        a.out[pixel] = f4(rad, 1.0f);
+        return kRetire;
+    }
+    const float u0 = rng.next_1d(), u1 = rng.next_1d();
+    const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
+    const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
+    store_shadow(q, buf, slot, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
+    // light reached from this vertex lies on the next one: sampled only
+    // where that vertex exists, so both strategies cover the same paths
+    if (L.area_nee && vertex + 1u < a.max_vertices) {
+        const float us = rng.next_1d(), a0 = rng.next_1d(), a1 = rng.next_1d();
+        const AreaSample as = area_nee_sample(s, sd, us, a0, a1);
+        if (as.valid)
+            store_shadow(q, buf, queue_slot(ctl + kShd, true), p, sd.origin_front, as.dir, thp * as.contrib, kKindSun,
+                         as.tmax);
+    }
+    const float e0 = rng.next_1d(), e1 = rng.next_1d();
+    float pdf;
+    const f3 wo = cosine_sample_hemisphere(e0, e1, &pdf);
+    pdf = maxf(pdf, 1e-6f);
+    st.zpdf[p] = make_float2(0.0f, pdf);
+    thp = thp * ((f * fabsf(wo.z)) / pdf);
+    st.ro[p] = f4(sd.origin_front, 0.0f);
+    st.rd[p] = f4(sd.frame.to_global(wo), L.t_max);
+    const uint32_t next = vertex + 1u;
+    st.thp[p] = f4(thp, 0.0f);
+    st.rad[p] = f4(rad, 0.0f);
+    st.rng[p] = rng.state;
+    st.flags[p] = (flags & ~kBounceMask) | (next << kBounceShift);
+    return next >= a.max_vertices ? kAwaitClose : kWalk;
+}
+
+__global__ void __launch_bounds__(kStageThreads, 6) k_wf_screen_stage(SceneView s, LightingRaw lraw, ScreenArgs a,
+                                                                   WfState st, WfQueues q, int buf, uint32_t* ctl) {
+    __shared__ BlockAppend sh[2];
     const uint32_t walking = *(volatile uint32_t*)(ctl + kExt);
     const uint32_t count = walking + *(volatile uint32_t*)(ctl + kClose);
-    uint32_t* ctl_next = ctl + kCtlWords;
-    const int nbuf = buf ^ 1;
     const LightParams L = make_light(lraw);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
-        if (idx >= walking) {
-            f3 r = xyz(st.rad[p]);
-            if (L.area_nee) r = r + xyz(st.si[p]);
-            a.out[st.unit[p]] = f4(r, 1.0f);
-            continue;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
+        const uint32_t idx = base + threadIdx.x;
+        const bool live = idx < count;
+        uint32_t p = 0u, flags = 0u, flat = 0xffffffffu;
+        float4 h = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (live) p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
+        if (idx < walking) {
+            flags = st.flags[p];
+            h = st.hit[p];
+            flat = __float_as_uint(h.x);
         }
-        const uint32_t flags = st.flags[p];
-        const float4 h = st.hit[p];
-        const f3 d = xyz(st.rd[p]);
-        f3 thp = xyz(st.thp[p]), rad = xyz(st.rad[p]);
-        if (L.area_nee) rad = fold_area_term(st, p, rad);
         const uint32_t vertex = (flags & kBounceMask) >> kBounceShift;
-        const uint32_t flat = __float_as_uint(h.x);
-        if (flat == 0xffffffffu) {
-            f3 sky = sky_radiance(L, d);
-            if (vertex == 0u && L.sun_disk) sky = sky + sun_disk(L, d);
-            rad = rad + thp * sky;
-            // (an area-light term of zero: the last vertex's is in rad)
-            if (L.area_nee) rad = rad + mk3(0.0f, 0.0f, 0.0f);
-            a.out[st.unit[p]] = f4(rad, 1.0f);
-            continue;
-        }
-        Rng rng(0u, 0u, 0u);
-        rng.state = st.rng[p];
-        const uint2 ref = __ldg(s.tri_refs + flat);
-        const Shading sd = shading_data(s, ref.x, ref.y, h.z, h.w, -d);
-        if (L.area_nee && vertex > 0u)
-            rad = rad + thp * (sd.emissive * area_mis_weight(s, sd.emissive, sd.face_normal, d, h.y, st.zpdf[p].y));
-        else
-            rad = rad + thp * sd.emissive;
-        const f3 f = sd.diffuse * kInvPi;
-        if (a.cached && vertex == a.cache.vertex) {
-            // the rest of the path is the cache's irradiance at this point;
-            // at vertex 0 the sun is still sampled (NEE) and the cache holds
-            // the indirect irradiance only
-            if (vertex == 0u) {
-                const float u0 = rng.next_1d(), u1 = rng.next_1d();
-                const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
-                const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
-                push_shadow(q, buf, ctl, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
-            }
-            const uint32_t pixel = st.unit[p];
-            const uint32_t qi = queue_slot(a.cache.query_count, true);
-            const float4 q0 = make_float4(sd.position.x, sd.position.y, sd.position.z, __uint_as_float(pixel));
-            const float4 q1 = f4(sd.frame.n, 0.0f);
-            a.cache.queries[2u * qi] = q0;
-            a.cache.queries[2u * qi + 1u] = q1;
-            a.cache.weights[qi] = f4(thp * f, 0.0f);
-            const uint32_t P = a.width * a.height;
-            const uint32_t rel = pixel >= a.cache.train_offset ? pixel - a.cache.train_offset
-                                                               : pixel + (P - a.cache.train_offset);
-            const uint32_t ti = (uint32_t)(((uint64_t)rel * a.cache.train_inverse) % P);
-            if (ti < a.cache.train_count) {
-                // a back side exists for double-sided materials only (as texel back slots)
-                const bool two = (__float_as_uint(__ldg(tri_refs(s, ref.x, ref.y).mat + 3)) & 1u) != 0u;
-                const bool back = two && dot3(world_flat_normal(s, ref.x, ref.y), -d) < 0.0f;
-                a.cache.train_points[ti] = make_float4(h.z, h.w, __uint_as_float(ref.x),
-                                                       __uint_as_float(ref.y | (back ? 0x80000000u : 0u)));
-                a.cache.train_queries[2u * ti] = q0;
-                a.cache.train_queries[2u * ti + 1u] = q1;
-            }
-            if (vertex == 0u) {
-                st.rad[p] = f4(rad, 0.0f);
-                push_close(q, nbuf, ctl_next, p);  // its sun ray is in flight
-            } else {
+        const bool at_hit = flat != 0xffffffffu;
+        const bool at_cache = at_hit && a.cached && vertex == a.cache.vertex;
+        const uint32_t slot = shadow_slots(sh[0], ctl, at_hit && !(at_cache && vertex > 0u));
+        PathNext next = kRetire;
+        if (at_hit) {
+            next = screen_shade_path(s, L, a, st, q, buf, ctl, p, flags, vertex, h, at_cache, slot);
+        } else if (live) {
+            f3 rad = xyz(st.rad[p]);
+            // the last vertex's area-light term follows its sun term
+            if (L.area_nee) rad = rad + xyz(st.si[p]);
+            if (idx < walking) {
+                const f3 d = xyz(st.rd[p]);
+                f3 sky = sky_radiance(L, d);
+                if (vertex == 0u && L.sun_disk) sky = sky + sun_disk(L, d);
+                rad = rad + xyz(st.thp[p]) * sky;
                 if (L.area_nee) rad = rad + mk3(0.0f, 0.0f, 0.0f);
-                a.out[pixel] = f4(rad, 1.0f);
             }
-            continue;
+            a.out[st.unit[p]] = f4(rad, 1.0f);
         }
-        const float u0 = rng.next_1d(), u1 = rng.next_1d();
-        const f3 l = sample_cone_direction(L.sun_dir, L.cos_half, u0, u1);
-        const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
-        push_shadow(q, buf, ctl, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee);
-        // light reached from this vertex lies on the next one: sampled only
-        // where that vertex exists, so both strategies cover the same paths
-        if (L.area_nee && vertex + 1u < a.max_vertices) {
-            const float us = rng.next_1d(), a0 = rng.next_1d(), a1 = rng.next_1d();
-            const AreaSample as = area_nee_sample(s, sd, us, a0, a1);
-            if (as.valid) push_shadow(q, buf, ctl, p, sd.origin_front, as.dir, thp * as.contrib, kKindSun, as.tmax);
-        }
-        const float e0 = rng.next_1d(), e1 = rng.next_1d();
-        float pdf;
-        const f3 wo = cosine_sample_hemisphere(e0, e1, &pdf);
-        pdf = maxf(pdf, 1e-6f);
-        st.zpdf[p] = make_float2(0.0f, pdf);
-        thp = thp * ((f * fabsf(wo.z)) / pdf);
-        st.ro[p] = f4(sd.origin_front, 0.0f);
-        st.rd[p] = f4(sd.frame.to_global(wo), L.t_max);
-        const uint32_t next = vertex + 1u;
-        st.thp[p] = f4(thp, 0.0f);
-        st.rad[p] = f4(rad, 0.0f);
-        st.rng[p] = rng.state;
-        st.flags[p] = (flags & ~kBounceMask) | (next << kBounceShift);
-        if (next >= a.max_vertices) push_close(q, nbuf, ctl_next, p);
-        else push_path(q, nbuf, ctl_next, p);
+        push_paths(sh[1], q, buf ^ 1, ctl + kCtlWords, p, next);
     }
 }
 
@@ -863,11 +970,9 @@ __device__ __forceinline__ Shading probe_surface(const SceneView& s, const Probe
     return shading_data(s, __float_as_uint(surf.z), __float_as_uint(surf.w), surf.x, surf.y, view);
 }
 
-// One cosine sample around the face normal (no sun at the probe itself); the
-// path goes to the queue of the round of (buf, ctl).
-__device__ __forceinline__ void probe_start_sample(const SceneView& s, const LightParams& L, const ProbeArgs& a,
-                                                   const WfState& st, const WfQueues& q, int buf, uint32_t* ctl,
-                                                   uint32_t p, uint32_t flags, Rng& rng) {
+// One cosine sample around the face normal (no sun at the probe itself).
+__device__ __forceinline__ PathNext probe_start_sample(const SceneView& s, const LightParams& L, const ProbeArgs& a,
+                                                       const WfState& st, uint32_t p, uint32_t flags, Rng& rng) {
     const float4 surf = st.surf[p];
     const Shading sd = probe_surface(s, a, st.unit[p], surf);
     const float kr = st.si[p].w;
@@ -887,23 +992,22 @@ __device__ __forceinline__ void probe_start_sample(const SceneView& s, const Lig
         b.x = 0u;
         b.w = radial_texel(dir);
         st.pb[p] = b;
-        push_path(q, buf, ctl, p);
     } else {
         flags |= kFlagNoPath;
-        push_close(q, buf, ctl, p);
     }
     st.flags[p] = flags;
+    return (flags & kFlagNoPath) ? kAwaitClose : kWalk;
 }
 
 // Per-path bodies of the probe stages, shared by the one-scene kernels and the
 // multi-scene batch kernels (which look up the path's probe set first).
-__device__ __forceinline__ bool probe_generate_path(const SceneView& s, const LightParams& L, const ProbeArgs& a,
-                                                    const WfState& st, const WfQueues& q, uint32_t probe, uint32_t p) {
+__device__ __forceinline__ PathNext probe_generate_path(const SceneView& s, const LightParams& L, const ProbeArgs& a,
+                                                        const WfState& st, uint32_t probe, uint32_t p) {
     const uint4 meta = __ldg(reinterpret_cast<const uint4*>(a.probes) + 3u * probe + 2u);
     const uint32_t inst = meta.w >> 8;
     if (inst >= a.probe_instance_count || !valid_prim(s, inst, meta.x)) {
         atomicOr(s.status, kStatusBadRecord);
-        return false;
+        return kRetire;
     }
     const float4 params = __ldg(a.pinst + 3u * inst + 2u);
     st.unit[p] = probe;
@@ -918,31 +1022,34 @@ __device__ __forceinline__ bool probe_generate_path(const SceneView& s, const Li
     if (a.reset)
         for (int t = 0; t < 16; ++t) a.out.radial[16u * probe + (uint32_t)t] = 0u;
     Rng rng(probe, inst, a.iteration * a.n);
-    probe_start_sample(s, L, a, st, q, 0, q.ctl + kCtlWords, p, 0u, rng);
+    const PathNext next = probe_start_sample(s, L, a, st, p, 0u, rng);
     st.rng[p] = rng.state;
-    return true;
+    return next;
 }
 
-// Shades the path's hit. False when the path has left the scene: its sample
-// has no shadow ray in flight and can be closed.
-__device__ __forceinline__ bool probe_shade_path(const SceneView& s, const LightParams& L, const ProbeArgs& a,
-                                                 const WfState& st, const WfQueues& q, int buf, uint32_t* ctl,
-                                                 uint32_t p) {
+// The path leaves the scene: its sample can be closed.
+__device__ __forceinline__ void probe_miss_path(const LightParams& L, const WfState& st, uint32_t p) {
+    const uint32_t bounce = (st.flags[p] & kBounceMask) >> kBounceShift;
+    if (bounce == 0u) {
+        float4 pa = st.pa[p];
+        pa.w = 2.0f * st.si[p].w;
+        st.pa[p] = pa;
+    }
+    st.rad[p] = f4(xyz(st.rad[p]) + xyz(st.thp[p]) * sky_radiance(L, xyz(st.rd[p])), 0.0f);
+}
+
+// Shades the path's hit; its sun ray goes to `slot` of the round's shadow
+// queue.
+__device__ __forceinline__ PathNext probe_shade_path(const SceneView& s, const LightParams& L, const ProbeArgs& a,
+                                                     const WfState& st, const WfQueues& q, int buf, uint32_t slot,
+                                                     uint32_t p, float4 h) {
     uint32_t flags = st.flags[p];
-    const float4 h = st.hit[p];
     const f3 d = xyz(st.rd[p]);
     f3 thp = xyz(st.thp[p]), rad = xyz(st.rad[p]);
     float4 pa = st.pa[p];  // src inst, src prim, src offset, first hit
     const uint32_t bounce = (flags & kBounceMask) >> kBounceShift;
     const float radial_max = 2.0f * st.si[p].w;
     const uint32_t flat = __float_as_uint(h.x);
-    if (flat == 0xffffffffu) {
-        if (bounce == 0u) pa.w = radial_max;
-        rad = rad + thp * sky_radiance(L, d);
-        st.pa[p] = pa;
-        st.rad[p] = f4(rad, 0.0f);
-        return false;
-    }
     if (bounce == 0u) pa.w = minf(h.y, radial_max);
     const uint2 ref = __ldg(s.tri_refs + flat);
     const uint32_t src_inst = __float_as_uint(pa.x), src_prim = __float_as_uint(pa.y);
@@ -963,7 +1070,7 @@ __device__ __forceinline__ bool probe_shade_path(const SceneView& s, const Light
     const float ndl = maxf(0.0f, dot3(sd.frame.n, l));
     const f3 f = sd.diffuse * kInvPi;
     // the set's own t_max travels with the shadow ray (the batch mixes scenes)
-    push_shadow(q, buf, ctl, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee, L.t_max);
+    store_shadow(q, buf, slot, p, sd.origin_front, l, thp * ((f * L.illum) * ndl), kKindNee, L.t_max);
     const float e0 = rng.next_1d(), e1 = rng.next_1d();
     float pdf;
     const f3 sdir = cosine_sample_hemisphere(e0, e1, &pdf);
@@ -985,16 +1092,13 @@ __device__ __forceinline__ bool probe_shade_path(const SceneView& s, const Light
     st.rad[p] = f4(rad, 0.0f);
     st.rng[p] = rng.state;
     st.flags[p] = flags;
-    if (ended) push_close(q, buf ^ 1, ctl + kCtlWords, p);
-    else push_path(q, buf ^ 1, ctl + kCtlWords, p);
-    return true;
+    return ended ? kAwaitClose : kWalk;
 }
 
-// Closes the path's sample: the next one starts in the next round, or the
-// probe's running mean is stored.
-__device__ __forceinline__ void probe_close_path(const SceneView& s, const LightParams& L, const ProbeArgs& a,
-                                                 const WfState& st, const WfQueues& q, int buf, uint32_t* ctl,
-                                                 uint32_t p) {
+// Closes the path's sample: the next one starts, or the probe's running mean
+// is stored.
+__device__ __forceinline__ PathNext probe_close_path(const SceneView& s, const LightParams& L, const ProbeArgs& a,
+                                                     const WfState& st, uint32_t p) {
     const uint32_t flags = st.flags[p];
     const uint32_t probe = st.unit[p];
     f3 irr = xyz(st.irr[p]);
@@ -1019,10 +1123,10 @@ __device__ __forceinline__ void probe_close_path(const SceneView& s, const Light
         st.irr[p] = f4(irr, 0.0f);
         Rng rng(0u, 0u, 0u);
         rng.state = st.rng[p];
-        probe_start_sample(s, L, a, st, q, buf ^ 1, ctl + kCtlWords, p,
-                           (flags & ((1u << kSampleShift) - 1u)) | (k << kSampleShift), rng);
+        const PathNext next =
+            probe_start_sample(s, L, a, st, p, (flags & ((1u << kSampleShift) - 1u)) | (k << kSampleShift), rng);
         st.rng[p] = rng.state;
-        return;
+        return next;
     }
     irr = irr / (float)a.n;
     const uint32_t prev = a.reset ? 0u : a.out.counts[probe];
@@ -1038,27 +1142,58 @@ __device__ __forceinline__ void probe_close_path(const SceneView& s, const Light
     a.out.counts[probe] = min(prev + 1u, 65535u);
     const uint32_t prev_self = a.reset ? 0u : a.out.self_hits[probe];
     a.out.self_hits[probe] = prev_self + b.y;
+    return kRetire;
 }
 
-__global__ void __launch_bounds__(128) k_wf_probe_generate(SceneView s, LightingRaw lraw, ProbeArgs a, WfState st,
-                                                           WfQueues q, uint32_t begin, uint32_t count,
-                                                           unsigned long long* counters) {
-    const uint32_t slot_p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot_p >= count) return;
-    if (!probe_generate_path(s, make_light(lraw), a, st, q, begin + slot_p, slot_p)) return;
-    RayTally none{0u, 0u};
-    flush_tally(counters, none, 1u, a.n);
+// A block's entry of a round's queue: its path and, while it walks, the hit
+// the trace found.
+struct StageEntry {
+    uint32_t p;
+    float4 hit;
+    bool live, walks, at_hit;
+};
+
+__device__ __forceinline__ StageEntry stage_entry(const WfState& st, const WfQueues& q, int buf, uint32_t walking,
+                                                  uint32_t count, uint32_t idx) {
+    StageEntry e;
+    e.live = idx < count;
+    e.walks = idx < walking;
+    e.p = 0u;
+    e.hit = make_float4(__uint_as_float(0xffffffffu), 0.0f, 0.0f, 0.0f);
+    if (e.live) e.p = q.ext[buf][e.walks ? idx : q.cap - 1u - (idx - walking)];
+    if (e.walks) e.hit = st.hit[e.p];
+    e.at_hit = __float_as_uint(e.hit.x) != 0xffffffffu;
+    return e;
 }
 
-__global__ void __launch_bounds__(128, 6) k_wf_probe_stage(SceneView s, LightingRaw lraw, ProbeArgs a, WfState st,
-                                                        WfQueues q, int buf, uint32_t* ctl) {
+__global__ void __launch_bounds__(kStageThreads) k_wf_probe_generate(SceneView s, LightingRaw lraw, ProbeArgs a,
+                                                                  WfState st, WfQueues q, uint32_t begin,
+                                                                  uint32_t count, unsigned long long* counters) {
+    __shared__ BlockAppend sh;
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    PathNext next = kRetire;
+    if (p < count) next = probe_generate_path(s, make_light(lraw), a, st, begin + p, p);
+    push_paths(sh, q, 0, q.ctl + kCtlWords, p, next);
+    count_units(counters, next != kRetire, a.n);
+}
+
+__global__ void __launch_bounds__(kStageThreads, 6) k_wf_probe_stage(SceneView s, LightingRaw lraw, ProbeArgs a,
+                                                                  WfState st, WfQueues q, int buf, uint32_t* ctl) {
+    __shared__ BlockAppend sh[2];
     const uint32_t walking = *(volatile uint32_t*)(ctl + kExt);
     const uint32_t count = walking + *(volatile uint32_t*)(ctl + kClose);
     const LightParams L = make_light(lraw);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
-        if (idx >= walking || !probe_shade_path(s, L, a, st, q, buf, ctl, p))
-            probe_close_path(s, L, a, st, q, buf, ctl, p);
+    for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
+        const StageEntry e = stage_entry(st, q, buf, walking, count, base + threadIdx.x);
+        const uint32_t slot = shadow_slots(sh[0], ctl, e.at_hit);
+        PathNext next = kRetire;
+        if (e.at_hit) {
+            next = probe_shade_path(s, L, a, st, q, buf, slot, e.p, e.hit);
+        } else if (e.live) {
+            if (e.walks) probe_miss_path(L, st, e.p);
+            next = probe_close_path(s, L, a, st, e.p);
+        }
+        push_paths(sh[1], q, buf ^ 1, ctl + kCtlWords, e.p, next);
     }
 }
 
@@ -1104,32 +1239,27 @@ __device__ __forceinline__ ProbeArgs batch_probe_args(const BatchWfArgs& m, cons
     return a;
 }
 
-__global__ void __launch_bounds__(128) k_wfb_probe_generate(BatchWfArgs m, WfState st, WfQueues q,
-                                                            unsigned long long* counters) {
+__global__ void __launch_bounds__(kStageThreads) k_wfb_probe_generate(BatchWfArgs m, WfState st, WfQueues q,
+                                                                   unsigned long long* counters) {
+    __shared__ BlockAppend sh;
     const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= m.total) return;
-    uint32_t lo = 0u, hi = m.set_count - 1u;  // set = last s with prefix[s] <= u
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1u) >> 1;
-        if (__ldg(m.prefix + mid) <= u) lo = mid;
-        else hi = mid - 1u;
+    PathNext next = kRetire;
+    if (u < m.total) {
+        const uint32_t set = batch_set_of_unit(m, u);
+        m.set_of[u] = set;
+        const BatchSet& b = m.sets[set];
+        next = probe_generate_path(b.s, make_light(b.light), batch_probe_args(m, b), st, u - __ldg(m.prefix + set), u);
     }
-    m.set_of[u] = lo;
-    const BatchSet& b = m.sets[lo];
-    const ProbeArgs a = batch_probe_args(m, b);
-    if (!probe_generate_path(b.s, make_light(b.light), a, st, q, u - __ldg(m.prefix + lo), u)) return;
-    RayTally none{0u, 0u};
-    flush_tally(counters, none, 1u, a.n);
+    push_paths(sh, q, 0, q.ctl + kCtlWords, u, next);
+    count_units(counters, next != kRetire, m.n);
 }
 
 // Independent samples (NAN_BATCH_WAVEFRONT_INDEPENDENT): sample k of a probe
 // draws from RNG(probe, instance, iteration * n + k) and is its own path, so a
-// frame is max_bounces rounds; every finished path stores its sample, and a
-// last pass folds each probe's samples in sample order, as the
-// independent-sample persistent kernel does.
-__global__ void __launch_bounds__(128) k_wfi_probe_generate(BatchWfArgs m, WfState st, WfQueues q) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= m.units * m.n) return;
+// frame is max_bounces rounds and one that closes; every finished path stores
+// its sample, and a last pass folds each probe's samples in sample order, as
+// the independent-sample persistent kernel does.
+__device__ __forceinline__ PathNext independent_generate_path(const BatchWfArgs& m, const WfState& st, uint32_t p) {
     const uint32_t uoff = p / m.n, k = p - uoff * m.n;
     const uint32_t u = m.unit_begin + uoff;
     const uint32_t set = batch_set_of_unit(m, u);
@@ -1148,7 +1278,7 @@ __global__ void __launch_bounds__(128) k_wfi_probe_generate(BatchWfArgs m, WfSta
         none.nd = 0.0f;
         none.has_path = false;
         m.samples[p] = none;
-        return;
+        return kRetire;
     }
     const float4 params = __ldg(a.pinst + 3u * inst + 2u);
     st.unit[p] = probe;
@@ -1157,35 +1287,53 @@ __global__ void __launch_bounds__(128) k_wfi_probe_generate(BatchWfArgs m, WfSta
     st.si[p] = make_float4(0.0f, 0.0f, 0.0f, maxf(params.x, 1e-6f));
     st.pb[p] = make_uint4(0u, 0u, 0u, 0u);
     Rng rng(probe, inst, a.iteration * m.n + k);
-    probe_start_sample(b.s, make_light(b.light), a, st, q, 0, q.ctl + kCtlWords, p, 0u, rng);
+    const PathNext next = probe_start_sample(b.s, make_light(b.light), a, st, p, 0u, rng);
     st.rng[p] = rng.state;
+    return next;
 }
 
-__global__ void __launch_bounds__(128, 6) k_wfi_probe_stage(BatchWfArgs m, WfState st, WfQueues q, int buf,
-                                                            uint32_t* ctl) {
+__global__ void __launch_bounds__(kStageThreads) k_wfi_probe_generate(BatchWfArgs m, WfState st, WfQueues q) {
+    __shared__ BlockAppend sh;
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    PathNext next = kRetire;
+    if (p < m.units * m.n) next = independent_generate_path(m, st, p);
+    push_paths(sh, q, 0, q.ctl + kCtlWords, p, next);
+}
+
+__global__ void __launch_bounds__(kStageThreads, 6) k_wfi_probe_stage(BatchWfArgs m, WfState st, WfQueues q, int buf,
+                                                                   uint32_t* ctl) {
+    __shared__ BlockAppend sh[2];
     const uint32_t walking = *(volatile uint32_t*)(ctl + kExt);
     const uint32_t count = walking + *(volatile uint32_t*)(ctl + kClose);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
-        if (idx < walking) {
+    for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
+        const StageEntry e = stage_entry(st, q, buf, walking, count, base + threadIdx.x);
+        const uint32_t slot = shadow_slots(sh[0], ctl, e.at_hit);
+        PathNext next = kRetire;
+        if (e.live) {
+            const uint32_t p = e.p;
             const BatchSet& b = m.sets[m.set_of[p]];
-            if (probe_shade_path(b.s, make_light(b.light), batch_probe_args(m, b), st, q, buf, ctl, p)) continue;
+            if (e.at_hit) {
+                next = probe_shade_path(b.s, make_light(b.light), batch_probe_args(m, b), st, q, buf, slot, p, e.hit);
+            } else {
+                if (e.walks) probe_miss_path(make_light(b.light), st, p);
+                ProbeSample r;
+                r.si = mk3(0.0f, 0.0f, 0.0f);
+                r.self_hits = 0u;
+                r.texel = 0u;
+                r.nd = 0.0f;
+                r.has_path = !(st.flags[p] & kFlagNoPath);
+                if (r.has_path) {
+                    const uint4 pb = st.pb[p];
+                    const float2 zp = st.zpdf[p];
+                    r.si = r.si + ((xyz(st.rad[p]) * zp.x) / zp.y);
+                    r.self_hits = pb.x;
+                    r.texel = pb.w;
+                    r.nd = st.pa[p].w / maxf(st.si[p].w, 1e-6f);
+                }
+                m.samples[p] = r;
+            }
         }
-        ProbeSample r;
-        r.si = mk3(0.0f, 0.0f, 0.0f);
-        r.self_hits = 0u;
-        r.texel = 0u;
-        r.nd = 0.0f;
-        r.has_path = !(st.flags[p] & kFlagNoPath);
-        if (r.has_path) {
-            const uint4 b = st.pb[p];
-            const float2 zp = st.zpdf[p];
-            r.si = r.si + ((xyz(st.rad[p]) * zp.x) / zp.y);
-            r.self_hits = b.x;
-            r.texel = b.w;
-            r.nd = st.pa[p].w / maxf(st.si[p].w, 1e-6f);
-        }
-        m.samples[p] = r;
+        push_paths(sh[1], q, buf ^ 1, ctl + kCtlWords, e.p, next);
     }
 }
 
@@ -1211,17 +1359,27 @@ __global__ void __launch_bounds__(128) k_wfi_probe_fold(BatchWfArgs m, unsigned 
     flush_tally(counters, none, 1u, m.n);
 }
 
-__global__ void __launch_bounds__(128, 6) k_wfb_probe_stage(BatchWfArgs m, WfState st, WfQueues q, int buf,
-                                                         uint32_t* ctl) {
+__global__ void __launch_bounds__(kStageThreads, 6) k_wfb_probe_stage(BatchWfArgs m, WfState st, WfQueues q, int buf,
+                                                                   uint32_t* ctl) {
+    __shared__ BlockAppend sh[2];
     const uint32_t walking = *(volatile uint32_t*)(ctl + kExt);
     const uint32_t count = walking + *(volatile uint32_t*)(ctl + kClose);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t p = q.ext[buf][idx < walking ? idx : q.cap - 1u - (idx - walking)];
-        const BatchSet& b = m.sets[m.set_of[p]];
-        const LightParams L = make_light(b.light);
-        const ProbeArgs a = batch_probe_args(m, b);
-        if (idx >= walking || !probe_shade_path(b.s, L, a, st, q, buf, ctl, p))
-            probe_close_path(b.s, L, a, st, q, buf, ctl, p);
+    for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
+        const StageEntry e = stage_entry(st, q, buf, walking, count, base + threadIdx.x);
+        const uint32_t slot = shadow_slots(sh[0], ctl, e.at_hit);
+        PathNext next = kRetire;
+        if (e.live) {
+            const BatchSet& b = m.sets[m.set_of[e.p]];
+            const LightParams L = make_light(b.light);
+            const ProbeArgs a = batch_probe_args(m, b);
+            if (e.at_hit) {
+                next = probe_shade_path(b.s, L, a, st, q, buf, slot, e.p, e.hit);
+            } else {
+                if (e.walks) probe_miss_path(L, st, e.p);
+                next = probe_close_path(b.s, L, a, st, e.p);
+            }
+        }
+        push_paths(sh[1], q, buf ^ 1, ctl + kCtlWords, e.p, next);
     }
 }
 
@@ -1313,7 +1471,7 @@ Grid grid_for(const NanContext* ctx, uint64_t paths) {
     Grid g;
     const int per_sm = ctx->tuning.trace_blocks_per_sm ? (int)ctx->tuning.trace_blocks_per_sm : std::max(occ, 1);
     g.persistent_blocks = (int)std::min<uint64_t>((uint64_t)sms * per_sm, std::max<uint64_t>((3 * paths + 3) / 4, 1));
-    g.stream_blocks = (int)std::min<uint64_t>((uint64_t)sms * 16, std::max<uint64_t>((paths + 127) / 128, 1));
+    g.stream_blocks = (int)std::min<uint64_t>((uint64_t)sms * 16, std::max<uint64_t>((paths + kStageThreads - 1) / kStageThreads, 1));
     return g;
 }
 
@@ -1555,10 +1713,10 @@ int launch_trace_texels_wavefront(NanContext* ctx, const NanMeshColorsDesc* lay,
     return wf_run(
         ctx, st, begin, end, rounds, cap, lr.ray_t_max,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t count) {
-            k_wf_texel_generate<<<(count + 127) / 128, 128, 0, st>>>(s, lr, a, S, q, first, count, counters);
+            k_wf_texel_generate<<<(count + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(s, lr, a, S, q, first, count, counters);
         },
         [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, int blocks) {
-            k_wf_texel_stage<<<blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
+            k_wf_texel_stage<<<blocks, kStageThreads, 0, st>>>(s, lr, a, S, q, buf, ctl);
         });
 }
 
@@ -1618,10 +1776,10 @@ int launch_trace_points_wavefront(NanContext* ctx, const float* points, uint32_t
     return wf_run(
         ctx, st, 0, count, rounds, cap, lr.ray_t_max,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t cnt) {
-            k_wf_point_generate<<<(cnt + 127) / 128, 128, 0, st>>>(s, lr, a, S, q, first, cnt, counters);
+            k_wf_point_generate<<<(cnt + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(s, lr, a, S, q, first, cnt, counters);
         },
         [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, int blocks) {
-            k_wf_texel_stage<<<blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
+            k_wf_texel_stage<<<blocks, kStageThreads, 0, st>>>(s, lr, a, S, q, buf, ctl);
         });
 }
 
@@ -1650,10 +1808,10 @@ int screen_wavefront(NanContext* ctx, float* out, uint32_t w, uint32_t h, uint32
     return wf_run(
         ctx, st, 0, pixels, rounds, cap, lr.ray_t_max,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t count) {
-            k_wf_screen_generate<<<(count + 127) / 128, 128, 0, st>>>(s, lr, a, S, q, first, count, counters);
+            k_wf_screen_generate<<<(count + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(s, lr, a, S, q, first, count, counters);
         },
         [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, int blocks) {
-            k_wf_screen_stage<<<blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
+            k_wf_screen_stage<<<blocks, kStageThreads, 0, st>>>(s, lr, a, S, q, buf, ctl);
         });
 }
 }  // namespace
@@ -1699,11 +1857,11 @@ int launch_batch_wavefront(NanContext* ctx, const void* sets, const uint32_t* pr
     wf_carve(ctx, total, rounds, S, q);
     cudaError_t err = cudaMemsetAsync(q.ctl, 0, ctl_words(rounds) * sizeof(uint32_t), st);
     if (err != cudaSuccess) return cuda_fail(err, "batch wavefront control reset");
-    k_wfb_probe_generate<<<(total + 127) / 128, 128, 0, st>>>(m, S, q, ctx->d_counters);
+    k_wfb_probe_generate<<<(total + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(m, S, q, ctx->d_counters);
     ctx->launches++;
     for (uint32_t it = 0; it < rounds; ++it) {
         launch_trace(ctx, g.persistent_blocks, st, false, src, q, it, t_max, S);
-        k_wfb_probe_stage<<<g.stream_blocks, 128, 0, st>>>(m, S, q, (int)(it & 1u), q.ctl + kCtlWords * (it + 1u));
+        k_wfb_probe_stage<<<g.stream_blocks, kStageThreads, 0, st>>>(m, S, q, (int)(it & 1u), q.ctl + kCtlWords * (it + 1u));
         ctx->launches++;
     }
     return cuda_fail(cudaGetLastError(), "batch wavefront launch");
@@ -1747,10 +1905,10 @@ int launch_batch_wavefront_independent(NanContext* ctx, const void* sets, const 
         wf_carve(ctx, paths, rounds, S, q);
         cudaError_t err = cudaMemsetAsync(q.ctl, 0, ctl_words(rounds) * sizeof(uint32_t), st);
         if (err != cudaSuccess) return cuda_fail(err, "batch wavefront control reset");
-        k_wfi_probe_generate<<<(paths + 127) / 128, 128, 0, st>>>(m, S, q);
+        k_wfi_probe_generate<<<(paths + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(m, S, q);
         for (uint32_t it = 0; it < rounds; ++it) {
             launch_trace(ctx, g.persistent_blocks, st, false, src, q, it, t_max, S);
-            k_wfi_probe_stage<<<g.stream_blocks, 128, 0, st>>>(m, S, q, (int)(it & 1u), q.ctl + kCtlWords * (it + 1u));
+            k_wfi_probe_stage<<<g.stream_blocks, kStageThreads, 0, st>>>(m, S, q, (int)(it & 1u), q.ctl + kCtlWords * (it + 1u));
         }
         k_wfi_probe_fold<<<(m.units + 127) / 128, 128, 0, st>>>(m, ctx->d_counters);
         ctx->launches += 2 + rounds;
@@ -1786,10 +1944,10 @@ int launch_trace_probes_wavefront(NanContext* ctx, float* values, uint32_t* coun
     return wf_run(
         ctx, st, begin, end, rounds, cap, lr.ray_t_max,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t count) {
-            k_wf_probe_generate<<<(count + 127) / 128, 128, 0, st>>>(s, lr, a, S, q, first, count, counters);
+            k_wf_probe_generate<<<(count + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(s, lr, a, S, q, first, count, counters);
         },
         [&](const WfState& S, const WfQueues& q, int buf, uint32_t* ctl, int blocks) {
-            k_wf_probe_stage<<<blocks, 128, 0, st>>>(s, lr, a, S, q, buf, ctl);
+            k_wf_probe_stage<<<blocks, kStageThreads, 0, st>>>(s, lr, a, S, q, buf, ctl);
         });
 }
 
