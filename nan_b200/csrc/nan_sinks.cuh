@@ -47,15 +47,18 @@ __device__ __forceinline__ uint32_t mc_address(uint32_t i, uint32_t j, uint32_t 
     return texel_offset + face.x + row + j;
 }
 
+// Row i of an address (the last row that starts at or before it) and column
+// j. Row i starts at i (2 r + 3 - i) / 2, so i is the smaller root of a
+// quadratic; the float root is within one of it for the resolutions here, and
+// exact steps settle it.
 __device__ __forceinline__ void mc_address_to_ij(uint32_t address, uint32_t r, uint32_t* oi, uint32_t* oj) {
-    uint32_t left = 0u, right = r;
-    while (left < right) {
-        const uint32_t mid = (left + right + 1u) / 2u;
-        const uint32_t ma = mid * (r + 1u) - mid * (mid - 1u) / 2u;
-        if (ma <= address) left = mid; else right = mid - 1u;
-    }
-    *oi = left;
-    *oj = address - (left * (r + 1u) - left * (left - 1u) / 2u);
+    const float b = (float)(2u * r + 3u);
+    uint32_t i = (uint32_t)maxf(0.5f * (b - sqrtf(maxf(b * b - 8.0f * (float)address, 0.0f))), 0.0f);
+    i = min(i, r);
+    while (i > 0u && i * (2u * r + 3u - i) / 2u > address) --i;
+    while (i < r && (i + 1u) * (2u * r + 2u - i) / 2u <= address) ++i;
+    *oi = i;
+    *oj = address - i * (2u * r + 3u - i) / 2u;
 }
 
 __device__ __forceinline__ float fracf(float x) { return x - floorf(x); }

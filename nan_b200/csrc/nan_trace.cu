@@ -537,104 +537,277 @@ __device__ __forceinline__ float normal_filter_weight(f3 c, f3 n, float sigma) {
     return expf(-0.5f * na * na);
 }
 
+// One of three values by index, by selects.
+template <class T>
+__device__ __forceinline__ T pick3(uint32_t k, T a, T b, T c) {
+    return k == 0u ? a : (k == 1u ? b : c);
+}
+
 // Lattice point candidate (x, y) outside the face, across `edge`: its
 // barycentrics in the adjacent face, or false.
 __device__ __forceinline__ bool map_edge_tap(int x, int y, uint32_t R, uint32_t adj_edge, bool flip, uint32_t edge,
                                              float nb[3]) {
     const float inv = 1.0f / (float)R;
-    const float sb[3] = {(float)x * inv, (float)y * inv, 1.0f - (float)(x + y) * inv};
-    const uint32_t s_start = edge, s_end = (edge + 1u) % 3u, s_opp = (edge + 2u) % 3u;
-    const uint32_t n_start = adj_edge, n_end = (adj_edge + 1u) % 3u, n_opp = (adj_edge + 2u) % 3u;
-    const float outside = sb[s_opp];
-    const uint32_t m_start = flip ? n_end : n_start, m_end = flip ? n_start : n_end;
-    nb[0] = nb[1] = nb[2] = 0.0f;
-    nb[m_start] = sb[s_start] + outside;
-    nb[m_end] = sb[s_end] + outside;
-    nb[n_opp] = -outside;
+    const float b0 = (float)x * inv, b1 = (float)y * inv, b2 = 1.0f - (float)(x + y) * inv;
+    // the edge runs from corner `edge` to the next one, the third is opposite
+    const float outside = pick3(edge, b2, b0, b1);
+    const float start = pick3(edge, b0, b1, b2) + outside, end = pick3(edge, b1, b2, b0) + outside;
+    const float first = flip ? end : start, second = flip ? start : end, third = -outside;
+    nb[0] = pick3(adj_edge, first, third, second);
+    nb[1] = pick3(adj_edge, second, first, third);
+    nb[2] = pick3(adj_edge, third, second, first);
+#pragma unroll
     for (int k = 0; k < 3; ++k)
         if (nb[k] < -1e-5f || nb[k] > 1.0f + 1e-5f) return false;
+#pragma unroll
     for (int k = 0; k < 3; ++k) nb[k] = maxf(nb[k], 0.0f);
     const float sum = maxf((nb[0] + nb[1]) + nb[2], 1e-6f);
+#pragma unroll
     for (int k = 0; k < 3; ++k) nb[k] = nb[k] / sum;
     return true;
 }
 
-__device__ __forceinline__ void filter_side(const FilterArgs& a, uint32_t front, int ci, int cj, uint4 inst,
-                                            uint2 side, uint2 face, uint32_t prim, f3 cn, bool back) {
-    const uint32_t center = mc_side_texel(front, inst, side, back);
-    const float4 c = __ldg(a.src + center);
-    f3 acc = mk3(c.x, c.y, c.z);
-    float wsum = 1.0f;
-    const int R = (int)face.y;
-    const int off[6][2] = {{1, 0}, {-1, 0}, {0, 1}, {0, -1}, {1, -1}, {-1, 1}};
-    for (int t = 0; t < 6; ++t) {
-        const int x = ci + off[t][0], y = cj + off[t][1];
-        if (x >= 0 && y >= 0 && x + y <= R) {
-            const uint32_t ft = mc_address((uint32_t)x, (uint32_t)y, inst.z, face);
-            const f3 v = mc_load(a.src, false, mc_side_texel(ft, inst, side, back));
-            acc = acc + a.neighbor_weight * v;
-            wsum = wsum + a.neighbor_weight;
-            continue;
-        }
-        const uint32_t edge = x < 0 ? 1u : (y < 0 ? 2u : 0u);
-        const uint4 adj4 = __ldg(a.adjacency + inst.x + prim);
-        const uint32_t packed = edge == 0u ? adj4.x : (edge == 1u ? adj4.y : adj4.z);
-        if (packed == 0xffffffffu) continue;
-        const uint32_t adj_face = inst.x + (packed >> 3);
-        float nb[3];
-        if (!map_edge_tap(x, y, face.y, packed & 3u, (packed & 4u) != 0u, edge, nb)) continue;
-        const float4 nn = __ldg(a.normals + adj_face);
-        const float w = a.neighbor_weight * normal_filter_weight(cn, mk3(nn.x, nn.y, nn.z), a.sigma);
-        const uint2 nface = __ldg(a.mc.face_infos + adj_face);
-        const f3 v = mc_sample(a.src, false, nb[0], nb[1], nb[2], inst, nface, side, back);
-        if (w > 0.0f) {
-            acc = acc + w * v;
-            wsum = wsum + w;
-        }
+// Position of the last entry <= u in an ascending table of `count` entries
+// (entry(0) <= u), by the whole warp: 32 probes a step.
+template <class Entry>
+__device__ __forceinline__ uint32_t warp_last_not_above(uint32_t count, uint32_t u, Entry entry) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t lo = 0u, n = count;
+    while (n > 1u) {
+        const uint32_t step = (n + 31u) >> 5, at = lane * step;
+        const unsigned hits = __ballot_sync(0xffffffffu, at < n && entry(lo + at) <= u);
+        const uint32_t k = hits ? 31u - (uint32_t)__clz(hits) : 0u;
+        lo += k * step;
+        n = min(step, n - k * step);
     }
-    const f3 r = acc / maxf(wsum, 1e-6f);
-    a.dst[center] = make_float4(r.x, r.y, r.z, c.w);
+    return lo;
 }
 
-__global__ void __launch_bounds__(128) k_filter_mesh_colors(FilterArgs a) {
-    const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= a.total_texels) return;
-    const McView& mc = a.mc;
-    uint32_t lo = 0u, hi = mc.instance_count - 1u;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1u) >> 1;
-        if (__ldg(mc.surface_prefix + mid) <= u) lo = mid; else hi = mid - 1u;
-    }
-    const uint32_t local = u - __ldg(mc.surface_prefix + lo);
-    const uint4 inst = __ldg(mc.instance_infos + lo);
-    if (local >= inst.w) return;
-    // mesh_colors_find_face (mesh_colors.slang:272-305)
+struct FilterTexel {
+    uint4 inst;
+    uint2 face;
+    uint2 side;
+    uint32_t prim, local;
+};
+
+// mesh_colors_find_face (mesh_colors.slang:272-305) for one texel of an
+// instance.
+__device__ __forceinline__ bool filter_find_face(const McView& mc, uint4 inst, uint32_t local, uint2* face,
+                                                 uint32_t* prim) {
     int left = (int)inst.x, right = (int)(inst.x + inst.y) - 1;
-    uint2 face = make_uint2(0u, 1u);
-    uint32_t prim = 0u;
-    bool found = false;
     while (left <= right) {
         const int mid = (left + right) / 2;
-        face = __ldg(mc.face_infos + mid);
-        const int loc = (int)local - (int)face.x;
-        const int count = (int)((face.y + 1u) * (face.y + 2u) / 2u);
+        *face = __ldg(mc.face_infos + mid);
+        const int loc = (int)local - (int)face->x;
+        const int count = (int)((face->y + 1u) * (face->y + 2u) / 2u);
         if (loc < 0) right = mid - 1;
         else if (loc >= count) left = mid + 1;
         else {
-            prim = (uint32_t)mid - inst.x;
-            found = true;
-            break;
+            *prim = (uint32_t)mid - inst.x;
+            return true;
         }
     }
-    if (!found) return;
-    const uint2 side = __ldg(mc.side_infos + lo);
-    uint32_t ti, tj;
-    mc_address_to_ij(local - face.x, face.y, &ti, &tj);
-    const float4 n4 = __ldg(a.normals + inst.x + prim);
-    const f3 cn = mk3(n4.x, n4.y, n4.z);
-    const uint32_t front = inst.z + local;
-    filter_side(a, front, (int)ti, (int)tj, inst, side, face, prim, cn, false);
-    if (side.y & 1u) filter_side(a, front, (int)ti, (int)tj, inst, side, face, prim, cn, true);
+    return false;
+}
+
+// Where a warp's last 32 texels lay: their instance, and the face of the last.
+struct FilterHint {
+    uint32_t instance, face;
+    bool known;
+};
+
+// The instance and face of surface texel u, for a warp of consecutive texels
+// whose first is u0 < total. A warp whose texels lie in one instance (nearly
+// all) searches once, 32 probes a step, or goes on from its last texels, and
+// its lanes find their faces among the next 32, a face holding 3 texels or
+// more; else each lane searches for itself.
+__device__ __forceinline__ bool filter_texel(const McView& mc, uint32_t u0, uint32_t total, FilterHint& hint,
+                                             FilterTexel* t) {
+    const uint32_t u = u0 + (threadIdx.x & 31u), lane = threadIdx.x & 31u;
+    const uint32_t last = min(u0 + 31u, total - 1u);
+    uint32_t i = hint.instance, first = 0u;
+    bool one_instance = false;
+    if (hint.known) {
+        one_instance = i + 1u == mc.instance_count || __ldg(mc.surface_prefix + i + 1u) > last;
+        hint.known = one_instance;
+    }
+    if (!one_instance) {
+        i = warp_last_not_above(mc.instance_count, u0, [&](uint32_t k) { return __ldg(mc.surface_prefix + k); });
+        one_instance = i + 1u == mc.instance_count || __ldg(mc.surface_prefix + i + 1u) > last;
+    }
+    if (one_instance) {
+        first = __ldg(mc.surface_prefix + i);
+        const uint4 inst = __ldg(mc.instance_infos + i);
+        t->inst = inst;
+        t->side = __ldg(mc.side_infos + i);
+        t->local = u - first;
+        if (inst.y == 0u) {
+            hint.known = false;
+            return false;  // the whole warp
+        }
+        const uint32_t f0 = hint.known ? hint.face
+                                       : warp_last_not_above(inst.y, u0 - first, [&](uint32_t k) {
+                                             return __ldg(mc.face_infos + inst.x + k).x;
+                                         });
+        const uint32_t start = f0 + lane < inst.y ? __ldg(mc.face_infos + inst.x + f0 + lane).x : 0xffffffffu;
+        uint32_t k = 0u;  // the last of the 32 faces that starts at or before the texel
+#pragma unroll
+        for (uint32_t step = 16u; step > 0u; step >>= 1)
+            if (__shfl_sync(0xffffffffu, start, k + step) <= t->local) k += step;
+        t->prim = f0 + k;
+        t->face = __ldg(mc.face_infos + inst.x + t->prim);
+        hint.instance = i;
+        hint.face = __shfl_sync(0xffffffffu, t->prim, 31);
+        hint.known = true;
+        return u < total && t->local < inst.w && t->local >= t->face.x &&
+               t->local - t->face.x < (t->face.y + 1u) * (t->face.y + 2u) / 2u;
+    }
+    hint.known = false;
+    if (u >= total) return false;
+    uint32_t hi = mc.instance_count - 1u;
+    while (i < hi) {
+        const uint32_t mid = (i + hi + 1u) >> 1;
+        if (__ldg(mc.surface_prefix + mid) <= u) i = mid; else hi = mid - 1u;
+    }
+    t->inst = __ldg(mc.instance_infos + i);
+    t->side = __ldg(mc.side_infos + i);
+    t->local = u - __ldg(mc.surface_prefix + i);
+    return t->local < t->inst.w && filter_find_face(mc, t->inst, t->local, &t->face, &t->prim);
+}
+
+// Taps inside the face are a load and four multiply-adds; those across an edge
+// (one in ten on the 200k terrain, but some in nearly every warp) are some 250
+// instructions. A warp lists the edge taps of its 32 texels in shared memory
+// and takes them 32 at a time, then every texel sums its taps in order. A warp
+// filters kFilterGroups x 32 consecutive texels, so the search for the
+// first one's face is paid once. Issue bound (0.76 an issue slot; 345 M
+// instructions against 518 M with one thread a texel, its own searches and six
+// divergent taps): 12.6 M texels in 411 us, 611 before. 10 blocks a SM (48
+// registers; 432 us at 64), 4 groups (8: 409, 1: about 2 % more).
+constexpr int kFilterThreads = 128;
+constexpr uint32_t kFilterGroups = 4u;
+
+struct FilterTap {  // a texel's part of its edge taps
+    uint2 face;
+    uint32_t i, j, face_index, face_base, texel_base;
+    uint2 side;
+};
+
+struct FilterScratch {
+    FilterTap texel[32];
+    float4 tap[6][32];  // weight x colour, weight (< 0: no tap)
+    uint16_t list[6 * 32];
+};
+
+__global__ void __launch_bounds__(kFilterThreads, 10) k_filter_mesh_colors(FilterArgs a) {
+    __shared__ FilterScratch scratch[kFilterThreads / 32];
+    FilterScratch& m = scratch[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    const McView& mc = a.mc;
+    constexpr int off[6][2] = {{1, 0}, {-1, 0}, {0, 1}, {0, -1}, {1, -1}, {-1, 1}};
+    const uint64_t begin = ((uint64_t)blockIdx.x * (kFilterThreads / 32) + (threadIdx.x >> 5)) * 32u * kFilterGroups;
+    FilterHint hint{0u, 0u, false};
+    for (uint32_t g = 0; g < kFilterGroups; ++g) {
+        const uint64_t at = begin + 32u * g;
+        if (at >= a.total_texels) break;  // the whole warp
+        FilterTexel t;
+        const bool live = filter_texel(mc, (uint32_t)at, a.total_texels, hint, &t);
+        uint32_t ci = 0u, cj = 0u;
+        uint32_t outside = 0u;  // taps across an edge
+        bool two_sided = false;
+        if (live) {
+            mc_address_to_ij(t.local - t.face.x, t.face.y, &ci, &cj);
+            two_sided = (t.side.y & 1u) != 0u;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                const int x = (int)ci + off[k][0], y = (int)cj + off[k][1];
+                if (!(x >= 0 && y >= 0 && x + y <= (int)t.face.y)) outside |= 1u << k;
+            }
+            if (outside) {
+                FilterTap tap;
+                tap.face = t.face;
+                tap.i = ci;
+                tap.j = cj;
+                tap.face_index = t.inst.x + t.prim;
+                tap.face_base = t.inst.x;
+                tap.texel_base = t.inst.z;
+                tap.side = t.side;
+                m.texel[lane] = tap;
+            }
+        }
+        const int sides = __any_sync(0xffffffffu, two_sided) ? 2 : 1;
+        for (int back = 0; back < sides; ++back) {
+            const bool mine = live && (back == 0 || two_sided);
+            uint32_t taps = 0u;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                const bool has = mine && ((outside >> k) & 1u);
+                const unsigned who = __ballot_sync(0xffffffffu, has);
+                if (has) m.list[taps + (uint32_t)__popc(who & below)] = (uint16_t)(lane * 8u + (uint32_t)k);
+                taps += (uint32_t)__popc(who);
+            }
+            __syncwarp();
+            for (uint32_t e = lane; e < taps; e += 32u) {
+                const uint32_t who = m.list[e] >> 3, k = m.list[e] & 7u;
+                const FilterTap tap = m.texel[who];
+                int dx = 0, dy = 0;
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    if ((int)k == q) {
+                        dx = off[q][0];
+                        dy = off[q][1];
+                    }
+                const int x = (int)tap.i + dx, y = (int)tap.j + dy;
+                float4 r = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+                const uint32_t edge = x < 0 ? 1u : (y < 0 ? 2u : 0u);
+                const uint4 adj4 = __ldg(a.adjacency + tap.face_index);
+                const uint32_t packed = edge == 0u ? adj4.x : (edge == 1u ? adj4.y : adj4.z);
+                float nb[3];
+                if (packed != 0xffffffffu &&
+                    map_edge_tap(x, y, tap.face.y, packed & 3u, (packed & 4u) != 0u, edge, nb)) {
+                    const uint32_t adj_face = tap.face_base + (packed >> 3);
+                    const float4 cn = __ldg(a.normals + tap.face_index), nn = __ldg(a.normals + adj_face);
+                    const float w = a.neighbor_weight *
+                                    normal_filter_weight(mk3(cn.x, cn.y, cn.z), mk3(nn.x, nn.y, nn.z), a.sigma);
+                    const uint4 inst = make_uint4(tap.face_base, 0u, tap.texel_base, 0u);
+                    const f3 v = mc_sample(a.src, false, nb[0], nb[1], nb[2], inst, __ldg(mc.face_infos + adj_face),
+                                           tap.side, back != 0);
+                    if (w > 0.0f) {
+                        const f3 c = w * v;
+                        r = make_float4(c.x, c.y, c.z, w);
+                    }
+                }
+                m.tap[k][who] = r;
+            }
+            __syncwarp();
+            if (mine) {
+                const uint32_t center = mc_side_texel(t.inst.z + t.local, t.inst, t.side, back != 0);
+                const float4 c = __ldg(a.src + center);
+                f3 acc = mk3(c.x, c.y, c.z);
+                float wsum = 1.0f;
+                // a row is R + 1 - i texels long, so the taps lie at fixed steps
+                const uint32_t up = t.face.y + 1u - ci, down = t.face.y + 2u - ci;
+                const uint32_t step[6] = {up, 0u - down, 1u, 0u - 1u, up - 1u, 1u - down};
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    if (!((outside >> k) & 1u)) {
+                        const f3 v = mc_load(a.src, false, center + step[k]);
+                        acc = acc + a.neighbor_weight * v;
+                        wsum = wsum + a.neighbor_weight;
+                    } else {
+                        const float4 r = m.tap[k][lane];
+                        if (r.w > 0.0f) {
+                            acc = acc + mk3(r.x, r.y, r.z);
+                            wsum = wsum + r.w;
+                        }
+                    }
+                }
+                const f3 r = acc / maxf(wsum, 1e-6f);
+                a.dst[center] = make_float4(r.x, r.y, r.z, c.w);
+            }
+            __syncwarp();
+        }
+    }
 }
 
 // accumulator.slang:9-19
@@ -1100,7 +1273,7 @@ int launch_filter_mesh_colors(NanContext* ctx, const NanMeshColorsDesc* lay, con
     a.neighbor_weight = neighbor_weight;
     a.sigma = sigma;
     a.total_texels = lay->total_surface_texels;
-    k_filter_mesh_colors<<<blocks_for(a.total_texels, 128), 128, 0, st>>>(a);
+    k_filter_mesh_colors<<<blocks_for(a.total_texels, kFilterThreads * kFilterGroups), kFilterThreads, 0, st>>>(a);
     ctx->launches++;
     return cuda_fail(cudaGetLastError(), "filter_mesh_colors launch");
 }
