@@ -374,7 +374,8 @@ __global__ void __launch_bounds__(128) k_resolve_probes(SceneView s, LightingRaw
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t px = blockIdx.x * 16u + (warp & 1u) * 8u + (lane & 7u);
     const uint32_t py = blockIdx.y * 8u + (warp >> 1) * 4u + (lane >> 3);
-    if (px >= w || py >= h) return;
+    __shared__ ProbeWalk walks[4];
+    const bool inside = px < w && py < h;
     const LightParams L = make_light(lraw);
     float pxf = ((float)px + 0.5f) / (float)w;
     float pyf = ((float)py + 0.5f) / (float)h;
@@ -388,41 +389,53 @@ __global__ void __launch_bounds__(128) k_resolve_probes(SceneView s, LightingRaw
     const f3 dir = normalize3((nx * U + ny * V) + W);
     const float inv_cos = 1.0f / dot3(normalize3(W), dir);
     const f3 o = mk3(cam.position[0], cam.position[1], cam.position[2]);
-    const HitInfo hit = trace_closest(s, o, dir, cam.near_clip * inv_cos, cam.far_clip * inv_cos);
     const size_t pix = (size_t)py * w + px;
     const bool beauty = a.debug_view == 0u || a.debug_view == 6u;
-    if (!hit.valid) {
+    HitInfo hit;
+    hit.valid = false;
+    if (inside) hit = trace_closest(s, o, dir, cam.near_clip * inv_cos, cam.far_clip * inv_cos);
+    if (inside && !hit.valid) {
         f3 c = mk3(0.02f, 0.02f, 0.02f);
         if (beauty) {
             c = sky_radiance(L, dir);
             if (L.sun_disk) c = c + sun_disk(L, dir);
         }
         out[pix] = make_float4(c.x, c.y, c.z, 1.0f);
-        return;
     }
-    const uint2 ref = __ldg(s.tri_refs + hit.flat);
-    const Shading sd = shading_data(s, ref.x, ref.y, hit.b1, hit.b2, -dir);
-    f3 sun = mk3(0.0f, 0.0f, 0.0f);
-    if (beauty) {
-        Rng rng(px, py, a.frame);
-        const float ux = rng.next_1d();
-        const float uy = rng.next_1d();
-        RayTally tally{0u, 0u};
-        sun = sun_nee<DefaultTracer>(s, L, sd, ux, uy, tally);
+    bool gathers = inside && hit.valid;
+    uint2 ref = make_uint2(0u, 0u);
+    Shading sd;
+    f3 sun = mk3(0.0f, 0.0f, 0.0f), q = sun, qn = sun;
+    ProbeInstance ins;
+    if (gathers) {
+        ref = __ldg(s.tri_refs + hit.flat);
+        sd = shading_data(s, ref.x, ref.y, hit.b1, hit.b2, -dir);
+        if (beauty) {
+            Rng rng(px, py, a.frame);
+            const float ux = rng.next_1d();
+            const float uy = rng.next_1d();
+            RayTally tally{0u, 0u};
+            sun = sun_nee<DefaultTracer>(s, L, sd, ux, uy, tally);
+        }
+        if (ref.x >= a.layout.instance_count) {
+            atomicOr(s.status, kStatusBadRecord);
+            gathers = false;
+        }
     }
-    if (ref.x >= a.layout.instance_count) {
-        atomicOr(s.status, kStatusBadRecord);
-        return;
+    if (gathers) {
+        ins = load_probe_instance(a.layout, ref.x);
+        q = sd.position;
+        qn = normalize3(sd.face_normal);
+        if (ins.offsets.w == 0u) {
+            const f3 c = beauty ? sd.emissive + sun : gather_count_color(0u);
+            out[pix] = make_float4(c.x, c.y, c.z, 1.0f);
+            gathers = false;
+        }
     }
-    const ProbeInstance ins = load_probe_instance(a.layout, ref.x);
-    if (ins.offsets.w == 0u) {
-        const f3 c = beauty ? sd.emissive + sun : gather_count_color(0u);
-        out[pix] = make_float4(c.x, c.y, c.z, 1.0f);
-        return;
-    }
-    Candidates cand;
-    const ProbeReconstruction r = probe_reconstruct(a.layout, a.field, ins, sd.position, normalize3(sd.face_normal),
-                                                    a.min_gather, a.use_radial != 0u, cand, s.status);
+    if (!__any_sync(0xffffffffu, gathers)) return;
+    const ProbeReconstruction r = probe_reconstruct(a.layout, a.field, ins, ref.x, q, qn, a.min_gather,
+                                                    a.use_radial != 0u, gathers, walks[warp], s.status);
+    if (!gathers) return;
     const uint32_t side = sd.back_side ? 1u : 0u;
     const float b0 = (1.0f - hit.b1) - hit.b2;
     const float bary[3] = {b0, hit.b1, hit.b2};
