@@ -540,6 +540,7 @@ struct FilterArgs {
     float neighbor_weight;
     float sigma;
     uint32_t total_texels;
+    uint32_t groups;  // of 32 texels a warp
 };
 
 __device__ __forceinline__ float normal_filter_weight(f3 c, f3 n, float sigma) {
@@ -692,12 +693,15 @@ __device__ __forceinline__ bool filter_texel(const McView& mc, uint32_t u0, uint
 // (one in ten on the 200k terrain, but some in nearly every warp) are some 250
 // instructions. A warp lists the edge taps of its 32 texels in shared memory
 // and takes them 32 at a time, then every texel sums its taps in order. A warp
-// filters kFilterGroups x 32 consecutive texels, so the search for the
-// first one's face is paid once. Issue bound (0.76 an issue slot; 345 M
+// filters up to kFilterGroups x 32 consecutive texels, so the search for the
+// first one's face is paid once; fewer where the texels would not give every
+// warp slot of the chip that many, since the groups of a warp run one after
+// the other (395,718 texels: four groups
+// 27.0 us, by this rule 18.5, one thread a texel 20.5). Issue bound (0.76 an issue slot; 345 M
 // instructions against 518 M with one thread a texel, its own searches and six
 // divergent taps): 12.6 M texels in 411 us, 611 before. 10 blocks a SM (48
 // registers; 432 us at 64), 4 groups (8: 409, 1: about 2 % more).
-constexpr int kFilterThreads = 128;
+constexpr int kFilterThreads = 128, kFilterBlocks = 10;  // blocks: per SM
 constexpr uint32_t kFilterGroups = 4u;
 
 struct FilterTap {  // a texel's part of its edge taps
@@ -712,15 +716,15 @@ struct FilterScratch {
     uint16_t list[6 * 32];
 };
 
-__global__ void __launch_bounds__(kFilterThreads, 10) k_filter_mesh_colors(FilterArgs a) {
+__global__ void __launch_bounds__(kFilterThreads, kFilterBlocks) k_filter_mesh_colors(FilterArgs a) {
     __shared__ FilterScratch scratch[kFilterThreads / 32];
     FilterScratch& m = scratch[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
     const McView& mc = a.mc;
     constexpr int off[6][2] = {{1, 0}, {-1, 0}, {0, 1}, {0, -1}, {1, -1}, {-1, 1}};
-    const uint64_t begin = ((uint64_t)blockIdx.x * (kFilterThreads / 32) + (threadIdx.x >> 5)) * 32u * kFilterGroups;
+    const uint64_t begin = ((uint64_t)blockIdx.x * (kFilterThreads / 32) + (threadIdx.x >> 5)) * 32u * a.groups;
     FilterHint hint{0u, 0u, false};
-    for (uint32_t g = 0; g < kFilterGroups; ++g) {
+    for (uint32_t g = 0; g < a.groups; ++g) {
         const uint64_t at = begin + 32u * g;
         if (at >= a.total_texels) break;  // the whole warp
         FilterTexel t;
@@ -1286,7 +1290,10 @@ int launch_filter_mesh_colors(NanContext* ctx, const NanMeshColorsDesc* lay, con
     a.neighbor_weight = neighbor_weight;
     a.sigma = sigma;
     a.total_texels = lay->total_surface_texels;
-    k_filter_mesh_colors<<<blocks_for(a.total_texels, kFilterThreads * kFilterGroups), kFilterThreads, 0, st>>>(a);
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    a.groups = std::min(std::max(a.total_texels / ((uint32_t)sms * kFilterBlocks * kFilterThreads), 1u), kFilterGroups);
+    k_filter_mesh_colors<<<blocks_for(a.total_texels, kFilterThreads * a.groups), kFilterThreads, 0, st>>>(a);
     ctx->launches++;
     return cuda_fail(cudaGetLastError(), "filter_mesh_colors launch");
 }

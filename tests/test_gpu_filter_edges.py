@@ -32,7 +32,8 @@ def _strip(instances, triangles, seed):
 
 
 @pytest.mark.parametrize("instances,triangles,resolution", [(1, 1, 1), (1, 2, 1), (1, 11, 1), (1, 43, 1), (5, 2, 1),
-                                                            (40, 1, 2), (7, 5, 4), (3, 2, 64), (130, 3, 1)])
+                                                            (40, 1, 2), (7, 5, 4), (3, 2, 64), (130, 3, 1),
+                                                            (120, 23, 16), (180, 31, 16)])
 def test_filter_matches_oracle(device, instances, triangles, resolution):
     import torch
 
@@ -42,7 +43,7 @@ def test_filter_matches_oracle(device, instances, triangles, resolution):
 
     node = _strip(instances, triangles, seed=instances + triangles)
     layout = MeshColorsLayout.build(node, texels_per_unit=1.0, min_resolution=resolution, max_resolution=resolution,
-                                    max_total_texels=1_000_000)
+                                    max_total_texels=4_000_000)
     rng = np.random.default_rng(3)
     data = np.zeros((layout.total_payload_count, 4), np.float32)
     data[:, :3] = rng.uniform(0.0, 2.0, (data.shape[0], 3))
