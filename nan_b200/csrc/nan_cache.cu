@@ -113,30 +113,46 @@ __device__ __forceinline__ float corner_weight(const LevelCell& cell, int k) {
     return __fmul_rn(__fmul_rn(wx, wy), wz);
 }
 
-// Network input row: 32 hash features, normal, 1, zeros (as float).
-__device__ __forceinline__ void encode_row(const CacheView& c, float4 q0, float4 q1, float* x) {
-    const float3 u = unit_position(c, make_float3(q0.x, q0.y, q0.z));
-#pragma unroll 1
-    for (int l = 0; l < kLevels; ++l) {
+// The hash features of kCount levels from l0 on. The gathers bound it: 128 a
+// query, each lane's in a line of its own at the fine levels (L1 at 80 % of
+// its rate). The two corners along x lie side by side for every other cell
+// (the hash leaves x as it is, so an even x and the next differ in the last bit
+// only): the 8 bytes that hold the first corner are loaded, and the second one
+// apart only where it is not among them. Two levels' loads are in flight at a
+// time. 1920x1080 queries of a 2^19 table: 625 -> 515 us (536 us with one
+// level at a time; the sums keep their order).
+template <int kCount>
+__device__ __forceinline__ void encode_levels(const CacheView& c, float3 u, int l0, float* x) {
+#pragma unroll 2
+    for (int i = 0; i < kCount; ++i) {
+        const int l = l0 + i;
         const LevelCell cell = level_cell(c, u, l);
         const __half2* t = c.table + (size_t)l * (c.table_mask + 1u);
         float a0 = 0.0f, a1 = 0.0f;
+        uint2 pair[4];
+        uint32_t second[4], idx[4];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float w = corner_weight(cell, k);
-            const float2 f = __half22float2(__ldg(t + corner_index(c, cell, l, k)));
-            a0 = __fadd_rn(a0, __fmul_rn(w, f.x));
-            a1 = __fadd_rn(a1, __fmul_rn(w, f.y));
+        for (int m = 0; m < 4; ++m) {
+            idx[m] = corner_index(c, cell, l, 2 * m);
+            const uint32_t next = corner_index(c, cell, l, 2 * m + 1);
+            pair[m] = __ldg(reinterpret_cast<const uint2*>(t) + (idx[m] >> 1));
+            if ((idx[m] ^ next) == 1u) second[m] = (idx[m] & 1u) ? pair[m].x : pair[m].y;
+            else second[m] = __ldg(reinterpret_cast<const uint32_t*>(t) + next);
         }
-        x[2 * l] = a0;
-        x[2 * l + 1] = a1;
-    }
-    x[32] = q1.x;
-    x[33] = q1.y;
-    x[34] = q1.z;
-    x[35] = 1.0f;
 #pragma unroll
-    for (int i = 36; i < kInputs; ++i) x[i] = 0.0f;
+        for (int m = 0; m < 4; ++m) {
+            const uint32_t first = (idx[m] & 1u) ? pair[m].y : pair[m].x;
+            const float w0 = corner_weight(cell, 2 * m), w1 = corner_weight(cell, 2 * m + 1);
+            const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&first));
+            const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&second[m]));
+            a0 = __fadd_rn(a0, __fmul_rn(w0, f0.x));
+            a1 = __fadd_rn(a1, __fmul_rn(w0, f0.y));
+            a0 = __fadd_rn(a0, __fmul_rn(w1, f1.x));
+            a1 = __fadd_rn(a1, __fmul_rn(w1, f1.y));
+        }
+        x[2 * i] = a0;
+        x[2 * i + 1] = a1;
+    }
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
@@ -161,6 +177,32 @@ __device__ __forceinline__ void load8(const unsigned char* tile, uint32_t r, uin
     for (int i = 0; i < 4; ++i) {
         v[2 * i] = __uint_as_float(u[i] << 16);
         v[2 * i + 1] = __uint_as_float(u[i] & 0xFFFF0000u);
+    }
+}
+
+// Part `part` of kParts of a query's network input (32 hash features, normal,
+// 1, zeros), as bf16 into row r of the tile: four levels are 8 columns.
+template <int kParts>
+__device__ __forceinline__ void encode_row(const CacheView& c, const float4* __restrict__ query, bool valid,
+                                           unsigned char* tile, uint32_t r, uint32_t part) {
+    float4 q0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), q1 = q0;
+    if (valid) {
+        q0 = query[0];
+        q1 = query[1];
+    }
+    const float3 u = unit_position(c, make_float3(q0.x, q0.y, q0.z));
+#pragma unroll 1
+    for (uint32_t b = part; b < 4u; b += kParts) {
+        float x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = 0.0f;
+        if (valid) encode_levels<4>(c, u, 4 * (int)b, x);
+        store8(tile, r, 8u * b, kInputs, x);
+    }
+    for (uint32_t b = part; b < 2u; b += kParts) {
+        const float x[8] = {b ? 0.0f : q1.x, b ? 0.0f : q1.y, b ? 0.0f : q1.z, !b && valid ? 1.0f : 0.0f,
+                            0.0f, 0.0f, 0.0f, 0.0f};
+        store8(tile, r, 32u + 8u * b, kInputs, x);
     }
 }
 
@@ -207,7 +249,7 @@ constexpr int kInferSub = 2;
 
 template <int kSub>
 __global__ void __launch_bounds__(kSub * kTile, infer_ctas_per_sm<kSub>())
-    k_cache_infer(CacheView c, const uint4* __restrict__ img, InferArgs a) {
+    k_cache_infer(const __grid_constant__ CacheView c, const uint4* __restrict__ img, InferArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr uint32_t kActTile = kTile * kHidden * 2;
     unsigned char* s_w = smem;
@@ -236,17 +278,7 @@ __global__ void __launch_bounds__(kSub * kTile, infer_ctas_per_sm<kSub>())
     for (uint32_t group = blockIdx.x; group < groups && ok; group += gridDim.x) {
         const uint32_t q = (group * kSub + sub) * kTile + r;
         const bool valid = q < count;
-        {
-            float x[kInputs];
-            if (valid) {
-                encode_row(c, a.queries[2 * q], a.queries[2 * q + 1], x);
-            } else {
-#pragma unroll
-                for (int i = 0; i < kInputs; ++i) x[i] = 0.0f;
-            }
-#pragma unroll
-            for (int c0 = 0; c0 < kInputs; c0 += 8) store8(s_act, r, c0, kInputs, x + c0);
-        }
+        encode_row<1>(c, a.queries + 2 * (size_t)q, valid, s_act, r, 0u);
         for (int layer = 0; layer < 5 && ok; ++layer) {
             tc::fence_smem_to_async();
             tc::fence_before_sync();
@@ -329,7 +361,15 @@ constexpr int kActBytes0 = kTile * kInputs * 2;
 constexpr int kActBytes = kTile * kHidden * 2;
 constexpr int kTrainSmem = kImgBytes + kActBytes0 + 4 * kActBytes + kActBytes + 64;
 
-__global__ void __launch_bounds__(kTile, 1) k_cache_train(CacheView c, const uint4* __restrict__ img, TrainArgs a) {
+// kTrainParts threads take a sample: each a part of its encoding, of the columns
+// between layers and of the table scatter. With one thread a sample an SM had
+// four warps, each waiting on its own gathers: 16,384 samples 55 us, now 48
+// (bound by the latency of the gathers and of ten dependent MMA groups).
+constexpr int kTrainParts = 4;
+static_assert(kHidden / kTrainParts == 16, "one TMEM load per layer and thread");
+
+__global__ void __launch_bounds__(kTile * kTrainParts, 1)
+    k_cache_train(const __grid_constant__ CacheView c, const uint4* __restrict__ img, TrainArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char* s_w = smem;
     unsigned char* s_act[5];
@@ -338,19 +378,21 @@ __global__ void __launch_bounds__(kTile, 1) k_cache_train(CacheView c, const uin
     unsigned char* s_delta = s_act[4] + kActBytes;
     uint64_t* bar = reinterpret_cast<uint64_t*>(s_delta + kActBytes);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
-    const uint32_t r = threadIdx.x, warp = r >> 5, lane = r & 31u;
+    const uint32_t r = threadIdx.x & (kTile - 1), part = threadIdx.x / kTile;
+    const uint32_t quarter = r >> 5, lane = r & 31u;  // the warp's quarter of the TMEM lanes
+    const bool first_warp = threadIdx.x < 32u;
     const uint32_t tiles = (a.count + kTile - 1) / kTile;
     if (blockIdx.x >= tiles) return;
 
     load_weights(s_w, img);
-    if (r == 0) tc::mbar_init(bar, 1);
-    if (warp == 0) tc::tmem_alloc(tslot, kTrainTmemCols);
+    if (threadIdx.x == 0) tc::mbar_init(bar, 1);
+    if (first_warp) tc::tmem_alloc(tslot, kTrainTmemCols);
     tc::fence_smem_to_async();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tslot;
-    const uint32_t my_lane = tmem + ((warp * 32u) << 16);
+    const uint32_t my_lane = tmem + ((quarter * 32u) << 16);
     const uint32_t w_addr = tc::smem_addr(s_w), delta_addr = tc::smem_addr(s_delta);
     uint32_t act_addr[5];
     for (int i = 0; i < 5; ++i) act_addr[i] = tc::smem_addr(s_act[i]);
@@ -363,7 +405,7 @@ __global__ void __launch_bounds__(kTile, 1) k_cache_train(CacheView c, const uin
         tc::fence_smem_to_async();
         tc::fence_before_sync();
         __syncthreads();
-        if (r == 0) {
+        if (threadIdx.x == 0) {
             tc::fence_after_sync();
             issue();
             tc::commit(bar);
@@ -382,20 +424,7 @@ __global__ void __launch_bounds__(kTile, 1) k_cache_train(CacheView c, const uin
             const float4 y = a.targets[q];
             valid = !(y.w < 0.0f) && isfinite(y.x) && isfinite(y.y) && isfinite(y.z);
         }
-        float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
-        {
-            float x[kInputs];
-            if (valid) {
-                q0 = a.queries[2 * q];
-                q1 = a.queries[2 * q + 1];
-                encode_row(c, q0, q1, x);
-            } else {
-#pragma unroll
-                for (int i = 0; i < kInputs; ++i) x[i] = 0.0f;
-            }
-#pragma unroll
-            for (int c0 = 0; c0 < kInputs; c0 += 8) store8(s_act[0], r, c0, kInputs, x + c0);
-        }
+        encode_row<kTrainParts>(c, a.queries + 2 * (size_t)q, valid, s_act[0], r, part);
         // forward
         for (int layer = 0; layer < 5 && ok; ++layer) {
             sync_issue_wait([&] {
@@ -405,35 +434,35 @@ __global__ void __launch_bounds__(kTile, 1) k_cache_train(CacheView c, const uin
             });
             if (!ok) break;
             if (layer < 4) {
-#pragma unroll
-                for (int c0 = 0; c0 < kHidden; c0 += 16) {
-                    float v[16];
-                    tc::tmem_load16(my_lane + kColFwd + c0, v);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
-                    store8(s_act[layer + 1], r, c0, kHidden, v);
-                    store8(s_act[layer + 1], r, c0 + 8, kHidden, v + 8);
-                }
-            } else {
+                const int c0 = 16 * (int)part;
                 float v[16];
-                tc::tmem_load16(my_lane + kColFwd, v);
-                float d[64];
+                tc::tmem_load16(my_lane + kColFwd + c0, v);
 #pragma unroll
-                for (int i = 0; i < 64; ++i) d[i] = 0.0f;
-                if (valid) {
-                    const float4 y = a.targets[q];
-                    const float yy[3] = {y.x, y.y, y.z};
+                for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
+                store8(s_act[layer + 1], r, c0, kHidden, v);
+                store8(s_act[layer + 1], r, c0 + 8, kHidden, v + 8);
+            } else {
+                float d[16];
 #pragma unroll
-                    for (int ch = 0; ch < 3; ++ch) {
-                        const float o = v[ch];
-                        const float den = __fadd_rn(__fmul_rn(o, o), a.loss_eps);
-                        const float e = __fsub_rn(o, yy[ch]);
-                        loss = __fadd_rn(loss, __fmul_rn(__fdiv_rn(__fmul_rn(e, e), den), a.inv_batch));
-                        d[ch] = __fdiv_rn(__fmul_rn(2.0f, e), __fmul_rn(den, a.batch));
+                for (int i = 0; i < 16; ++i) d[i] = 0.0f;
+                if (part == 0u) {  // whole warps: the outputs are columns 0 to 2
+                    float v[16];
+                    tc::tmem_load16(my_lane + kColFwd, v);
+                    if (valid) {
+                        const float4 y = a.targets[q];
+                        const float yy[3] = {y.x, y.y, y.z};
+#pragma unroll
+                        for (int ch = 0; ch < 3; ++ch) {
+                            const float o = v[ch];
+                            const float den = __fadd_rn(__fmul_rn(o, o), a.loss_eps);
+                            const float e = __fsub_rn(o, yy[ch]);
+                            loss = __fadd_rn(loss, __fmul_rn(__fdiv_rn(__fmul_rn(e, e), den), a.inv_batch));
+                            d[ch] = __fdiv_rn(__fmul_rn(2.0f, e), __fmul_rn(den, a.batch));
+                        }
                     }
                 }
-#pragma unroll
-                for (int c0 = 0; c0 < 64; c0 += 8) store8(s_delta, r, c0, 64, d + c0);
+                store8(s_delta, r, 16u * part, 64, d);
+                store8(s_delta, r, 16u * part + 8u, 64, d + 8);
             }
         }
         // backward
@@ -458,33 +487,35 @@ __global__ void __launch_bounds__(kTile, 1) k_cache_train(CacheView c, const uin
             if (!ok) break;
             if (layer > 0) {
                 // delta of the layer below: g masked by its ReLU, as bf16
+                const int c0 = 16 * (int)part;
+                float g[16], act[16];
+                tc::tmem_load16(my_lane + kColBwd + c0, g);
+                load8(s_act[layer], r, c0, kHidden, act);
+                load8(s_act[layer], r, c0 + 8, kHidden, act + 8);
 #pragma unroll
-                for (int c0 = 0; c0 < kHidden; c0 += 16) {
-                    float g[16], act[16];
-                    tc::tmem_load16(my_lane + kColBwd + c0, g);
-                    load8(s_act[layer], r, c0, kHidden, act);
-                    load8(s_act[layer], r, c0 + 8, kHidden, act + 8);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) g[i] = act[i] > 0.0f ? g[i] : 0.0f;
-                    store8(s_delta, r, c0, 64, g);
-                    store8(s_delta, r, c0 + 8, 64, g + 8);
-                }
+                for (int i = 0; i < 16; ++i) g[i] = act[i] > 0.0f ? g[i] : 0.0f;
+                store8(s_delta, r, c0, 64, g);
+                store8(s_delta, r, c0 + 8, 64, g + 8);
             } else {
-                float g[32];
-                tc::tmem_load16(my_lane + kColBwd, g);
-                tc::tmem_load16(my_lane + kColBwd + 16, g + 16);
+                // columns 8 part .. 8 part + 7: the features of levels 4 part .. 4 part + 3
+                float g[16];
+                tc::tmem_load16(my_lane + kColBwd + 16u * (part >> 1), g);
                 if (valid) {
+                    const float4 q0 = a.queries[2 * (size_t)q];
                     const float3 u = unit_position(c, make_float3(q0.x, q0.y, q0.z));
                     const size_t T = (size_t)c.table_mask + 1u;
-#pragma unroll 1
-                    for (int l = 0; l < kLevels; ++l) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int l = 4 * (int)part + i;
+                        const float g0 = (part & 1u) ? g[8 + 2 * i] : g[2 * i];
+                        const float g1 = (part & 1u) ? g[9 + 2 * i] : g[2 * i + 1];
                         const LevelCell cell = level_cell(c, u, l);
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {
                             const float w = corner_weight(cell, k);
                             const uint32_t idx = corner_index(c, cell, l, k);
                             atomicAdd(a.table_grad + (size_t)l * T + idx,
-                                      make_float2(__fmul_rn(w, g[2 * l]), __fmul_rn(w, g[2 * l + 1])));
+                                      make_float2(__fmul_rn(w, g0), __fmul_rn(w, g1)));
                         }
                     }
                 }
@@ -497,15 +528,15 @@ __global__ void __launch_bounds__(kTile, 1) k_cache_train(CacheView c, const uin
     __syncthreads();
     tc::fence_after_sync();
     // into this CTA's partial (summed by k_cache_reduce); zeros if it had no tile
-    float* part = a.partials + (size_t)blockIdx.x * kMlpParams;
+    float* dst = a.partials + (size_t)blockIdx.x * kMlpParams;
     for (int layer = 0; layer < 5; ++layer) {
         const int n_out = rows_of(layer), n_in = cols_of(layer);
-        const int m = 16 * (int)warp + (int)lane;  // valid for lanes 0-15
-        for (int c0 = 0; c0 < n_in; c0 += 16) {
+        const int m = 16 * (int)quarter + (int)lane;  // valid for lanes 0-15
+        for (int c0 = 16 * (int)part; c0 < n_in; c0 += 16 * kTrainParts) {  // whole warps
             float v[16];
             tc::tmem_load16(my_lane + dw_col(layer) + c0, v);
             if (lane < 16 && m < n_out) {
-                float4* gp = reinterpret_cast<float4*>(part + off_of(layer) + m * n_in + c0);
+                float4* gp = reinterpret_cast<float4*>(dst + off_of(layer) + m * n_in + c0);
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     gp[i] = (ok && !first) ? make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3])
@@ -517,11 +548,11 @@ __global__ void __launch_bounds__(kTile, 1) k_cache_train(CacheView c, const uin
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
     if (lane == 0 && loss != 0.0f) atomicAdd(a.loss, loss);
-    if (!ok && r == 0) atomicOr(c.status, kStatusTensorWait);
+    if (!ok && threadIdx.x == 0) atomicOr(c.status, kStatusTensorWait);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    if (warp == 0) tc::tmem_dealloc(tmem, kTrainTmemCols);
+    if (first_warp) tc::tmem_dealloc(tmem, kTrainTmemCols);
 }
 
 // grad[i] += sum over CTAs of partials[c][i] (fixed order: deterministic).
@@ -529,6 +560,7 @@ __global__ void k_cache_reduce(const float* __restrict__ partials, int parts, fl
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= kMlpParams) return;
     float acc = 0.0f;
+#pragma unroll 16
     for (int c = 0; c < parts; ++c) acc += partials[(size_t)c * kMlpParams + i];
     grad[i] += acc;
 }
@@ -757,8 +789,8 @@ int launch_cache_backward(NanCache* k, const float* queries, const float* target
     const uint32_t tiles = (count + kTile - 1) / kTile;
     // one CTA per SM: 512 TMEM columns and 124 KB shared memory each
     const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)sm_count(k->ctx->device));
-    k_cache_train<<<grid, kTile, kTrainSmem, st>>>(cache_view(k), reinterpret_cast<const uint4*>(k->img), a);
-    k_cache_reduce<<<kMlpParams / 256, 256, 0, st>>>(k->partials, (int)grid, k->mlp + 3 * kMlpParams);
+    k_cache_train<<<grid, kTile * kTrainParts, kTrainSmem, st>>>(cache_view(k), reinterpret_cast<const uint4*>(k->img), a);
+    k_cache_reduce<<<kMlpParams / 64, 64, 0, st>>>(k->partials, (int)grid, k->mlp + 3 * kMlpParams);
     k->ctx->launches += 2;
     return cuda_fail(cudaGetLastError(), "cache training");
 }
