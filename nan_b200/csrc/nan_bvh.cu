@@ -825,15 +825,17 @@ __global__ void k_wide_level(const WideItem* __restrict__ items, const uint32_t*
 // splits at the bin boundary of least (left area x left count + right area x
 // right count), down to single triangles; the SAH leaf collapse and the
 // depth-first emission above then run on this tree as on PLOC's.
-// Nodes of more than kSahSeqMax triangles are split level by level over the
-// whole GPU: bins accumulate with atomics (per block in shared memory for the
-// block's main node), one thread per node picks the split, and a scan of the
-// left flags partitions each node's range stably. Nodes of at most
-// kSahSeqMax triangles are built by one warp each, with the same split rule.
+// Nodes of more than kSahMidMax triangles are split level by level over the
+// whole GPU: bins accumulate in shared memory by block, then with atomics, a
+// warp per node picks the split, and a scan of the left flags partitions each
+// node's range stably. A block builds each node of at most kSahMidMax
+// triangles down to kSahSeqMax, and a warp each node of at most kSahSeqMax,
+// with the same split rule.
 // A node whose centroids coincide on every axis splits its range in half.
 // ---------------------------------------------------------------------------
 constexpr int kSahBins = 32;
 constexpr uint32_t kSahSeqMax = 64;
+constexpr uint32_t kSahMidMax = 1024;
 constexpr int kSahBinWords = 13;  // box lo, hi, centroid lo, hi (ordered ints), count
 constexpr int kSahTaskWords = 3 * kSahBins * kSahBinWords;
 constexpr int kSahMaxLevels = 512;
@@ -858,12 +860,13 @@ struct SahSmall {
 struct SahCounters {
     uint32_t nodes, large, small, level;
     uint32_t overflow;  // nonzero: a bound below was exceeded (nothing was written past it)
+    uint32_t mid;       // mid tasks (appended)
 };
 
-// Capacities of the next-level task list, the small-task list and the
-// interior nodes (n - 1).
+// Capacities of the next-level task list, the small-task list, the interior
+// nodes (n - 1) and the mid-task list.
 struct SahLimits {
-    uint32_t large, small, nodes;
+    uint32_t large, small, nodes, mid;
 };
 
 __device__ __forceinline__ float sah_half_area(float lx, float ly, float lz, float hx, float hy, float hz) {
@@ -894,11 +897,12 @@ __global__ void k_sah_init(uint32_t n, int* __restrict__ ids, int* __restrict__ 
 }
 
 __global__ void k_sah_root(uint32_t n, const Bounds* __restrict__ bounds, SahTask* __restrict__ tasks,
-                           SahSmall* __restrict__ small, SahCounters* __restrict__ ctr) {
+                           SahTask* __restrict__ mid, SahSmall* __restrict__ small, SahCounters* __restrict__ ctr) {
     ctr->nodes = 1u;
     ctr->large = 0u;
-    ctr->level = n > kSahSeqMax ? 1u : 0u;
+    ctr->level = n > kSahMidMax ? 1u : 0u;
     ctr->overflow = 0u;
+    ctr->mid = n > kSahSeqMax && n <= kSahMidMax ? 1u : 0u;
     if (n > kSahSeqMax) {
         SahTask t;
         t.first = 0u;
@@ -912,7 +916,8 @@ __global__ void k_sah_root(uint32_t n, const Bounds* __restrict__ bounds, SahTas
         t.split_bin = 0u;
         t.left_count = 0u;
         t.child_task[0] = t.child_task[1] = -1;
-        tasks[0] = t;
+        if (n > kSahMidMax) tasks[0] = t;
+        else mid[0] = t;
         ctr->small = 0u;
     } else {
         small[0] = SahSmall{0u, n, 0};
@@ -928,113 +933,160 @@ __global__ void k_sah_bins_reset(uint32_t words, uint32_t* __restrict__ bins) {
     bins[i] = (w < 3 || (w >= 6 && w < 9)) ? 0xffffffffu : 0u;
 }
 
-__device__ __forceinline__ void sah_bin_add(uint32_t* b, float4 lo, float4 hi, float3 c) {
-    const uint32_t v[12] = {float_to_ordered(lo.x), float_to_ordered(lo.y), float_to_ordered(lo.z),
-                            float_to_ordered(hi.x), float_to_ordered(hi.y), float_to_ordered(hi.z),
-                            float_to_ordered(c.x),  float_to_ordered(c.y),  float_to_ordered(c.z),
-                            float_to_ordered(c.x),  float_to_ordered(c.y),  float_to_ordered(c.z)};
+// A warp's triangles into shared bins, `set` the lane's node among those in
+// s_bins (< 0: the lane has none). The order is the Morton code's, so
+// neighbours fall into the same bins and their atomics would queue up: a run
+// that shares its first lane's bin is reduced across the warp and added once.
+__device__ __forceinline__ void sah_bins_add(uint32_t* s_bins, int set, float4 lo, float4 hi, float3 c,
+                                             const int bin[3]) {
+    constexpr uint32_t kFull = 0xffffffffu, kMinGroup = 6u;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t vlo[6] = {float_to_ordered(lo.x), float_to_ordered(lo.y), float_to_ordered(lo.z),
+                             float_to_ordered(c.x), float_to_ordered(c.y), float_to_ordered(c.z)};
+    const uint32_t vhi[6] = {float_to_ordered(hi.x), float_to_ordered(hi.y), float_to_ordered(hi.z),
+                             vlo[3], vlo[4], vlo[5]};
 #pragma unroll
-    for (int k = 0; k < 12; ++k) {
-        if (k < 3 || (k >= 6 && k < 9)) atomicMin(b + k, v[k]);
-        else atomicMax(b + k, v[k]);
+    for (int a = 0; a < 3; ++a) {
+        const uint32_t key = set < 0 ? 0xffffffffu : (uint32_t)((set * 3 + a) * kSahBins + bin[a]);
+        uint32_t todo = __ballot_sync(kFull, set >= 0);
+        for (int g = 0; g < 2 && todo != 0u; ++g) {
+            const uint32_t leader = (uint32_t)__ffs(todo) - 1u;
+            const uint32_t shared_key = __shfl_sync(kFull, key, leader);
+            const uint32_t same = __ballot_sync(kFull, key == shared_key);
+            if ((uint32_t)__popc(same) < kMinGroup) break;
+            const bool in = key == shared_key;
+            uint32_t rlo[6], rhi[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                rlo[k] = __reduce_min_sync(kFull, in ? vlo[k] : 0xffffffffu);
+                rhi[k] = __reduce_max_sync(kFull, in ? vhi[k] : 0u);
+            }
+            if (lane == leader) {
+                uint32_t* d = s_bins + shared_key * kSahBinWords;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    atomicMin(d + k, rlo[k]);
+                    atomicMax(d + 3 + k, rhi[k]);
+                    atomicMin(d + 6 + k, rlo[3 + k]);
+                    atomicMax(d + 9 + k, rhi[3 + k]);
+                }
+                atomicAdd(d + 12, (uint32_t)__popc(same));
+            }
+            todo &= ~same;
+        }
+        if ((todo >> lane) & 1u) {
+            uint32_t* d = s_bins + key * kSahBinWords;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                atomicMin(d + k, vlo[k]);
+                atomicMax(d + 3 + k, vhi[k]);
+                atomicMin(d + 6 + k, vlo[3 + k]);
+                atomicMax(d + 9 + k, vhi[3 + k]);
+            }
+            atomicAdd(d + 12, 1u);
+        }
     }
-    atomicAdd(b + 12, 1u);
 }
 
-constexpr int kSahBinPerThread = 4;
+constexpr int kSahBinPerThread = 2;
 
 // Bins of every triangle in a large node. A block covers kThreads x
-// kSahBinPerThread consecutive positions and keeps the bins of the node at
-// its first position in shared memory.
+// kSahBinPerThread consecutive positions; a large node has more than that, so
+// at most two of them meet there, each with its bins in shared memory.
+// What bounds it is the shared atomics, which queue on the bins that neighbours
+// share. A level of 200k triangles: 16 us; 52 us with every lane's atomics apart
+// and one node a block in shared memory.
 __global__ void __launch_bounds__(kThreads) k_sah_bin(uint32_t n, const int* __restrict__ ids,
                                                       const int* __restrict__ task_of,
                                                       const SahTask* __restrict__ tasks,
                                                       const float4* __restrict__ leaf_lo,
                                                       const float4* __restrict__ leaf_hi, uint32_t* __restrict__ bins) {
-    __shared__ uint32_t s_bins[kSahTaskWords];
-    __shared__ uint32_t s_first;
+    static_assert(kThreads * kSahBinPerThread <= kSahMidMax, "two large nodes a block at most");
+    __shared__ uint32_t s_bins[2 * kSahTaskWords];
+    __shared__ uint32_t s_first[2];
     const uint32_t base = blockIdx.x * (uint32_t)(kThreads * kSahBinPerThread);
-    if (threadIdx.x == 0) s_first = 0xffffffffu;
-    for (int i = threadIdx.x; i < kSahTaskWords; i += kThreads) {
+    if (threadIdx.x < 2) s_first[threadIdx.x] = 0xffffffffu;
+    for (int i = threadIdx.x; i < 2 * kSahTaskWords; i += kThreads) {
         const int w = i % kSahBinWords;
         s_bins[i] = (w < 3 || (w >= 6 && w < 9)) ? 0xffffffffu : 0u;
     }
     __syncthreads();
-    for (int k = 0; k < kSahBinPerThread; ++k) {
-        const uint32_t p = base + (uint32_t)k * kThreads + threadIdx.x;
-        if (p < n && task_of[p] >= 0) {
-            atomicMin(&s_first, p);
-            break;
-        }
-    }
-    __syncthreads();
-    if (s_first == 0xffffffffu) return;
-    const int main_task = task_of[s_first];
-    for (int k = 0; k < kSahBinPerThread; ++k) {
-        const uint32_t p = base + (uint32_t)k * kThreads + threadIdx.x;
-        if (p >= n) break;
-        const int t = task_of[p];
-        if (t < 0) continue;
-        const int prim = ids[p];
-        const float4 lo = leaf_lo[prim], hi = leaf_hi[prim];
-        const float3 c = sah_centroid(lo, hi);
-        const SahTask& task = tasks[t];
-        const float cc[3] = {c.x, c.y, c.z};
-        uint32_t* dst = t == main_task ? s_bins : bins + (size_t)t * kSahTaskWords;
+    int t[kSahBinPerThread];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const int b = sah_bin(cc[a], ordered_to_float(task.clo[a]), ordered_to_float(task.chi[a]));
-            sah_bin_add(dst + (a * kSahBins + b) * kSahBinWords, lo, hi, c);
-        }
+    for (int k = 0; k < kSahBinPerThread; ++k) {
+        const uint32_t p = base + (uint32_t)k * kThreads + threadIdx.x;
+        t[k] = p < n ? task_of[p] : -1;
+        const unsigned live = __ballot_sync(0xffffffffu, t[k] >= 0);
+        if (live != 0u && (threadIdx.x & 31u) == (uint32_t)__ffs(live) - 1u) atomicMin(&s_first[0], p);
     }
     __syncthreads();
-    uint32_t* g = bins + (size_t)main_task * kSahTaskWords;
-    for (int i = threadIdx.x; i < kSahTaskWords; i += kThreads) {
-        const int w = i % kSahBinWords;
-        const uint32_t v = s_bins[i];
-        if (w < 3 || (w >= 6 && w < 9)) {
-            if (v != 0xffffffffu) atomicMin(g + i, v);
-        } else if (v != 0u) {
-            if (w == 12) atomicAdd(g + i, v);
-            else atomicMax(g + i, v);
+    if (s_first[0] == 0xffffffffu) return;
+    const int first_task = task_of[s_first[0]];
+#pragma unroll
+    for (int k = 0; k < kSahBinPerThread; ++k) {
+        const uint32_t p = base + (uint32_t)k * kThreads + threadIdx.x;
+        const unsigned other = __ballot_sync(0xffffffffu, t[k] >= 0 && t[k] != first_task);
+        if (other != 0u && (threadIdx.x & 31u) == (uint32_t)__ffs(other) - 1u) atomicMin(&s_first[1], p);
+    }
+    __syncthreads();
+    const int second_task = s_first[1] == 0xffffffffu ? -1 : task_of[s_first[1]];
+#pragma unroll
+    for (int k = 0; k < kSahBinPerThread; ++k) {
+        const uint32_t p = base + (uint32_t)k * kThreads + threadIdx.x;
+        const int set = t[k] < 0 ? -1 : t[k] == first_task ? 0 : t[k] == second_task ? 1 : -1;
+        float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+        float3 c = make_float3(0.0f, 0.0f, 0.0f);
+        int bin[3] = {0, 0, 0};
+        if (set >= 0) {
+            const int prim = ids[p];
+            lo = leaf_lo[prim];
+            hi = leaf_hi[prim];
+            c = sah_centroid(lo, hi);
+            const SahTask& task = tasks[t[k]];
+            const float cc[3] = {c.x, c.y, c.z};
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                bin[a] = sah_bin(cc[a], ordered_to_float(task.clo[a]), ordered_to_float(task.chi[a]));
+        }
+        sah_bins_add(s_bins, set, lo, hi, c, bin);
+    }
+    __syncthreads();
+    for (int set = 0; set < 2; ++set) {
+        const int task = set ? second_task : first_task;
+        if (task < 0) break;
+        uint32_t* g = bins + (size_t)task * kSahTaskWords;
+        for (int i = threadIdx.x; i < kSahTaskWords; i += kThreads) {
+            const int w = i % kSahBinWords;
+            const uint32_t v = s_bins[set * kSahTaskWords + i];
+            if (w < 3 || (w >= 6 && w < 9)) {
+                if (v != 0xffffffffu) atomicMin(g + i, v);
+            } else if (v != 0u) {
+                if (w == 12) atomicAdd(g + i, v);
+                else atomicMax(g + i, v);
+            }
         }
     }
 }
 
-// One warp per large node, lane b holding bin b of each axis: the node's box
-// (the union of its axis-0 bins), the best split (left and right sweeps as
-// warp scans of the bins' ordered-int boxes and counts; the first minimum over
-// axes 0..2, then bins 0..30), and the children, which lane 0 allocates:
-// interior ids, next-level or small tasks.
+// The split of a node from its bins, by a warp, lane b holding bin b of each
+// axis: left and right sweeps as warp scans of the bins' ordered-int boxes and
+// counts; the first minimum over axes 0..2, then bins 0..30.
+struct SahSplit {
+    int axis;  // -1: halve the range
+    uint32_t bin, left;
+    uint32_t cb[2][6];  // children's centroid bounds
+};
+
 static_assert(kSahBins == 32, "one bin per lane");
-__global__ void __launch_bounds__(128) k_sah_split(const uint32_t* __restrict__ count, SahTask* __restrict__ tasks,
-                            const uint32_t* __restrict__ bins, SahTask* __restrict__ next, SahSmall* __restrict__ small,
-                            SahCounters* __restrict__ ctr, SahLimits lim, int2* __restrict__ children,
-                            int* __restrict__ node_parent, float4* __restrict__ node_lo, float4* __restrict__ node_hi) {
+__device__ __forceinline__ SahSplit sah_best_split(const uint32_t* tb, uint32_t count, const uint32_t clo[3],
+                                                   const uint32_t chi[3]) {
     constexpr uint32_t kFull = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (t >= *count) return;  // the whole warp leaves together
-    SahTask task = tasks[t];
-    const uint32_t* tb = bins + (size_t)t * kSahTaskWords;
-    {
-        const uint32_t* w = tb + lane * kSahBinWords;
-        uint32_t box[6];
-        for (int k = 0; k < 3; ++k) {
-            box[k] = __reduce_min_sync(kFull, w[k]);
-            box[3 + k] = __reduce_max_sync(kFull, w[3 + k]);
-        }
-        if (lane == 0) {
-            node_lo[task.node] =
-                make_float4(ordered_to_float(box[0]), ordered_to_float(box[1]), ordered_to_float(box[2]), 0.f);
-            node_hi[task.node] =
-                make_float4(ordered_to_float(box[3]), ordered_to_float(box[4]), ordered_to_float(box[5]), 0.f);
-        }
-    }
+    SahSplit out;
     float best_cost = INFINITY;
     int best_axis = -1, best_bin = 0;
     for (int a = 0; a < 3; ++a) {
-        const float ext = ordered_to_float(task.chi[a]) - ordered_to_float(task.clo[a]);
+        const float ext = ordered_to_float(chi[a]) - ordered_to_float(clo[a]);
         if (!(ext > 0.0f)) continue;  // uniform across the warp
         const uint32_t* w = tb + (a * kSahBins + lane) * kSahBinWords;
         // empty bins hold the identities (min fields all ones, max fields 0)
@@ -1087,28 +1139,80 @@ __global__ void __launch_bounds__(128) k_sah_split(const uint32_t* __restrict__ 
             best_bin = __ffs(__ballot_sync(kFull, cost == m)) - 1;  // the first bin reaching it
         }
     }
-    uint32_t left = task.count / 2u;
-    uint32_t cb[2][6];  // children's centroid bounds
+    uint32_t left = count / 2u;
     if (best_axis >= 0) {
         const uint32_t* w = tb + (best_axis * kSahBins + lane) * kSahBinWords;
         const bool in_left = (int)lane <= best_bin;
         left = __reduce_add_sync(kFull, in_left ? w[12] : 0u);
         for (int k = 0; k < 3; ++k) {
-            cb[0][k] = __reduce_min_sync(kFull, in_left ? w[6 + k] : 0xffffffffu);
-            cb[0][3 + k] = __reduce_max_sync(kFull, in_left ? w[9 + k] : 0u);
-            cb[1][k] = __reduce_min_sync(kFull, in_left ? 0xffffffffu : w[6 + k]);
-            cb[1][3 + k] = __reduce_max_sync(kFull, in_left ? 0u : w[9 + k]);
+            out.cb[0][k] = __reduce_min_sync(kFull, in_left ? w[6 + k] : 0xffffffffu);
+            out.cb[0][3 + k] = __reduce_max_sync(kFull, in_left ? w[9 + k] : 0u);
+            out.cb[1][k] = __reduce_min_sync(kFull, in_left ? 0xffffffffu : w[6 + k]);
+            out.cb[1][3 + k] = __reduce_max_sync(kFull, in_left ? 0u : w[9 + k]);
         }
     } else {
         for (int s = 0; s < 2; ++s)
             for (int k = 0; k < 3; ++k) {
-                cb[s][k] = task.clo[k];
-                cb[s][3 + k] = task.chi[k];
+                out.cb[s][k] = clo[k];
+                out.cb[s][3 + k] = chi[k];
             }
     }
+    out.axis = best_axis;
+    out.bin = (uint32_t)best_bin;
+    out.left = left;
+    return out;
+}
+
+// A node's box: the union of its axis-0 bins.
+__device__ __forceinline__ void sah_store_box(const uint32_t* tb, int node, float4* node_lo, float4* node_hi) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t* w = tb + lane * kSahBinWords;
+    uint32_t box[6];
+    for (int k = 0; k < 3; ++k) {
+        box[k] = __reduce_min_sync(kFull, w[k]);
+        box[3 + k] = __reduce_max_sync(kFull, w[3 + k]);
+    }
+    if (lane == 0) {
+        node_lo[node] = make_float4(ordered_to_float(box[0]), ordered_to_float(box[1]), ordered_to_float(box[2]), 0.f);
+        node_hi[node] = make_float4(ordered_to_float(box[3]), ordered_to_float(box[4]), ordered_to_float(box[5]), 0.f);
+    }
+}
+
+__device__ __forceinline__ SahTask sah_task(uint32_t first, uint32_t count, int node, const uint32_t cb[6]) {
+    SahTask c;
+    c.first = first;
+    c.count = count;
+    c.node = node;
+    c.axis = -1;
+    for (int k = 0; k < 3; ++k) {
+        c.clo[k] = cb[k];
+        c.chi[k] = cb[3 + k];
+    }
+    c.split_bin = 0u;
+    c.left_count = 0u;
+    c.child_task[0] = c.child_task[1] = -1;
+    return c;
+}
+
+// One warp per large node: its box, the best split, and the children, which
+// lane 0 allocates: interior ids, next-level, mid or small tasks.
+__global__ void __launch_bounds__(128) k_sah_split(const uint32_t* __restrict__ count, SahTask* __restrict__ tasks,
+                            const uint32_t* __restrict__ bins, SahTask* __restrict__ next, SahTask* __restrict__ mid,
+                            SahSmall* __restrict__ small, SahCounters* __restrict__ ctr, SahLimits lim,
+                            int2* __restrict__ children, int* __restrict__ node_parent, float4* __restrict__ node_lo,
+                            float4* __restrict__ node_hi) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (t >= *count) return;  // the whole warp leaves together
+    SahTask task = tasks[t];
+    const uint32_t* tb = bins + (size_t)t * kSahTaskWords;
+    sah_store_box(tb, task.node, node_lo, node_hi);
+    const SahSplit split = sah_best_split(tb, task.count, task.clo, task.chi);
+    const uint32_t left = split.left;
     if (lane != 0u) return;
-    task.axis = best_axis;
-    task.split_bin = (uint32_t)best_bin;
+    task.axis = split.axis;
+    task.split_bin = split.bin;
     task.left_count = left;
     const uint32_t counts[2] = {left, task.count - left};
     int refs[2] = {0, 0};
@@ -1123,26 +1227,21 @@ __global__ void __launch_bounds__(128) k_sah_split(const uint32_t* __restrict__ 
         refs[s] = id;
         node_parent[id] = task.node;
         const uint32_t first = task.first + (s ? left : 0u);
-        if (counts[s] > kSahSeqMax) {
+        if (counts[s] > kSahMidMax) {
             const uint32_t ti = atomicAdd(&ctr->large, 1u);
             if (ti >= lim.large) {
                 atomicOr(&ctr->overflow, 2u);
                 continue;
             }
-            SahTask c;
-            c.first = first;
-            c.count = counts[s];
-            c.node = id;
-            c.axis = -1;
-            for (int k = 0; k < 3; ++k) {
-                c.clo[k] = cb[s][k];
-                c.chi[k] = cb[s][3 + k];
-            }
-            c.split_bin = 0u;
-            c.left_count = 0u;
-            c.child_task[0] = c.child_task[1] = -1;
-            next[ti] = c;
+            next[ti] = sah_task(first, counts[s], id, split.cb[s]);
             task.child_task[s] = (int)ti;
+        } else if (counts[s] > kSahSeqMax) {
+            const uint32_t mi = atomicAdd(&ctr->mid, 1u);
+            if (mi >= lim.mid) {
+                atomicOr(&ctr->overflow, 32u);
+                continue;
+            }
+            mid[mi] = sah_task(first, counts[s], id, split.cb[s]);
         } else {
             const uint32_t si = atomicAdd(&ctr->small, 1u);
             if (si >= lim.small) {
@@ -1215,6 +1314,167 @@ __global__ void k_sah_scatter(uint32_t n, const int* __restrict__ ids, const int
         else children[task.node].y = ~prim;
         leaf_parent[prim] = task.node;
     }
+}
+
+// A block builds a mid node down to small ones: its triangles' order lies in
+// shared memory, a stack holds the nodes still to split, and each is binned,
+// split by the first warp and partitioned stably, as the large ones are.
+// What bounds it is the chain of nodes a block walks, six barriers each. With it
+// the 200k-triangle build has 10 levels over the whole GPU instead of 16, each
+// six launches and a readback: rebuild 2.85 -> 2.07 ms, this kernel 0.17 ms
+// (with k_sah_bin's gain).
+struct MidScratch {
+    uint32_t bins[kSahTaskWords];
+    int ids[kSahMidMax];
+    SahTask stack[kSahMidMax / (kSahSeqMax + 1u) + 1u];  // disjoint ranges of more than kSahSeqMax
+    SahTask task;
+    uint32_t chunk_left[kSahMidMax / 32u];
+    int depth;
+};
+
+__global__ void __launch_bounds__(kThreads) k_sah_mid(const SahTask* __restrict__ mid, int* __restrict__ ids,
+                                                      const float4* __restrict__ leaf_lo,
+                                                      const float4* __restrict__ leaf_hi, SahSmall* __restrict__ small,
+                                                      SahCounters* __restrict__ ctr, SahLimits lim,
+                                                      int2* __restrict__ children, int* __restrict__ node_parent,
+                                                      int* __restrict__ leaf_parent, float4* __restrict__ node_lo,
+                                                      float4* __restrict__ node_hi) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    constexpr int kPer = (int)kSahMidMax / kThreads;
+    constexpr uint32_t kWarps = kThreads / 32;
+    static_assert(kPer * (int)kWarps == 32, "one chunk of 32 positions per lane");
+    __shared__ MidScratch m;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t base = mid[blockIdx.x].first, total = mid[blockIdx.x].count;
+    if (total > kSahMidMax) {
+        if (threadIdx.x == 0) atomicOr(&ctr->overflow, 32u);
+        return;  // the whole block
+    }
+    for (uint32_t r = threadIdx.x; r < total; r += kThreads) m.ids[r] = ids[base + r];
+    if (threadIdx.x == 0) {
+        m.stack[0] = mid[blockIdx.x];
+        m.depth = 1;
+    }
+    for (;;) {
+        __syncthreads();
+        const int depth = m.depth;
+        if (depth == 0) break;
+        const uint32_t first = m.stack[depth - 1].first - base, cnt = m.stack[depth - 1].count;
+        const int node = m.stack[depth - 1].node;
+        float clo[3], chi[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            clo[a] = ordered_to_float(m.stack[depth - 1].clo[a]);
+            chi[a] = ordered_to_float(m.stack[depth - 1].chi[a]);
+        }
+        for (int i = threadIdx.x; i < kSahTaskWords; i += kThreads) {
+            const int w = i % kSahBinWords;
+            m.bins[i] = (w < 3 || (w >= 6 && w < 9)) ? 0xffffffffu : 0u;
+        }
+        __syncthreads();
+        int prim[kPer];
+        uint32_t bins[kPer];  // axis a in byte a
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const uint32_t r = (uint32_t)k * kThreads + threadIdx.x;
+            prim[k] = 0;
+            bins[k] = 0u;
+            if ((uint32_t)k * kThreads + 32u * warp >= cnt) continue;  // the whole warp
+            float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+            float3 c = make_float3(0.0f, 0.0f, 0.0f);
+            int bin[3] = {0, 0, 0};
+            if (r < cnt) {
+                prim[k] = m.ids[first + r];
+                lo = leaf_lo[prim[k]];
+                hi = leaf_hi[prim[k]];
+                c = sah_centroid(lo, hi);
+                const float cc[3] = {c.x, c.y, c.z};
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    bin[a] = sah_bin(cc[a], clo[a], chi[a]);
+                    bins[k] |= (uint32_t)bin[a] << (8 * a);
+                }
+            }
+            sah_bins_add(m.bins, r < cnt ? 0 : -1, lo, hi, c, bin);
+        }
+        __syncthreads();
+        if (warp == 0u) {
+            SahTask task = m.stack[depth - 1];
+            sah_store_box(m.bins, node, node_lo, node_hi);
+            const SahSplit split = sah_best_split(m.bins, cnt, task.clo, task.chi);
+            if (lane == 0u) {
+                task.axis = split.axis;
+                task.split_bin = split.bin;
+                task.left_count = split.left;
+                const uint32_t counts[2] = {split.left, cnt - split.left};
+                int d = depth - 1;
+                for (int s = 0; s < 2; ++s) {
+                    if (counts[s] == 1u) continue;  // a leaf: the partition writes it
+                    const int id = (int)atomicAdd(&ctr->nodes, 1u);
+                    if ((uint32_t)id >= lim.nodes) {
+                        atomicOr(&ctr->overflow, 1u);
+                        continue;
+                    }
+                    node_parent[id] = node;
+                    if (s == 0) children[node].x = id;
+                    else children[node].y = id;
+                    const uint32_t f = task.first + (s ? split.left : 0u);
+                    if (counts[s] > kSahSeqMax) {
+                        m.stack[d++] = sah_task(f, counts[s], id, split.cb[s]);
+                    } else {
+                        const uint32_t si = atomicAdd(&ctr->small, 1u);
+                        if (si >= lim.small) {
+                            atomicOr(&ctr->overflow, 4u);
+                            continue;
+                        }
+                        small[si] = SahSmall{f, counts[s], id};
+                    }
+                }
+                m.depth = d;
+                m.task = task;
+            }
+        }
+        __syncthreads();
+        const int axis = m.task.axis;
+        const uint32_t split_bin = m.task.split_bin, left = m.task.left_count;
+        uint32_t to_left[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const uint32_t r = (uint32_t)k * kThreads + threadIdx.x;
+            const bool goes = axis < 0 ? r < left : ((bins[k] >> (8 * axis)) & 0xffu) <= split_bin;
+            to_left[k] = __ballot_sync(kFull, r < cnt && goes);
+            if (lane == 0u) m.chunk_left[(uint32_t)k * kWarps + warp] = (uint32_t)__popc(to_left[k]);
+        }
+        __syncthreads();
+        // left ones before each chunk of 32 positions
+        const uint32_t mine = m.chunk_left[lane];
+        uint32_t before = mine;
+        for (uint32_t d = 1u; d < 32u; d <<= 1) {
+            const uint32_t up = __shfl_up_sync(kFull, before, d);
+            if (lane >= d) before += up;
+        }
+        const uint32_t all = __shfl_sync(kFull, before, 31);
+        before -= mine;
+        if (all != left) {  // the flags and the bins disagree: stop before writing
+            if (threadIdx.x == 0) atomicOr(&ctr->overflow, 8u);
+            break;  // the whole block
+        }
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const uint32_t r = (uint32_t)k * kThreads + threadIdx.x;
+            const uint32_t start = __shfl_sync(kFull, before, (uint32_t)k * kWarps + warp);
+            if (r >= cnt) continue;
+            const uint32_t rank = start + (uint32_t)__popc(to_left[k] & ((1u << lane) - 1u));
+            const bool goes = ((to_left[k] >> lane) & 1u) != 0u;
+            m.ids[first + (goes ? rank : left + (r - rank))] = prim[k];
+            if ((goes ? left : cnt - left) == 1u) {
+                if (goes) children[node].x = ~prim[k];
+                else children[node].y = ~prim[k];
+                leaf_parent[prim[k]] = node;
+            }
+        }
+    }
+    for (uint32_t r = threadIdx.x; r < total; r += kThreads) ids[base + r] = m.ids[r];
 }
 
 // One warp builds the whole subtree of a small node, with the same split rule.
@@ -1464,14 +1724,15 @@ int finish_binary(NanContext* ctx, uint32_t n, const float4* tris_sorted, const 
 
 // Binned-SAH hierarchy over the leaves (kernels k_sah_*): large nodes level by
 // level, one host readback of the next level's node count per level, then
-// the small nodes in one launch; the root is interior node 0.
+// the mid nodes and the small nodes in one launch each; the root is interior
+// node 0.
 int build_binned(NanContext* ctx, uint32_t n, const float4* tris_sorted, const float4* leaf_lo,
                  const float4* leaf_hi, int2* children, int* node_parent, int* leaf_parent, float4* node_lo,
                  float4* node_hi, uint32_t* arrivals, uint32_t* depth, double* sah, const Bounds* bounds,
                  cudaStream_t s) {
     cudaError_t err = cudaSuccess;
-    const uint32_t max_large = n / (kSahSeqMax + 1u) + 1u;
-    const SahLimits lim{max_large, n / 2u + 1u, n - 1u};
+    const uint32_t max_large = n / (kSahMidMax + 1u) + 1u, max_mid = n / (kSahSeqMax + 1u) + 1u;
+    const SahLimits lim{max_large, n / 2u + 1u, n - 1u, max_mid};
     int* ids_a = dmalloc<int>(n, s, &err);
     int* ids_b = dmalloc<int>(n, s, &err);
     int* task_a = dmalloc<int>(n, s, &err);
@@ -1480,6 +1741,7 @@ int build_binned(NanContext* ctx, uint32_t n, const float4* tris_sorted, const f
     uint32_t* rank = dmalloc<uint32_t>(n + 1, s, &err);
     SahTask* level_a = dmalloc<SahTask>(max_large, s, &err);
     SahTask* level_b = dmalloc<SahTask>(max_large, s, &err);
+    SahTask* mid = dmalloc<SahTask>(max_mid, s, &err);
     SahSmall* small = dmalloc<SahSmall>(n / 2u + 1u, s, &err);
     uint32_t* bins = dmalloc<uint32_t>((size_t)max_large * kSahTaskWords, s, &err);
     SahCounters* ctr = dmalloc<SahCounters>(1, s, &err);
@@ -1489,7 +1751,7 @@ int build_binned(NanContext* ctx, uint32_t n, const float4* tris_sorted, const f
     void* scan_tmp = dmalloc<uint8_t>(scan_bytes, s, &err);
     auto release = [&] {
         for (void* p : {(void*)ids_a, (void*)ids_b, (void*)task_a, (void*)task_b, (void*)flags, (void*)rank,
-                        (void*)level_a, (void*)level_b, (void*)small, (void*)bins, (void*)ctr, (void*)root_dev,
+                        (void*)level_a, (void*)level_b, (void*)mid, (void*)small, (void*)bins, (void*)ctr, (void*)root_dev,
                         scan_tmp})
             if (p) cudaFreeAsync(p, s);
     };
@@ -1506,10 +1768,10 @@ int build_binned(NanContext* ctx, uint32_t n, const float4* tris_sorted, const f
     if (err != cudaSuccess) return fail(err, "binned SAH scratch allocation");
     cudaMemsetAsync(root_dev, 0, sizeof(int), s);
     cudaMemsetAsync(node_parent, 0xff, (n - 1u) * sizeof(int), s);  // the root's parent stays -1
-    k_sah_init<<<blocks(n), kThreads, 0, s>>>(n, ids_a, task_a, n > kSahSeqMax ? 0 : -1);
-    k_sah_root<<<1, 1, 0, s>>>(n, bounds, level_a, small, ctr);
+    k_sah_init<<<blocks(n), kThreads, 0, s>>>(n, ids_a, task_a, n > kSahMidMax ? 0 : -1);
+    k_sah_root<<<1, 1, 0, s>>>(n, bounds, level_a, mid, small, ctr);
     ctx->launches += 2;
-    uint32_t large = n > kSahSeqMax ? 1u : 0u;
+    uint32_t large = n > kSahMidMax ? 1u : 0u;
     int levels = 0;
     const uint32_t bin_grid = (uint32_t)((n + kThreads * kSahBinPerThread - 1) / (kThreads * kSahBinPerThread));
     while (large > 0u) {
@@ -1517,8 +1779,8 @@ int build_binned(NanContext* ctx, uint32_t n, const float4* tris_sorted, const f
         const uint32_t words = large * (uint32_t)kSahTaskWords;
         k_sah_bins_reset<<<blocks(words), kThreads, 0, s>>>(words, bins);
         k_sah_bin<<<bin_grid, kThreads, 0, s>>>(n, ids_a, task_a, level_a, leaf_lo, leaf_hi, bins);
-        k_sah_split<<<(large * 32u + 127u) / 128u, 128, 0, s>>>(&ctr->level, level_a, bins, level_b, small, ctr, lim,
-                                                                children, node_parent, node_lo, node_hi);
+        k_sah_split<<<(large * 32u + 127u) / 128u, 128, 0, s>>>(&ctr->level, level_a, bins, level_b, mid, small, ctr,
+                                                                lim, children, node_parent, node_lo, node_hi);
         k_sah_flags<<<blocks(n + 1), kThreads, 0, s>>>(n, ids_a, task_a, level_a, leaf_lo, leaf_hi, flags);
         cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, flags, rank, n + 1, s);
         k_sah_scatter<<<blocks(n), kThreads, 0, s>>>(n, ids_a, task_a, level_a, flags, rank, ids_b, task_b, children,
@@ -1541,6 +1803,16 @@ int build_binned(NanContext* ctx, uint32_t n, const float4* tris_sorted, const f
     err = cudaMemcpyAsync(&c, ctr, sizeof(SahCounters), cudaMemcpyDeviceToHost, s);
     if (err == cudaSuccess) err = cudaStreamSynchronize(s);
     if (err != cudaSuccess) return fail(err, "binned SAH counters");
+    if (c.overflow != 0u || c.mid > max_mid) return limit("binned SAH build exceeded a bound of its node lists");
+    if (c.mid > 0u) {
+        k_sah_mid<<<c.mid, kThreads, 0, s>>>(mid, ids_a, leaf_lo, leaf_hi, small, ctr, lim, children, node_parent,
+                                             leaf_parent, node_lo, node_hi);
+        ctx->launches++;
+        err = cudaMemcpyAsync(&c, ctr, sizeof(SahCounters), cudaMemcpyDeviceToHost, s);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+        if (err != cudaSuccess) return fail(err, "binned SAH mid nodes");
+        if (c.overflow != 0u) return limit("binned SAH build exceeded a bound of its node lists");
+    }
     if (c.small > 0u) {
         k_sah_small<<<(c.small + kSmallWarps - 1u) / kSmallWarps, 32 * kSmallWarps, 0, s>>>(&ctr->small, small, ids_a, leaf_lo, leaf_hi, ctr, lim,
                                                              children, node_parent, leaf_parent, node_lo, node_hi);
