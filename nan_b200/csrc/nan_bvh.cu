@@ -655,167 +655,227 @@ __global__ void k_wide_root(const int* __restrict__ root, WideItem* __restrict__
 
 // One level of the wide conversion: *count_in items of this level in, the
 // next level's items appended at *count_out (counters[0] and [1] count the
-// wide nodes and triangles written so far).
-__global__ void k_wide_level(const WideItem* __restrict__ items, const uint32_t* __restrict__ count_in,
-                             WideItem* __restrict__ items_out, uint32_t* __restrict__ count_out,
-                             uint32_t* __restrict__ counters, const int2* __restrict__ children,
-                             const float4* __restrict__ node_lo, const float4* __restrict__ node_hi,
-                             const float4* __restrict__ leaf_lo, const float4* __restrict__ leaf_hi,
-                             const SubtreeInfo* __restrict__ info, const uint32_t* __restrict__ tri_off,
-                             const uint32_t* __restrict__ tri_pos, const float4* __restrict__ tris_dfs,
-                             const Bounds* __restrict__ bounds, uint4* __restrict__ wnodes,
-                             float4* __restrict__ wtris) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= *count_in) return;
-    const WideItem it = items[k];
-    int ent[8];
-    float4 elo[8], ehi[8];
-    int m = 0;
-    if (expandable(it.bnode, info)) {
-        const int2 ch = children[it.bnode];
-        ent[0] = ch.x;
-        ent[1] = ch.y;
-        m = 2;
-    } else {
-        ent[0] = it.bnode;  // a root that is a single leaf
-        m = 1;
+// wide nodes and triangles written so far). Eight lanes take a node: a lane
+// holds an entry while the node opens, then the child of its slot. Space for
+// the children is taken from the counters once a block. With one thread a node
+// the entries, scores and bytes lay in local memory and every node queued at
+// the counters: 200k triangles,
+// 8 levels, 532 us; 143 us in this form.
+constexpr int kWideLanes = 8;
+
+__global__ void __launch_bounds__(kThreads) k_wide_level(
+    const WideItem* __restrict__ items, const uint32_t* __restrict__ count_in, WideItem* __restrict__ items_out,
+    uint32_t* __restrict__ count_out, uint32_t* __restrict__ counters, const int2* __restrict__ children,
+    const float4* __restrict__ node_lo, const float4* __restrict__ node_hi, const float4* __restrict__ leaf_lo,
+    const float4* __restrict__ leaf_hi, const SubtreeInfo* __restrict__ info, const uint32_t* __restrict__ tri_off,
+    const uint32_t* __restrict__ tri_pos, const float4* __restrict__ tris_dfs, const Bounds* __restrict__ bounds,
+    uint4* __restrict__ wnodes, float4* __restrict__ wtris) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    __shared__ uint32_t s_count[2], s_base[3];
+    const uint32_t count = *count_in;
+    if ((uint64_t)blockIdx.x * (kThreads / kWideLanes) >= count) return;  // the whole block
+    if (threadIdx.x < 2) s_count[threadIdx.x] = 0u;
+    const uint32_t lane = threadIdx.x & 31u, sl = lane & 7u, group = lane & 24u;
+    const uint32_t k = blockIdx.x * (kThreads / kWideLanes) + threadIdx.x / kWideLanes;
+    const bool live = k < count;
+    const WideItem it = live ? items[k] : WideItem{0, 0u};
+    // entries: lane i of the group holds entry i < m
+    int ent = 0;
+    bool inner = false;  // the entry can be opened
+    float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+    auto take = [&](int c) {
+        ent = c;
+        inner = expandable(c, info);
+        entry_box(c, node_lo, node_hi, leaf_lo, leaf_hi, &lo, &hi);
+    };
+    uint32_t m = 0u;
+    if (live) {
+        if (expandable(it.bnode, info)) {
+            const int2 ch = children[it.bnode];
+            if (sl < 2u) take(sl ? ch.y : ch.x);
+            m = 2u;
+        } else {  // a root that is a single leaf
+            if (sl == 0u) take(it.bnode);
+            m = 1u;
+        }
     }
-    for (int i = 0; i < m; ++i) entry_box(ent[i], node_lo, node_hi, leaf_lo, leaf_hi, &elo[i], &ehi[i]);
-    while (m < 8) {
-        int best = -1;
-        float best_area = -1.0f;
-        for (int i = 0; i < m; ++i) {
-            if (!expandable(ent[i], info)) continue;
-            const float a = half_area4(elo[i], ehi[i]);
-            if (a > best_area) {
-                best_area = a;
-                best = i;
+    // open the largest entry (the first of equals) while there is room
+    for (int step = 0; step < kWideLanes - 1; ++step) {
+        float area = -1.0f;
+        if (sl < m && inner) {
+            const float x = half_area4(lo, hi);
+            area = x > -1.0f ? x : -1.0f;
+        }
+        float most = area;
+#pragma unroll
+        for (int d = 1; d < kWideLanes; d <<= 1) most = fmaxf(most, __shfl_xor_sync(kFull, most, d));
+        const uint32_t hits = (__ballot_sync(kFull, area == most) >> group) & 0xffu;
+        const uint32_t best = (uint32_t)__ffs(hits) - 1u;
+        const bool open = live && m < (uint32_t)kWideLanes && most > -1.0f;
+        if (__ballot_sync(kFull, open) == 0u) break;
+        int2 ch = make_int2(0, 0);
+        if (open && sl == best) ch = children[ent];
+        const int second = __shfl_sync(kFull, ch.y, (int)(group + (best & 7u)));
+        if (open) {
+            if (sl == best) take(ch.x);
+            else if (sl == m) take(second);
+            ++m;
+        }
+    }
+    // node box, over the entries in order
+    float4 plo = lo, phi = hi;
+    {
+        const bool has = sl < m;
+        float v[6] = {has ? lo.x : INFINITY, has ? lo.y : INFINITY, has ? lo.z : INFINITY,
+                      has ? -hi.x : INFINITY, has ? -hi.y : INFINITY, has ? -hi.z : INFINITY};
+#pragma unroll
+        for (int d = 1; d < kWideLanes; d <<= 1)
+#pragma unroll
+            for (int q = 0; q < 6; ++q) v[q] = fminf(v[q], __shfl_xor_sync(kFull, v[q], d));
+        plo = make_float4(v[0], v[1], v[2], 0.0f);
+        phi = make_float4(-v[3], -v[4], -v[5], 0.0f);
+    }
+    // slots by octant direction of each entry's centre: the best (entry, slot)
+    // pair left, the first of equals, m times; lane `slot` notes its entry
+    const float vx = 0.5f * (lo.x + hi.x) - 0.5f * (plo.x + phi.x);
+    const float vy = 0.5f * (lo.y + hi.y) - 0.5f * (plo.y + phi.y);
+    const float vz = 0.5f * (lo.z + hi.z) - 0.5f * (plo.z + phi.z);
+    uint32_t free_slots = 0xffu;
+    bool placed = !(sl < m);
+    int entry_of = -1;
+    for (int r = 0; r < kWideLanes; ++r) {
+        const bool more = (uint32_t)r < m;
+        if (__ballot_sync(kFull, more) == 0u) break;
+        float score = -INFINITY;
+        uint32_t slot = (uint32_t)__ffs(free_slots) - 1u;
+        bool first = true;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const float x = ((q & 1) ? vx : -vx) + ((q & 2) ? vy : -vy) + ((q & 4) ? vz : -vz);
+            if (((free_slots >> q) & 1u) && (first || x > score)) {
+                score = x;
+                slot = (uint32_t)q;
+                first = false;
             }
         }
-        if (best < 0) break;
-        const int2 ch = children[ent[best]];
-        ent[best] = ch.x;
-        ent[m] = ch.y;
-        entry_box(ent[best], node_lo, node_hi, leaf_lo, leaf_hi, &elo[best], &ehi[best]);
-        entry_box(ent[m], node_lo, node_hi, leaf_lo, leaf_hi, &elo[m], &ehi[m]);
-        ++m;
-    }
-    // node box and slot assignment by octant direction of each child's centre
-    float4 plo = elo[0], phi = ehi[0];
-    for (int i = 1; i < m; ++i) {
-        plo = make_float4(fminf(plo.x, elo[i].x), fminf(plo.y, elo[i].y), fminf(plo.z, elo[i].z), 0.0f);
-        phi = make_float4(fmaxf(phi.x, ehi[i].x), fmaxf(phi.y, ehi[i].y), fmaxf(phi.z, ehi[i].z), 0.0f);
-    }
-    const float pcx = 0.5f * (plo.x + phi.x), pcy = 0.5f * (plo.y + phi.y), pcz = 0.5f * (plo.z + phi.z);
-    float score[8][8];
-    for (int i = 0; i < m; ++i) {
-        const float vx = 0.5f * (elo[i].x + ehi[i].x) - pcx;
-        const float vy = 0.5f * (elo[i].y + ehi[i].y) - pcy;
-        const float vz = 0.5f * (elo[i].z + ehi[i].z) - pcz;
-        for (int sl = 0; sl < 8; ++sl)
-            score[i][sl] = ((sl & 1) ? vx : -vx) + ((sl & 2) ? vy : -vy) + ((sl & 4) ? vz : -vz);
-    }
-    int slot_of[8];
-    uint32_t used_slots = 0u, done = 0u;
-    for (int r = 0; r < m; ++r) {
-        float best = -INFINITY;
-        int bi = -1, bs = -1;
-        for (int i = 0; i < m; ++i) {
-            if (done & (1u << i)) continue;
-            for (int sl = 0; sl < 8; ++sl) {
-                if (used_slots & (1u << sl)) continue;
-                if (score[i][sl] > best || bi < 0) {
-                    best = score[i][sl];
-                    bi = i;
-                    bs = sl;
-                }
-            }
+        // a NaN score counts as the lowest
+        const float mine = placed || !(score == score) ? -INFINITY : score;
+        float most = mine;
+#pragma unroll
+        for (int d = 1; d < kWideLanes; d <<= 1) most = fmaxf(most, __shfl_xor_sync(kFull, most, d));
+        const uint32_t hits = (__ballot_sync(kFull, !placed && mine == most) >> group) & 0xffu;
+        const uint32_t who = hits ? (uint32_t)__ffs(hits) - 1u : 0u;
+        const uint32_t to = __shfl_sync(kFull, slot, (int)(group + who));
+        if (more) {
+            if (sl == who) placed = true;
+            if (sl == to) entry_of = (int)who;
+            free_slots &= ~(1u << to);
         }
-        slot_of[bi] = bs;
-        done |= 1u << bi;
-        used_slots |= 1u << bs;
     }
-    int slot_ent[8];
-    for (int sl = 0; sl < 8; ++sl) slot_ent[sl] = -1;
-    for (int i = 0; i < m; ++i) slot_ent[slot_of[i]] = i;
+    // each lane's slot: its child's code, box and kind
+    const int from = (int)group + max(entry_of, 0);
+    const int child = __shfl_sync(kFull, ent, from);
+    const bool filled = entry_of >= 0;
+    const bool is_inner = (__shfl_sync(kFull, inner ? 1 : 0, from) != 0) && filled;
+    const float clo[3] = {__shfl_sync(kFull, lo.x, from), __shfl_sync(kFull, lo.y, from),
+                          __shfl_sync(kFull, lo.z, from)};
+    const float chi[3] = {__shfl_sync(kFull, hi.x, from), __shfl_sync(kFull, hi.y, from),
+                          __shfl_sync(kFull, hi.z, from)};
     // allocation: interior children and leaf triangles, both in slot order
-    uint32_t n_int = 0u, n_tri = 0u;
-    for (int sl = 0; sl < 8; ++sl) {
-        const int i = slot_ent[sl];
-        if (i < 0) continue;
-        if (expandable(ent[i], info)) ++n_int;
-        else n_tri += ent[i] < 0 ? 1u : info[ent[i]].tris;
+    const uint32_t imask = (__ballot_sync(kFull, is_inner) >> group) & 0xffu;
+    const uint32_t rank = (uint32_t)__popc(imask & ((1u << sl) - 1u)), n_int = (uint32_t)__popc(imask);
+    const uint32_t tris = !filled || is_inner ? 0u : child < 0 ? 1u : info[child].tris;
+    uint32_t toff = tris;
+#pragma unroll
+    for (uint32_t d = 1u; d < (uint32_t)kWideLanes; d <<= 1) {
+        const uint32_t up = __shfl_up_sync(kFull, toff, d, kWideLanes);
+        if (sl >= d) toff += up;
     }
-    const uint32_t child_base = n_int ? atomicAdd(&counters[0], n_int) : 0u;
-    const uint32_t tri_base = n_tri ? atomicAdd(&counters[1], n_tri) : 0u;
-    const uint32_t out_base = n_int ? atomicAdd(count_out, n_int) : 0u;
-    // quantization grid: p = node lo, scale 2^e with 255 * 2^e >= extent
+    const uint32_t n_tri = __shfl_sync(kFull, toff, (int)group + 7);
+    toff -= tris;
+    __syncthreads();
+    uint32_t at_int = 0u, at_tri = 0u;
+    if (sl == 0u) {
+        at_int = n_int ? atomicAdd(&s_count[0], n_int) : 0u;
+        at_tri = n_tri ? atomicAdd(&s_count[1], n_tri) : 0u;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t ints = s_count[0], all = s_count[1];
+        s_base[0] = ints ? atomicAdd(&counters[0], ints) : 0u;
+        s_base[1] = all ? atomicAdd(&counters[1], all) : 0u;
+        s_base[2] = ints ? atomicAdd(count_out, ints) : 0u;
+    }
+    __syncthreads();
+    at_int = __shfl_sync(kFull, at_int, (int)group);
+    at_tri = __shfl_sync(kFull, at_tri, (int)group);
+    const uint32_t child_base = s_base[0] + at_int, tri_base = s_base[1] + at_tri, out_base = s_base[2] + at_int;
+    // quantization grid: p = node lo, scale 2^e with 255 * 2^e >= extent; lane
+    // a finds axis a's
     const float pad = ordered_to_float(bounds->max_abs) * 3.814697265625e-6f + 1e-30f;
-    const double lo3[3] = {(double)plo.x - pad, (double)plo.y - pad, (double)plo.z - pad};
-    const double hi3[3] = {(double)phi.x + pad, (double)phi.y + pad, (double)phi.z + pad};
-    float p3[3];
-    int e3[3];
-    for (int a = 0; a < 3; ++a) {
-        p3[a] = (float)lo3[a];
-        if ((double)p3[a] > lo3[a]) p3[a] = nextafterf(p3[a], -INFINITY);  // p <= lo
-        const double ext = hi3[a] - (double)p3[a];
-        int e = -126;
-        if (ext > 0.0) {
-            e = (int)ceil(log2(ext / 255.0));
-            while (ldexp(255.0, e) < ext) ++e;
-            e = max(min(e, 127), -126);
-        }
-        e3[a] = e;
+    const double alo = (double)(sl == 0u ? plo.x : sl == 1u ? plo.y : plo.z) - pad;
+    const double ahi = (double)(sl == 0u ? phi.x : sl == 1u ? phi.y : phi.z) + pad;
+    float p = (float)alo;
+    if ((double)p > alo) p = nextafterf(p, -INFINITY);  // p <= lo
+    const double ext = ahi - (double)p;
+    int e = -126;
+    if (ext > 0.0) {
+        e = (int)ceil(log2(ext / 255.0));
+        while (ldexp(255.0, e) < ext) ++e;
+        e = max(min(e, 127), -126);
     }
-    uint32_t imask = 0u, rank = 0u, toff = 0u;
-    uint8_t meta[8], qlo[3][8], qhi[3][8];
-    for (int sl = 0; sl < 8; ++sl) {
-        meta[sl] = 0u;
-        for (int a = 0; a < 3; ++a) {
-            qlo[a][sl] = 1u;  // empty slot: an inverted box
-            qhi[a][sl] = 0u;
-        }
-        const int i = slot_ent[sl];
-        if (i < 0) continue;
-        const double clo[3] = {(double)elo[i].x - pad, (double)elo[i].y - pad, (double)elo[i].z - pad};
-        const double chi[3] = {(double)ehi[i].x + pad, (double)ehi[i].y + pad, (double)ehi[i].z + pad};
-        for (int a = 0; a < 3; ++a) {
-            const double sc = ldexp(1.0, e3[a]);
-            const double ql = floor((clo[a] - (double)p3[a]) / sc);
-            const double qh = ceil((chi[a] - (double)p3[a]) / sc);
-            qlo[a][sl] = (uint8_t)fmax(0.0, fmin(255.0, ql));
-            qhi[a][sl] = (uint8_t)fmax(0.0, fmin(255.0, qh));
-        }
-        const int c = ent[i];
-        if (expandable(c, info)) {
-            imask |= 1u << sl;
-            items_out[out_base + rank] = WideItem{c, child_base + rank};
-            ++rank;
+    // the child's box on the grid (a scale of 2^e divides exactly); empty slots
+    // hold an inverted box
+    uint32_t quant[6];
+    float p3[3];
+    uint32_t ebits = 0u;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        p3[a] = __shfl_sync(kFull, p, (int)group + a);
+        const int ea = __shfl_sync(kFull, e, (int)group + a);
+        ebits |= (uint32_t)(ea + 127) << (8 * a);
+        const double inv = __longlong_as_double((long long)(1023 - ea) << 52);
+        const double ql = floor((((double)clo[a] - pad) - (double)p3[a]) * inv);
+        const double qh = ceil((((double)chi[a] + pad) - (double)p3[a]) * inv);
+        quant[a] = filled ? (uint32_t)(uint8_t)fmax(0.0, fmin(255.0, ql)) : 1u;
+        quant[3 + a] = filled ? (uint32_t)(uint8_t)fmax(0.0, fmin(255.0, qh)) : 0u;
+    }
+    uint32_t meta = 0u;
+    if (live && filled) {
+        if (is_inner) {
+            items_out[out_base + rank] = WideItem{child, child_base + rank};
         } else {
-            const uint32_t cnt = c < 0 ? 1u : info[c].tris;
-            const uint32_t src = c < 0 ? tri_pos[~c] : tri_off[c];
-            for (uint32_t t = 0; t < cnt; ++t) {
+            const uint32_t src = child < 0 ? tri_pos[~child] : tri_off[child];
+            for (uint32_t t = 0; t < tris; ++t) {
                 const uint32_t d = tri_base + toff + t;
                 wtris[3u * d + 0] = tris_dfs[3u * (src + t) + 0];
                 wtris[3u * d + 1] = tris_dfs[3u * (src + t) + 1];
                 wtris[3u * d + 2] = tris_dfs[3u * (src + t) + 2];
             }
-            const uint32_t unary = cnt == 1u ? 1u : (cnt == 2u ? 3u : 7u);
-            meta[sl] = (uint8_t)((unary << 5) | toff);
-            toff += cnt;
+            meta = ((tris == 1u ? 1u : (tris == 2u ? 3u : 7u)) << 5) | toff;
         }
     }
-    auto pack4 = [](const uint8_t* b) {
-        return (uint32_t)b[0] | ((uint32_t)b[1] << 8) | ((uint32_t)b[2] << 16) | ((uint32_t)b[3] << 24);
+    // four lanes' bytes make a word
+    uint32_t* w = reinterpret_cast<uint32_t*>(wnodes + 5u * (size_t)it.wnode);
+    auto word = [&](uint32_t v) {
+        v <<= 8u * (sl & 3u);
+        v |= __shfl_xor_sync(kFull, v, 1);
+        return v | __shfl_xor_sync(kFull, v, 2);
     };
-    const uint32_t ebits = (uint32_t)(e3[0] + 127) | ((uint32_t)(e3[1] + 127) << 8) |
-                           ((uint32_t)(e3[2] + 127) << 16) | (imask << 24);
-    uint4* w = wnodes + 5u * it.wnode;
-    w[0] = make_uint4(__float_as_uint(p3[0]), __float_as_uint(p3[1]), __float_as_uint(p3[2]), ebits);
-    w[1] = make_uint4(child_base, tri_base, pack4(meta), pack4(meta + 4));
-    w[2] = make_uint4(pack4(qlo[0]), pack4(qlo[0] + 4), pack4(qlo[1]), pack4(qlo[1] + 4));
-    w[3] = make_uint4(pack4(qlo[2]), pack4(qlo[2] + 4), pack4(qhi[0]), pack4(qhi[0] + 4));
-    w[4] = make_uint4(pack4(qhi[1]), pack4(qhi[1] + 4), pack4(qhi[2]), pack4(qhi[2] + 4));
+    const uint32_t metas = word(meta);
+    uint32_t quants[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) quants[q] = word(quant[q]);
+    if (!live || (sl & 3u) != 0u) return;
+    const uint32_t half = sl >> 2;
+    if (half == 0u) {
+        *reinterpret_cast<uint4*>(w) = make_uint4(__float_as_uint(p3[0]), __float_as_uint(p3[1]),
+                                                  __float_as_uint(p3[2]), ebits | (imask << 24));
+        *reinterpret_cast<uint2*>(w + 4) = make_uint2(child_base, tri_base);
+    }
+    w[6u + half] = metas;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) w[8u + 2u * (uint32_t)q + half] = quants[q];
 }
 
 // ---------------------------------------------------------------------------
@@ -1966,7 +2026,7 @@ int finish_binary(NanContext* ctx, uint32_t n, const float4* tris_sorted, const 
                 }
                 const WideItem* in = (level & 1) ? items_b : items_a;
                 WideItem* out = (level & 1) ? items_a : items_b;
-                k_wide_level<<<blocks(bound), kThreads, 0, s>>>(in, wcount + 2 + level, out, wcount + 3 + level,
+                k_wide_level<<<blocks(bound * kWideLanes), kThreads, 0, s>>>(in, wcount + 2 + level, out, wcount + 3 + level,
                                                                 wcount, children, node_lo, node_hi, leaf_lo, leaf_hi,
                                                                 info, tri_off, tri_pos, ctx->tris, bounds,
                                                                 ctx->wnodes, ctx->wtris);
