@@ -89,10 +89,11 @@ __global__ void k_occluded(SceneView s, const float4* __restrict__ rays, uint32_
 // per sample, the table's rays leave position + normalize(normal) * bias (a
 // zero or non-finite normal: (0,0,1) and an origin one float nearer each
 // ray, as tinybvh has no t_min) and are tested for any hit in
-// [0, t_max]. One warp per sample: lanes take rays r = lane + 32 w, a ballot
-// per 32 rays leaves mask word w in lane w; lanes 0-15 then sum coefficient
-// `lane` of the unoccluded rays' weighted SH in the caster's order (64-ray
-// batches, each summed in ray order, then added to the total).
+// [0, t_max]. One warp per sample: it takes the rays 32 at a time in an order
+// that keeps neighbouring directions together and marks the unoccluded ones in
+// a mask by ray; lanes 0-15 then sum coefficient `lane` of their weighted SH in
+// the caster's order (64-ray batches, each summed in ray order, then added to
+// the total).
 // ---------------------------------------------------------------------------
 constexpr uint32_t kVisTableStride = 20;  // floats per ray: direction xyz, 0, 16 weighted SH values
 
@@ -102,8 +103,73 @@ __device__ __forceinline__ float nudge_toward(float o, float d) {
     return o;
 }
 
-// 9 blocks of 128 per SM (56 registers): 5.56 ms for 65,536 samples x 512 rays
-// on the 200k-triangle scene, against 5.77 with 8 blocks and 5.66 with 10.
+// The cell of a direction among kVisCells x kVisCells of the octahedral map, by
+// Morton code.
+constexpr uint32_t kVisCells = 16u, kVisCellCount = kVisCells * kVisCells;
+
+__device__ __forceinline__ uint32_t visibility_cell(float x, float y, float z) {
+    const float inv = 1.0f / (fabsf(x) + fabsf(y) + fabsf(z));
+    float u = x * inv, v = y * inv;
+    if (z < 0.0f) {
+        const float fu = (1.0f - fabsf(v)) * (u < 0.0f ? -1.0f : 1.0f);
+        v = (1.0f - fabsf(u)) * (v < 0.0f ? -1.0f : 1.0f);
+        u = fu;
+    }
+    const int n = (int)kVisCells;
+    uint32_t a = (uint32_t)min(max((int)((u * 0.5f + 0.5f) * (float)n), 0), n - 1);
+    uint32_t b = (uint32_t)min(max((int)((v * 0.5f + 0.5f) * (float)n), 0), n - 1);
+    uint32_t cell = 0u;
+#pragma unroll
+    for (uint32_t k = 0u; k < 4u; ++k) cell |= ((a >> k) & 1u) << (2u * k) | ((b >> k) & 1u) << (2u * k + 1u);
+    return cell;
+}
+
+// The table's rays in the order of their cells (any order within one), by the
+// whole block: a counting sort.
+__device__ __forceinline__ void visibility_order(const float* __restrict__ table, uint32_t rays, uint32_t* cells,
+                                                 uint16_t* order) {
+    for (uint32_t k = threadIdx.x; k < kVisCellCount; k += blockDim.x) cells[k] = 0u;
+    __syncthreads();
+    for (uint32_t r = threadIdx.x; r < rays; r += blockDim.x) {
+        const float* e = table + (size_t)kVisTableStride * r;
+        atomicAdd(cells + visibility_cell(__ldg(e), __ldg(e + 1), __ldg(e + 2)), 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32u) {
+        constexpr uint32_t kPer = kVisCellCount / 32u;
+        uint32_t own[kPer], sum = 0u;
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) {
+            own[k] = cells[kPer * threadIdx.x + k];
+            sum += own[k];
+        }
+        uint32_t at = sum;
+#pragma unroll
+        for (uint32_t d = 1u; d < 32u; d <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, at, d);
+            if (threadIdx.x >= d) at += up;
+        }
+        at -= sum;
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) {
+            cells[kPer * threadIdx.x + k] = at;
+            at += own[k];
+        }
+    }
+    __syncthreads();
+    for (uint32_t r = threadIdx.x; r < rays; r += blockDim.x) {
+        const float* e = table + (size_t)kVisTableStride * r;
+        order[atomicAdd(cells + visibility_cell(__ldg(e), __ldg(e + 1), __ldg(e + 2)), 1u)] = (uint16_t)r;
+    }
+    __syncthreads();
+}
+
+// What bounds it is instruction issue with few of a warp's lanes on. Any hit
+// needs no order, so a warp's rays are put together by direction; in table
+// order 32 of 512 rays span a slice from pole to pole. 65,536 samples x 512
+// rays on the 200k-triangle scene: 5.58 -> 4.94 ms (cells of half the
+// resolution 5.01). 9 blocks of 128 per SM (56 registers): 8 blocks 5.10, 10
+// 4.98 ms.
 __global__ void __launch_bounds__(128, 9) k_visibility_sh16(SceneView s, const float* __restrict__ pos,
                                                          const float* __restrict__ nrm, uint32_t n,
                                                          const float* __restrict__ table, uint32_t rays, float tmax,
@@ -112,6 +178,10 @@ __global__ void __launch_bounds__(128, 9) k_visibility_sh16(SceneView s, const f
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    __shared__ uint32_t s_cells[kVisCellCount], s_mask[4][NAN_VISIBILITY_MAX_RAYS / 32];
+    __shared__ uint16_t s_order[NAN_VISIBILITY_MAX_RAYS];
+    visibility_order(table, rays, s_cells, s_order);
+    uint32_t* mask = s_mask[threadIdx.x >> 5];
     const uint32_t words = (rays + 31u) >> 5;
     RayTally tally{0u, 0u};
     for (uint32_t i = warp; i < n; i += warps) {
@@ -125,20 +195,21 @@ __global__ void __launch_bounds__(128, 9) k_visibility_sh16(SceneView s, const f
             u = mk3(nx * inv, ny * inv, nz * inv);
         }
         const f3 o = mk3(px + u.x * bias, py + u.y * bias, pz + u.z * bias);
-        uint32_t word = 0u;
+        if (lane < words) mask[lane] = 0u;
+        __syncwarp();
         for (uint32_t w = 0; w < words; ++w) {
-            const uint32_t r = 32u * w + lane;
-            bool visible = false;
-            if (r < rays) {
+            if (32u * w + lane < rays) {
+                const uint32_t r = s_order[32u * w + lane];
                 const float* e = table + (size_t)kVisTableStride * r;
                 const f3 d = mk3(__ldg(e), __ldg(e + 1), __ldg(e + 2));
                 const f3 oo = has_normal ? o : mk3(nudge_toward(o.x, d.x), nudge_toward(o.y, d.y), nudge_toward(o.z, d.z));
-                visible = !trace_any(s, oo, d, 0.0f, tmax);
+                if (!trace_any(s, oo, d, 0.0f, tmax)) atomicOr(mask + (r >> 5), 1u << (r & 31u));
                 tally.shadow++;
             }
-            const unsigned m = __ballot_sync(0xffffffffu, visible);
-            if (lane == w) word = m;
+            __syncwarp();
         }
+        const uint32_t word = lane < words ? mask[lane] : 0u;
+        __syncwarp();
         const uint32_t seen = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(word));
         float total = 0.0f;
         for (uint32_t b = 0; b < words; b += 2u) {
