@@ -6,8 +6,9 @@ seeded 200,688-triangle scene (313x313-vertex displaced terrain + 500 boxes
 with sides U[0.2, 3] and random yaw, albedo U[0.1, 0.9]); 16 texels/unit,
 per-triangle lattice resolution 4..64, 1 hemisphere sample per texel, 3
 bounces, sun at 45 deg with irradiance 3, constant sky 0.5. One step = one
-iteration (the wavefront integrator's generate/extend/shade/shadow/finalize
-launches). Metric: Mrays/s, every closest-hit (extend) and any-hit (shadow)
+iteration (the wavefront integrator's generate, extend, shadow and stage
+launches; without kernel timing one launch traces a round's extend and shadow
+rays). Metric: Mrays/s, every closest-hit (extend) and any-hit (shadow)
 ray counted on the device. The roofline is that of the traversal kernels
 (k_wf_extend + k_wf_shadow), timed by CUDA events the library records on the
 launching stream inside the timed region.

@@ -205,7 +205,8 @@ typedef struct NanTuning {
     uint32_t bvh_width;            /* traversed nodes: 0 or 2 = binary, 8 = compressed 8-wide (SAH or PLOC builds) */
     uint32_t kernel_timing;        /* 1: record CUDA events around each wavefront stage launch on the
                                       launching stream (read with nan_ctx_read_kernel_times); not for
-                                      use under stream capture */
+                                      use under stream capture. Closest-hit and shadow rays then run
+                                      as a launch each, where 0 traces a round's both in one */
     uint32_t ray_order;            /* wavefront extend queue: 0 = path order, 1 = regrouped by ray
                                       direction octant before each extend launch */
     uint32_t traversal;            /* wavefront traversal over binary nodes, same results in every
@@ -221,7 +222,7 @@ typedef struct NanTuning {
 typedef struct NanKernelTimes {
     double extend_ms;          /* k_wf_extend: closest-hit traversal */
     double shadow_ms;          /* k_wf_shadow: any-hit traversal */
-    double stage_ms;           /* generate / shade / finalize kernels */
+    double stage_ms;           /* generate / stage kernels (shading and finalizing) */
     uint64_t extend_launches;
     uint64_t shadow_launches;
     uint64_t stage_launches;
@@ -633,7 +634,7 @@ NAN_B200_API int nan_batch_set_tuning(NanBatch* batch, const NanBatchTuning* tun
  * iteration * samples + k), so a warp traces 32 samples of one probe at once;
  * the per-probe sums are still formed in sample order. WAVEFRONT: the
  * sequential sample streams, run as one multi-scene wavefront (every probe of
- * every set one path in flight; extend / shade / shadow / finalize rounds
+ * every set one path in flight; rounds of one trace and one stage launch
  * over all sets; bit-exact with SEQUENTIAL); allocates one path of scratch
  * per probe on the batch's context; the tuning's blocks_per_sm is the
  * traversal grid. WAVEFRONT_INDEPENDENT: the INDEPENDENT sample streams on

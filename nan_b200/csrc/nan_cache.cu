@@ -243,8 +243,8 @@ constexpr int infer_smem() { return kImgBytes + kSub * kTile * kHidden * 2 + 64;
 // CTAs per SM that shared memory and the 512 TMEM columns allow.
 template <int kSub>
 constexpr int infer_ctas_per_sm() { return kSub == 1 ? 4 : kSub == 2 ? 3 : 2; }
-// Measured render + inference time of a cached 1920x1080 frame on the
-// 998k-triangle terrain: 1 tile 2.17 ms, 2 tiles 2.06 ms, 4 tiles 2.07 ms.
+// 1920x1080 queries: 2 tiles 515 us, 4 tiles 556 us (with a load a corner,
+// render + inference of a frame: 1 tile 2.17, 2 tiles 2.06, 4 tiles 2.07 ms).
 constexpr int kInferSub = 2;
 
 template <int kSub>

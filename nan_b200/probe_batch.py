@@ -14,7 +14,7 @@ each sample of a probe draws from its own RNG stream and a warp traces 32
 samples of one probe at once (a different, equally valid sample set). With
 wavefront=True the reference's sample sequence runs as one multi-scene
 wavefront: every probe of every scene is a path in flight and each
-extend / shade / shadow / finalize round covers all scenes (results equal
+trace + stage round covers all scenes (results equal
 the per-scene bakes bit for bit); with both flags every (probe, sample) is
 a path and the samples are folded in order afterwards (results equal the
 independent-sample persistent kernel's).
