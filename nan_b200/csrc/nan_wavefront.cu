@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(128, 9) k_wf_extend(Src src, const uint32_t* _
             tally.extend++;
             HitInfo h;
             if constexpr (kShared > 0 && kWidth == 2) {
-                SplitStack<kShared, 128, kTraversalStack + 1> stk;
+                SplitStack<kShared, 128, kTraversalStack + 2> stk;
                 stk.top = stack_top + threadIdx.x;
                 h = trace_closest_binary_s<kTraversalStack>(s, stk, xyz(o), xyz(d), o.w, d.w);
             } else if constexpr (kSpec && kWidth == 2) {
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(128, 9) k_wf_shadow(Src src, const float4* __r
             const SceneView s = src.of(p);
             bool blocked;
             if constexpr (kShared > 0 && kWidth == 2) {
-                SplitStack<kShared, 128, kTraversalStack + 1> stk;
+                SplitStack<kShared, 128, kTraversalStack + 2> stk;
                 stk.top = stack_top + threadIdx.x;
                 blocked = trace_any_binary_s<kTraversalStack>(s, stk, xyz(a), xyz(b), 0.0f, c.w > 0.0f ? c.w : t_max);
             } else if constexpr (kSpec && kWidth == 2) {
