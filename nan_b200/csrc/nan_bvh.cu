@@ -284,10 +284,17 @@ __device__ __forceinline__ float node_pad(const Bounds* bounds) {
 
 // Padded interval [lo - pad, hi + pad] as (centre, half extent), the half
 // extent rounded up so that the centre's rounding never shrinks the interval.
+// A half extent above kOpenExtent (or a NaN) leaves the interval open, as
+// (0, infinity): with reciprocals of up to 1e20 (box_setup) the centre's
+// product overflows for a ray well inside such an interval, and an infinite
+// near distance would cull it.
+constexpr float kOpenExtent = 1e18f;
+
 __device__ __forceinline__ float2 centre_half(float lo, float hi, float pad) {
     const float l = lo - pad, h = hi + pad;
     const float c = 0.5f * l + 0.5f * h;
-    return make_float2(c, fmaxf(__fsub_ru(h, c), __fsub_ru(c, l)));
+    const float e = fmaxf(__fsub_ru(h, c), __fsub_ru(c, l));
+    return e <= kOpenExtent ? make_float2(c, e) : make_float2(0.0f, INFINITY);
 }
 
 // The three box words of a binary node (layout: SceneView, nan_scene.cuh).
