@@ -206,7 +206,8 @@ typedef struct NanTuning {
     uint32_t kernel_timing;        /* 1: record CUDA events around each wavefront stage launch on the
                                       launching stream (read with nan_ctx_read_kernel_times); not for
                                       use under stream capture. Closest-hit and shadow rays then run
-                                      as a launch each, where 0 traces a round's both in one */
+                                      as a launch each, where 0 traces a round's both in one. Not
+                                      for a batch: nan_batch_* frames record no events */
     uint32_t ray_order;            /* wavefront extend queue: 0 = path order, 1 = regrouped by ray
                                       direction octant before each extend launch */
     uint32_t traversal;            /* wavefront traversal over binary nodes, same results in every

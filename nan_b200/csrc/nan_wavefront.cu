@@ -1480,21 +1480,24 @@ Grid grid_for(const NanContext* ctx, uint64_t paths) {
 // The traversal of round `it`: the closest hits of its walking paths and the
 // shadow rays that the round before queued, in one launch; in two (extend, then
 // shadow) for the wide nodes, the other traversal forms and stage timing.
+// timed: the pass is one that NanTuning.kernel_timing covers. The batch is not:
+// its frames are captured in graphs, whose event records cannot be read.
 template <class Src>
-void launch_trace(NanContext* ctx, int blocks, cudaStream_t st, bool wide, Src src, const WfQueues& q, uint32_t it,
-                  float t_max, const WfState& S) {
+void launch_trace(NanContext* ctx, int blocks, cudaStream_t st, bool wide, bool timed, Src src, const WfQueues& q,
+                  uint32_t it, float t_max, const WfState& S) {
     const int buf = (int)(it & 1u);
     uint32_t* ctl = q.ctl + kCtlWords * (it + 1u);
-    if (!wide && ctx->tuning.traversal == 0u && !ctx->tuning.kernel_timing) {
+    timed = timed && ctx->tuning.kernel_timing;
+    if (!wide && ctx->tuning.traversal == 0u && !timed) {
         k_wf_trace<Src><<<blocks, 128, 0, st>>>(src, q.ext[buf], ctl, S.ro, S.rd, S.hit, q.shd[buf ^ 1],
                                                 ctl - kCtlWords, t_max, S.rad, S.si, ctx->d_counters);
         ctx->launches++;
         return;
     }
-    cudaEvent_t ev = nan_host::timing_begin(ctx, st);
+    cudaEvent_t ev = timed ? nan_host::timing_begin(ctx, st) : nullptr;
     launch_extend(ctx, blocks, st, wide, src, q.ext[buf], ctl, S);
     nan_host::timing_end(ctx, 0, ev, st);
-    ev = nan_host::timing_begin(ctx, st);
+    ev = timed ? nan_host::timing_begin(ctx, st) : nullptr;
     launch_shadow(ctx, blocks, st, wide, src, q.shd[buf ^ 1], ctl - kCtlWords, t_max, S);
     nan_host::timing_end(ctx, 1, ev, st);
     ctx->launches += 2;
@@ -1673,7 +1676,7 @@ int wf_run(NanContext* ctx, cudaStream_t st, uint64_t begin, uint64_t end, uint3
                 std::swap(q.ext[buf], q.ext_sorted);
                 ctx->launches += 3;
             }
-            launch_trace(ctx, g.persistent_blocks, st, s.wnodes != nullptr, OneScene{s}, q, it, t_max, S);
+            launch_trace(ctx, g.persistent_blocks, st, s.wnodes != nullptr, true, OneScene{s}, q, it, t_max, S);
             ev = timing_begin(ctx, st);
             stage(S, q, buf, ctl, g.stream_blocks);
             timing_end(ctx, 2, ev, st);
@@ -1862,7 +1865,7 @@ int launch_batch_wavefront(NanContext* ctx, const void* sets, const uint32_t* pr
     k_wfb_probe_generate<<<(total + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(m, S, q, ctx->d_counters);
     ctx->launches++;
     for (uint32_t it = 0; it < rounds; ++it) {
-        launch_trace(ctx, g.persistent_blocks, st, false, src, q, it, t_max, S);
+        launch_trace(ctx, g.persistent_blocks, st, false, false, src, q, it, t_max, S);
         k_wfb_probe_stage<<<g.stream_blocks, kStageThreads, 0, st>>>(m, S, q, (int)(it & 1u), q.ctl + kCtlWords * (it + 1u));
         ctx->launches++;
     }
@@ -1909,7 +1912,7 @@ int launch_batch_wavefront_independent(NanContext* ctx, const void* sets, const 
         if (err != cudaSuccess) return cuda_fail(err, "batch wavefront control reset");
         k_wfi_probe_generate<<<(paths + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(m, S, q);
         for (uint32_t it = 0; it < rounds; ++it) {
-            launch_trace(ctx, g.persistent_blocks, st, false, src, q, it, t_max, S);
+            launch_trace(ctx, g.persistent_blocks, st, false, false, src, q, it, t_max, S);
             k_wfi_probe_stage<<<g.stream_blocks, kStageThreads, 0, st>>>(m, S, q, (int)(it & 1u), q.ctl + kCtlWords * (it + 1u));
         }
         k_wfi_probe_fold<<<(m.units + 127) / 128, 128, 0, st>>>(m, ctx->d_counters);
