@@ -47,6 +47,7 @@ constexpr int kCellLimit = 1 << kCellBits;
 struct WseSet {
     double d_max, inv_cell, plane_limit;
     int cmin[3];
+    uint32_t begin, end;  // its candidates, sorted or not
 };
 
 struct WseArgs {
@@ -139,9 +140,9 @@ __global__ void k_wse_keys(WseArgs a, unsigned long long* keys, uint32_t* idx, i
     idx[i] = i;
 }
 
-__device__ __forceinline__ uint32_t lower_bound_key(const unsigned long long* keys, uint32_t n,
+// First entry of [lo, hi) whose key is k or above (hi: none).
+__device__ __forceinline__ uint32_t lower_bound_key(const unsigned long long* keys, uint32_t lo, uint32_t hi,
                                                     unsigned long long k) {
-    uint32_t lo = 0, hi = n;
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
         if (keys[mid] < k) lo = mid + 1;
@@ -178,7 +179,10 @@ __device__ __forceinline__ long long wse_contribution(const WseArgs& a, double d
 // z), so the three z-neighbours of one (x, y) column are one key range), then
 // all test the ranges' candidates together. One thread a candidate spent its
 // time in nine searches of 17 dependent loads and in lanes with lists of other
-// lengths: 0.40 ms a pass over 102,400 candidates, now 0.19 ms.
+// lengths: 0.40 ms a pass over 102,400 candidates, now 0.19 ms. The searches
+// stay within the set and a range's end is found in growing steps from its
+// start: in 2,000 sets of 40 candidates, two searches of 17 steps a column
+// took 106 us a pass where one thread a candidate took 70; now 79 us.
 constexpr uint32_t kWseLanes = 16u;
 
 // Number of the calling thread's group of kLanes consecutive threads.
@@ -209,8 +213,14 @@ __global__ void k_wse_neighbors(WseArgs a, const unsigned long long* keys, const
         if (r0 >= 0 && r1 >= 0) {
             const unsigned long long column = ((unsigned long long)si << 48) | ((unsigned long long)r0 << 32) |
                                               ((unsigned long long)r1 << 16);
-            range_b = lower_bound_key(keys, a.n, column | (unsigned long long)max(rz - 1, 0));
-            range_e = lower_bound_key(keys, a.n, (column | (unsigned long long)(rz + 1)) + 1ull);
+            range_b = lower_bound_key(keys, s.begin, s.end, column | (unsigned long long)max(rz - 1, 0));
+            const unsigned long long past = (column | (unsigned long long)(rz + 1)) + 1ull;
+            uint32_t last = range_b, step = 1u;  // the range is short: its end in growing steps
+            while (step < s.end - last && keys[last + step] < past) {
+                last += step;
+                step *= 2u;
+            }
+            range_e = lower_bound_key(keys, last, min(last + step, s.end), past);
         }
     }
     uint32_t count = 0u;
@@ -252,13 +262,18 @@ constexpr long long kWseGone = -0x7fffffffffffffffLL - 1;
 // mark and 22 us to remove in each of 72 rounds over 102,400 candidates with
 // tens of neighbours each; 16 lanes with two gathers in flight mark in 12 us,
 // and a warp for each of the few marked ones removes in 7 us (8 lanes for
-// both: 14 and 13 us). The whole elimination: 4.87 -> 2.10 ms.
-constexpr uint32_t kWseRoundLanes = 16u;
+// both: 14 and 13 us). The whole elimination: 4.87 -> 2.10 ms. Four lanes while
+// the candidates in play would fill the chip's threads more than twice with 16:
+// the rounds are then bound by issue, not by the chain (200,000 candidates 1.84
+// -> 1.73 ms, 64 sets of 3,000 1.80 -> 1.68 ms, 2,000 sets of 40 1.15 -> 1.09;
+// 20,000 candidates with 4 lanes 1.74 ms, with 16 1.51).
+constexpr uint32_t kWseRoundLanes = 16u, kWseNarrowLanes = 4u;
 
+template <uint32_t kLanes>
 __device__ __forceinline__ bool wse_tops(uint32_t i, long long wi, uint32_t begin, uint32_t end, const uint32_t* nbr,
                                          const long long* weight) {
-    for (uint32_t e = begin; e < end; e += 2u * kWseRoundLanes) {
-        const uint32_t f = e + kWseRoundLanes;
+    for (uint32_t e = begin; e < end; e += 2u * kLanes) {
+        const uint32_t f = e + kLanes;
         const uint32_t j = nbr[e], k = f < end ? nbr[f] : j;
         const long long wj = weight[j], wk = weight[k];
         if (!(wi > wj || (wi == wj && i < j)) || !(wi > wk || (wi == wk && i < k))) return false;
@@ -269,21 +284,22 @@ __device__ __forceinline__ bool wse_tops(uint32_t i, long long wi, uint32_t begi
 // The candidates of `list` (null: all of them) that top their lists, appended
 // to `marked`. out_offsets / out_nbr: the transposed lists of the adaptive
 // elimination (null when the relation is symmetric).
+template <uint32_t kLanes>
 __global__ void k_wse_mark(uint32_t n, const uint32_t* list, const uint32_t* offsets, const uint32_t* nbr,
                            const uint32_t* out_offsets, const uint32_t* out_nbr, const long long* weight,
                            uint32_t* marked, uint32_t* marked_count) {
-    const uint32_t at = lane_group<kWseRoundLanes>();
-    const uint32_t lane = threadIdx.x & 31u, sub = lane % kWseRoundLanes;
-    const unsigned group = 0xffffu << (lane - sub);
+    const uint32_t at = lane_group<kLanes>();
+    const uint32_t lane = threadIdx.x & 31u, sub = lane % kLanes;
+    const unsigned group = (0xffffffffu >> (32u - kLanes)) << (lane - sub);
     uint32_t i = 0u;
     bool top = false;
     if (at < n) {
         i = list ? list[at] : at;
         const long long wi = weight[i];
         top = wi != kWseGone;
-        if (top) top = wse_tops(i, wi, offsets[i] + sub, offsets[i + 1], nbr, weight);
+        if (top) top = wse_tops<kLanes>(i, wi, offsets[i] + sub, offsets[i + 1], nbr, weight);
         if (out_offsets && __all_sync(group, top))
-            top = wse_tops(i, wi, out_offsets[i] + sub, out_offsets[i + 1], out_nbr, weight);
+            top = wse_tops<kLanes>(i, wi, out_offsets[i] + sub, out_offsets[i + 1], out_nbr, weight);
         top = __all_sync(group, top);
     }
     const unsigned who = __ballot_sync(0xffffffffu, top && sub == 0u);
@@ -529,7 +545,7 @@ __device__ __forceinline__ void rep_neighbourhood(const RepairGrid& g, uint32_t 
                                               ((unsigned long long)r1 << 16);
             const unsigned long long lo = column | (unsigned long long)max(c[2] - 1, 0);
             const unsigned long long hi = column | (unsigned long long)(c[2] + 1);
-            for (uint32_t q = lower_bound_key(g.keys, g.n, lo); q < g.n && g.keys[q] <= hi; ++q) f(g.idx[q]);
+            for (uint32_t q = lower_bound_key(g.keys, 0u, g.n, lo); q < g.n && g.keys[q] <= hi; ++q) f(g.idx[q]);
         }
 }
 
@@ -749,8 +765,8 @@ __global__ void k_support_cells(uint32_t cells, const unsigned long long* cell_k
             if (r0 >= 0 && r1 >= 0) {
                 const unsigned long long column = inst + ((unsigned long long)r0 << 32) +
                                                   ((unsigned long long)r1 << 16);
-                b = lower_bound_key(g.keys, g.n, column + (unsigned long long)max(c2 - 1, 0));
-                e = lower_bound_key(g.keys, g.n, column + (unsigned long long)(c2 + 2));
+                b = lower_bound_key(g.keys, 0u, g.n, column + (unsigned long long)max(c2 - 1, 0));
+                e = lower_bound_key(g.keys, 0u, g.n, column + (unsigned long long)(c2 + 2));
             }
             range_b[9 * (size_t)u + r] = b;
             range_e[9 * (size_t)u + r] = e;
@@ -885,6 +901,8 @@ int launch_wse_eliminate(NanContext* ctx, const float* positions, const float* n
         s.inv_cell = 1.0 / std::max(s.d_max, 1e-8);
         s.plane_limit = std::max(s.d_max * (double)opt->plane_distance_scale, 1e-8);
         s.cmin[0] = s.cmin[1] = s.cmin[2] = 0x7fffffff;
+        s.begin = set_offsets[k];
+        s.end = set_offsets[k + 1];
         begin_host[k] = set_offsets[k];
         elim_host[k] = count > out ? count - out : 0u;
         if (poisson_radii)
@@ -1038,12 +1056,27 @@ int launch_wse_eliminate(NanContext* ctx, const float* positions, const float* n
     ok(cudaMemsetAsync(removed, 0, sizeof(unsigned int), st));
     const uint32_t* list = nullptr;  // the candidates in play, once some are gone
     int turn = 0;
-    const uint32_t g_remove = std::min<uint32_t>(g_round, 148u * 8u);
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    const uint32_t g_remove = std::min<uint32_t>(g_round, (uint32_t)sms * 8u);
+    const uint64_t resident = (uint64_t)sms * 2048u;  // threads
+    uint32_t left = n;
     while (e == cudaSuccess && done < n) {
-        const uint32_t left = n - done;
+        const uint32_t before = left;
+        left = n - done;
+        const bool narrow = (uint64_t)left * kWseRoundLanes > 2ull * resident;
+        const auto mark = narrow ? k_wse_mark<kWseNarrowLanes> : k_wse_mark<kWseRoundLanes>;
+        const uint32_t lanes = narrow ? kWseNarrowLanes : kWseRoundLanes;
         ok(cudaMemsetAsync(marked_counts, 0, (kRoundsPerCheck + 1) * sizeof(uint32_t), st));
+        if (rounds > 0u) {
+            k_wse_compact<<<blocks(before, 256), 256, 0, st>>>(before, list, weight, in_play[turn],
+                                                               marked_counts + kRoundsPerCheck);
+            ctx->launches++;
+            list = in_play[turn];
+            turn ^= 1;
+        }
         for (int k = 0; k < kRoundsPerCheck; ++k) {
-            k_wse_mark<<<blocks((uint64_t)left * kWseRoundLanes, 256), 256, 0, st>>>(
+            mark<<<blocks((uint64_t)left * lanes, 256), 256, 0, st>>>(
                 left, list, offsets, nbr, densities ? out_offsets : nullptr, densities ? out_nbr : nullptr, weight,
                 marked, marked_counts + k);
             k_wse_remove<<<g_remove, 256, 0, st>>>(marked, marked_counts + k, lose_offsets, lose_nbr, lose_contrib,
@@ -1051,11 +1084,6 @@ int launch_wse_eliminate(NanContext* ctx, const float* positions, const float* n
             ctx->launches += 2;
             ++rounds;
         }
-        k_wse_compact<<<blocks(left, 256), 256, 0, st>>>(left, list, weight, in_play[turn],
-                                                         marked_counts + kRoundsPerCheck);
-        ctx->launches++;
-        list = in_play[turn];
-        turn ^= 1;
         ok(cudaMemcpyAsync(&done, removed, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
         ok(cudaStreamSynchronize(st));
         if (rounds > 4u * n + 64u) break;  // each round removes at least the global maximum
