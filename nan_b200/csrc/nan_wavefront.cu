@@ -255,13 +255,40 @@ __device__ __forceinline__ uint32_t rays_per_grab(unsigned long long count) {
     return (uint32_t)min(32ull, max(1ull, (count + warps - 1u) / warps));
 }
 
+// Traversal forms. kShared > 0 (binary nodes): the first kShared
+// traversal-stack entries of a thread live in a shared-memory column
+// (stack_top, of the thread), the rest in local memory. kSpec (binary nodes):
+// the speculative while-while walk.
+template <int kWidth, int kShared, bool kSpec>
+__device__ __forceinline__ HitInfo closest_form(const SceneView& s, int* stack_top, f3 o, f3 d, float tmin,
+                                                float tmax) {
+    if constexpr (kShared > 0 && kWidth == 2) {
+        SplitStack<kShared, 128, kTraversalStack + 2> stk;
+        stk.top = stack_top;
+        return trace_closest_binary_s<kTraversalStack>(s, stk, o, d, tmin, tmax);
+    } else if constexpr (kSpec && kWidth == 2) {
+        return trace_closest_binary_spec(s, o, d, tmin, tmax);
+    } else {
+        return trace_closest_w<kWidth>(s, o, d, tmin, tmax);
+    }
+}
+
+template <int kWidth, int kShared, bool kSpec>
+__device__ __forceinline__ bool any_form(const SceneView& s, int* stack_top, f3 o, f3 d, float tmax) {
+    if constexpr (kShared > 0 && kWidth == 2) {
+        SplitStack<kShared, 128, kTraversalStack + 2> stk;
+        stk.top = stack_top;
+        return trace_any_binary_s<kTraversalStack>(s, stk, o, d, 0.0f, tmax);
+    } else if constexpr (kSpec && kWidth == 2) {
+        return trace_any_binary_spec(s, o, d, 0.0f, tmax);
+    } else {
+        return trace_any_w<kWidth>(s, o, d, 0.0f, tmax);
+    }
+}
+
+// The two kinds of rays as a launch each, for stage timing; their launch bounds
+// are k_wf_trace's.
 template <int kWidth, class Src, int kShared = 0, bool kSpec = false>
-// kShared > 0 (binary nodes): the first kShared traversal-stack entries of a
-// thread live in a shared-memory column, the rest in local memory. kSpec
-// (binary nodes): the speculative while-while walk.
-// 9 resident blocks of 128 per SM (56 registers a thread): the 200k-triangle
-// texel iteration takes 20.2 ms, against 20.6 with 8 blocks and 20.7 with 10
-// (48 registers, spills); the 16-scene probe batch 14.6, 14.9 and 15.9 ms.
 __global__ void __launch_bounds__(128, 9) k_wf_extend(Src src, const uint32_t* __restrict__ queue,
                                                    uint32_t* ctl, const float4* __restrict__ ro,
                                                    const float4* __restrict__ rd, float4* __restrict__ hit,
@@ -279,16 +306,8 @@ __global__ void __launch_bounds__(128, 9) k_wf_extend(Src src, const uint32_t* _
             const SceneView s = src.of(p);
             const float4 o = ro[p], d = rd[p];
             tally.extend++;
-            HitInfo h;
-            if constexpr (kShared > 0 && kWidth == 2) {
-                SplitStack<kShared, 128, kTraversalStack + 2> stk;
-                stk.top = stack_top + threadIdx.x;
-                h = trace_closest_binary_s<kTraversalStack>(s, stk, xyz(o), xyz(d), o.w, d.w);
-            } else if constexpr (kSpec && kWidth == 2) {
-                h = trace_closest_binary_spec(s, xyz(o), xyz(d), o.w, d.w);
-            } else {
-                h = trace_closest_w<kWidth>(s, xyz(o), xyz(d), o.w, d.w);
-            }
+            const HitInfo h =
+                closest_form<kWidth, kShared, kSpec>(s, stack_top + threadIdx.x, xyz(o), xyz(d), o.w, d.w);
             hit[p] = make_float4(__uint_as_float(h.valid ? h.flat : 0xffffffffu), h.t, h.b1, h.b2);
         }
         if (first >= count) break;
@@ -315,16 +334,8 @@ __global__ void __launch_bounds__(128, 9) k_wf_shadow(Src src, const float4* __r
             tally.shadow++;
             const uint32_t p = __float_as_uint(a.w);
             const SceneView s = src.of(p);
-            bool blocked;
-            if constexpr (kShared > 0 && kWidth == 2) {
-                SplitStack<kShared, 128, kTraversalStack + 2> stk;
-                stk.top = stack_top + threadIdx.x;
-                blocked = trace_any_binary_s<kTraversalStack>(s, stk, xyz(a), xyz(b), 0.0f, c.w > 0.0f ? c.w : t_max);
-            } else if constexpr (kSpec && kWidth == 2) {
-                blocked = trace_any_binary_spec(s, xyz(a), xyz(b), 0.0f, c.w > 0.0f ? c.w : t_max);
-            } else {
-                blocked = trace_any_w<kWidth>(s, xyz(a), xyz(b), 0.0f, c.w > 0.0f ? c.w : t_max);
-            }
+            const bool blocked = any_form<kWidth, kShared, kSpec>(s, stack_top + threadIdx.x, xyz(a), xyz(b),
+                                                                  c.w > 0.0f ? c.w : t_max);
             if (!blocked) {
                 float4* target = (__float_as_uint(b.w) == kKindNee) ? rad : si;
                 const float4 v = target[p];
@@ -343,8 +354,14 @@ __global__ void __launch_bounds__(128, 9) k_wf_shadow(Src src, const float4* __r
 // 32 rays of one kind, closest hits first. Against extend, shade, shadow and
 // finalize launches in turn: probe baker over 20,480 sites 6.14 -> 4.77 ms,
 // 256x256 box frame 267 -> 200 us, 1080p frame over 1M triangles
-// 2.71 -> 2.43 ms, 200k-triangle texel iteration 20.0 -> 19.6 ms.
-template <class Src>
+// 2.71 -> 2.43 ms, 200k-triangle texel iteration 20.0 -> 19.6 ms. The other
+// forms and widths that take whole grabs run the same way (8-wide nodes, a
+// 640x480 frame over 82k triangles 1.16 -> 0.91 ms).
+// 9 resident blocks of 128 per SM (56 registers a thread): the 200k-triangle
+// texel iteration takes 18.85 ms, against 19.06 with 8 blocks and 19.87 with 10
+// (48 registers, spills), the 16-scene probe batch 14.01, 14.25 and 15.40, the
+// 1080p frame 2.25, 2.27 and 2.37, the probe baker 4.81, 4.73 and 4.99.
+template <int kWidth, class Src, int kShared = 0, bool kSpec = false>
 __global__ void __launch_bounds__(128, 9) k_wf_trace(Src src, const uint32_t* __restrict__ queue, uint32_t* ctl,
                                                      const float4* __restrict__ ro, const float4* __restrict__ rd,
                                                      float4* __restrict__ hit, const float4* __restrict__ shadows,
@@ -357,6 +374,7 @@ __global__ void __launch_bounds__(128, 9) k_wf_trace(Src src, const uint32_t* __
     const uint32_t grab = rays_per_grab((unsigned long long)rays + shadow_rays);
     const uint32_t ray_chunks = (rays + grab - 1u) / grab, chunks = ray_chunks + (shadow_rays + grab - 1u) / grab;
     RayTally tally{0u, 0u};
+    __shared__ int stack_top[kShared > 0 ? kShared * 128 : 1];
     for (uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < chunks;) {
         if (c < ray_chunks) {
             const uint32_t idx = c * grab + lane;
@@ -365,7 +383,8 @@ __global__ void __launch_bounds__(128, 9) k_wf_trace(Src src, const uint32_t* __
                 const SceneView s = src.of(p);
                 const float4 o = ro[p], d = rd[p];
                 tally.extend++;
-                const HitInfo h = trace_closest_binary(s, xyz(o), xyz(d), o.w, d.w);
+                const HitInfo h =
+                    closest_form<kWidth, kShared, kSpec>(s, stack_top + threadIdx.x, xyz(o), xyz(d), o.w, d.w);
                 hit[p] = make_float4(__uint_as_float(h.valid ? h.flat : 0xffffffffu), h.t, h.b1, h.b2);
             }
         } else {
@@ -375,7 +394,8 @@ __global__ void __launch_bounds__(128, 9) k_wf_trace(Src src, const uint32_t* __
                 tally.shadow++;
                 const uint32_t p = __float_as_uint(a.w);
                 const SceneView s = src.of(p);
-                if (!trace_any_binary(s, xyz(a), xyz(b), 0.0f, e.w > 0.0f ? e.w : t_max)) {
+                if (!any_form<kWidth, kShared, kSpec>(s, stack_top + threadIdx.x, xyz(a), xyz(b),
+                                                      e.w > 0.0f ? e.w : t_max)) {
                     float4* target = (__float_as_uint(b.w) == kKindNee) ? rad : si;
                     const float4 v = target[p];
                     target[p] = make_float4(v.x + e.x, v.y + e.y, v.z + e.z, v.w);
@@ -396,7 +416,9 @@ __global__ void __launch_bounds__(128, 9) k_wf_trace(Src src, const uint32_t* __
 // Finished rays write their results in the same refill round, so ray set-up
 // and result stores run for the idle lanes together. kBurst steps run
 // between two refill checks. Without refill, a warp that took 32 rays runs
-// until the slowest of them ends.
+// until the slowest of them ends. As many lanes of a warp take rays as
+// rays_per_grab allows, and warps that the queue cannot reach leave before
+// their first atomic (probe baker over 2,000 sites, 8 samples, in form 1: 5.24 -> 2.79 ms).
 template <int kRefill, int kBurst, class Src>
 __global__ void __launch_bounds__(128, 9) k_wf_extend_refill(Src src, const uint32_t* __restrict__ queue,
                                                           uint32_t* ctl, const float4* __restrict__ ro,
@@ -405,16 +427,20 @@ __global__ void __launch_bounds__(128, 9) k_wf_extend_refill(Src src, const uint
     const uint32_t count = *(volatile uint32_t*)(ctl + kExt);
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
+    const uint32_t share = rays_per_grab(count);
+    if ((uint64_t)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * share >= count) return;  // the whole warp
+    const unsigned lanes = 0xffffffffu >> (32u - share);
+    const int refill = min(kRefill, (int)share);
     RayTally tally{0u, 0u};
     ClosestWalk w;
     int stack[kTraversalStack];
     bool alive = false, pending = false, drained = false;
     uint32_t p = 0u;
     for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, !alive);
+        const unsigned idle = __ballot_sync(0xffffffffu, !alive) & lanes;
         if (drained) {
-            if (idle == 0xffffffffu) break;
-        } else if (__popc(idle) >= kRefill) {
+            if (idle == lanes) break;
+        } else if (__popc(idle) >= refill) {
             if (pending) {
                 const HitInfo h = closest_end(src.of(p), w);
                 hit[p] = make_float4(__uint_as_float(h.valid ? h.flat : 0xffffffffu), h.t, h.b1, h.b2);
@@ -424,7 +450,7 @@ __global__ void __launch_bounds__(128, 9) k_wf_extend_refill(Src src, const uint
             uint32_t base = 0u;
             if (lane == 0u) base = atomicAdd(ctl + kExtFetch, n);
             base = __shfl_sync(0xffffffffu, base, 0);
-            if (!alive) {
+            if ((idle >> lane) & 1u) {
                 const uint32_t idx = base + (uint32_t)__popc(idle & below);
                 if (idx < count) {
                     p = queue[idx];
@@ -463,16 +489,20 @@ __global__ void __launch_bounds__(128, 9) k_wf_shadow_refill(Src src, const floa
     const uint32_t count = *(volatile uint32_t*)(ctl + kShd);
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
+    const uint32_t share = rays_per_grab(count);
+    if ((uint64_t)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * share >= count) return;  // the whole warp
+    const unsigned lanes = 0xffffffffu >> (32u - share);
+    const int refill = min(kRefill, (int)share);
     RayTally tally{0u, 0u};
     AnyWalk w;
     int stack[kTraversalStack];
     bool alive = false, pending = false, drained = false;
     uint32_t p = 0u, e = 0u;
     for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, !alive);
+        const unsigned idle = __ballot_sync(0xffffffffu, !alive) & lanes;
         if (drained) {
-            if (idle == 0xffffffffu) break;
-        } else if (__popc(idle) >= kRefill) {
+            if (idle == lanes) break;
+        } else if (__popc(idle) >= refill) {
             if (pending) {  // a ray that ended without a hit adds its contribution
                 const float4 b = queue[3u * e + 1u], c = queue[3u * e + 2u];
                 float4* target = (__float_as_uint(b.w) == kKindNee) ? rad : si;
@@ -484,7 +514,7 @@ __global__ void __launch_bounds__(128, 9) k_wf_shadow_refill(Src src, const floa
             uint32_t base = 0u;
             if (lane == 0u) base = atomicAdd(ctl + kShdFetch, n);
             base = __shfl_sync(0xffffffffu, base, 0);
-            if (!alive) {
+            if ((idle >> lane) & 1u) {
                 const uint32_t idx = base + (uint32_t)__popc(idle & below);
                 if (idx < count) {
                     e = idx;
@@ -1467,7 +1497,7 @@ Grid grid_for(const NanContext* ctx, uint64_t paths) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wf_trace<OneScene>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wf_trace<2, OneScene>, 128, 0);
     Grid g;
     const int per_sm = ctx->tuning.trace_blocks_per_sm ? (int)ctx->tuning.trace_blocks_per_sm : std::max(occ, 1);
     g.persistent_blocks = (int)std::min<uint64_t>((uint64_t)sms * per_sm, std::max<uint64_t>((3 * paths + 3) / 4, 1));
@@ -1479,28 +1509,42 @@ Grid grid_for(const NanContext* ctx, uint64_t paths) {
 
 // The traversal of round `it`: the closest hits of its walking paths and the
 // shadow rays that the round before queued, in one launch; in two (extend, then
-// shadow) for the wide nodes, the other traversal forms and stage timing.
+// shadow) for the traversal forms that refill lanes and for stage timing.
 // timed: the pass is one that NanTuning.kernel_timing covers. The batch is not:
 // its frames are captured in graphs, whose event records cannot be read.
+// Launches apart leave out the queues that are empty by the plan: no path
+// walks in the last of the rounds, and in the first there are shadow rays only
+// if the generated paths have them (gen_shadows).
 template <class Src>
-void launch_trace(NanContext* ctx, int blocks, cudaStream_t st, bool wide, bool timed, Src src, const WfQueues& q,
-                  uint32_t it, float t_max, const WfState& S) {
+void launch_trace(NanContext* ctx, int blocks, cudaStream_t st, bool wide, bool timed, bool gen_shadows, Src src,
+                  const WfQueues& q, uint32_t it, uint32_t rounds, float t_max, const WfState& S) {
     const int buf = (int)(it & 1u);
     uint32_t* ctl = q.ctl + kCtlWords * (it + 1u);
     timed = timed && ctx->tuning.kernel_timing;
-    if (!wide && ctx->tuning.traversal == 0u && !timed) {
-        k_wf_trace<Src><<<blocks, 128, 0, st>>>(src, q.ext[buf], ctl, S.ro, S.rd, S.hit, q.shd[buf ^ 1],
-                                                ctl - kCtlWords, t_max, S.rad, S.si, ctx->d_counters);
+    const uint32_t form = wide ? 0u : ctx->tuning.traversal;
+    if (!timed && (form == 0u || form >= 5u)) {
+#define NAN_TRACE_ARGS src, q.ext[buf], ctl, S.ro, S.rd, S.hit, q.shd[buf ^ 1], ctl - kCtlWords, t_max, S.rad, S.si, \
+                       ctx->d_counters
+        if (wide) k_wf_trace<8, Src><<<blocks, 128, 0, st>>>(NAN_TRACE_ARGS);
+        else if (form == 5u) k_wf_trace<2, Src, 16><<<blocks, 128, 0, st>>>(NAN_TRACE_ARGS);
+        else if (form == 6u) k_wf_trace<2, Src, 0, true><<<blocks, 128, 0, st>>>(NAN_TRACE_ARGS);
+        else k_wf_trace<2, Src><<<blocks, 128, 0, st>>>(NAN_TRACE_ARGS);
+#undef NAN_TRACE_ARGS
         ctx->launches++;
         return;
     }
-    cudaEvent_t ev = timed ? nan_host::timing_begin(ctx, st) : nullptr;
-    launch_extend(ctx, blocks, st, wide, src, q.ext[buf], ctl, S);
-    nan_host::timing_end(ctx, 0, ev, st);
-    ev = timed ? nan_host::timing_begin(ctx, st) : nullptr;
-    launch_shadow(ctx, blocks, st, wide, src, q.shd[buf ^ 1], ctl - kCtlWords, t_max, S);
-    nan_host::timing_end(ctx, 1, ev, st);
-    ctx->launches += 2;
+    if (it + 1u < rounds) {
+        cudaEvent_t ev = timed ? nan_host::timing_begin(ctx, st) : nullptr;
+        launch_extend(ctx, blocks, st, wide, src, q.ext[buf], ctl, S);
+        nan_host::timing_end(ctx, 0, ev, st);
+        ctx->launches++;
+    }
+    if (it > 0u || gen_shadows) {
+        cudaEvent_t ev = timed ? nan_host::timing_begin(ctx, st) : nullptr;
+        launch_shadow(ctx, blocks, st, wide, src, q.shd[buf ^ 1], ctl - kCtlWords, t_max, S);
+        nan_host::timing_end(ctx, 1, ev, st);
+        ctx->launches++;
+    }
 }
 
 }  // namespace
@@ -1645,10 +1689,11 @@ void wf_carve(NanContext* ctx, uint32_t count, uint32_t rounds, WfState& S, WfQu
 // Runs units [begin, end) in chunks: generate, then `rounds` rounds of trace
 // and stage. gen(S, q, first_unit, count) and stage(S, q, buf, ctl, blocks)
 // launch the integrator's own stages. The control block of round k is block
-// k + 1: the generated paths' shadow rays belong to block 0.
+// k + 1: the generated paths' shadow rays (gen_shadows: there may be some)
+// belong to block 0.
 template <class Gen, class Stage>
 int wf_run(NanContext* ctx, cudaStream_t st, uint64_t begin, uint64_t end, uint32_t rounds, uint64_t cap, float t_max,
-           Gen gen, Stage stage) {
+           bool gen_shadows, Gen gen, Stage stage) {
     const SceneView s = scene_view(ctx);
     const Grid g = grid_for(ctx, std::min<uint64_t>(cap, end - begin));
     for (uint64_t cb = begin; cb < end; cb += cap) {
@@ -1676,7 +1721,7 @@ int wf_run(NanContext* ctx, cudaStream_t st, uint64_t begin, uint64_t end, uint3
                 std::swap(q.ext[buf], q.ext_sorted);
                 ctx->launches += 3;
             }
-            launch_trace(ctx, g.persistent_blocks, st, s.wnodes != nullptr, true, OneScene{s}, q, it, t_max, S);
+            launch_trace(ctx, g.persistent_blocks, st, s.wnodes != nullptr, true, gen_shadows, OneScene{s}, q, it, rounds, t_max, S);
             ev = timing_begin(ctx, st);
             stage(S, q, buf, ctl, g.stream_blocks);
             timing_end(ctx, 2, ev, st);
@@ -1716,7 +1761,7 @@ int launch_trace_texels_wavefront(NanContext* ctx, const NanMeshColorsDesc* lay,
     a.reset = reset;
     unsigned long long* counters = ctx->d_counters;
     return wf_run(
-        ctx, st, begin, end, rounds, cap, lr.ray_t_max,
+        ctx, st, begin, end, rounds, cap, lr.ray_t_max, true,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t count) {
             k_wf_texel_generate<<<(count + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(s, lr, a, S, q, first, count, counters);
         },
@@ -1779,7 +1824,7 @@ int launch_trace_points_wavefront(NanContext* ctx, const float* points, uint32_t
     a.indirect_only = (flags & NAN_POINTS_INDIRECT_ONLY) != 0u;
     unsigned long long* counters = ctx->d_counters;
     return wf_run(
-        ctx, st, 0, count, rounds, cap, lr.ray_t_max,
+        ctx, st, 0, count, rounds, cap, lr.ray_t_max, !a.indirect_only,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t cnt) {
             k_wf_point_generate<<<(cnt + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(s, lr, a, S, q, first, cnt, counters);
         },
@@ -1811,7 +1856,7 @@ int screen_wavefront(NanContext* ctx, float* out, uint32_t w, uint32_t h, uint32
     else memset(&a.cache, 0, sizeof(a.cache));
     unsigned long long* counters = ctx->d_counters;
     return wf_run(
-        ctx, st, 0, pixels, rounds, cap, lr.ray_t_max,
+        ctx, st, 0, pixels, rounds, cap, lr.ray_t_max, false,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t count) {
             k_wf_screen_generate<<<(count + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(s, lr, a, S, q, first, count, counters);
         },
@@ -1823,7 +1868,7 @@ int screen_wavefront(NanContext* ctx, float* out, uint32_t w, uint32_t h, uint32
 
 size_t probe_sample_bytes() { return sizeof(ProbeSample); }
 
-const void* wavefront_extend_kernel() { return reinterpret_cast<const void*>(&k_wf_trace<ManyScenes>); }
+const void* wavefront_extend_kernel() { return reinterpret_cast<const void*>(&k_wf_trace<2, ManyScenes>); }
 
 // The multi-scene probe batch on the wavefront: generate every (set, probe)
 // unit as one path, then n * max_bounces rounds of extend / shade / shadow /
@@ -1865,7 +1910,7 @@ int launch_batch_wavefront(NanContext* ctx, const void* sets, const uint32_t* pr
     k_wfb_probe_generate<<<(total + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(m, S, q, ctx->d_counters);
     ctx->launches++;
     for (uint32_t it = 0; it < rounds; ++it) {
-        launch_trace(ctx, g.persistent_blocks, st, false, false, src, q, it, t_max, S);
+        launch_trace(ctx, g.persistent_blocks, st, false, false, false, src, q, it, rounds, t_max, S);
         k_wfb_probe_stage<<<g.stream_blocks, kStageThreads, 0, st>>>(m, S, q, (int)(it & 1u), q.ctl + kCtlWords * (it + 1u));
         ctx->launches++;
     }
@@ -1912,7 +1957,7 @@ int launch_batch_wavefront_independent(NanContext* ctx, const void* sets, const 
         if (err != cudaSuccess) return cuda_fail(err, "batch wavefront control reset");
         k_wfi_probe_generate<<<(paths + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(m, S, q);
         for (uint32_t it = 0; it < rounds; ++it) {
-            launch_trace(ctx, g.persistent_blocks, st, false, false, src, q, it, t_max, S);
+            launch_trace(ctx, g.persistent_blocks, st, false, false, false, src, q, it, rounds, t_max, S);
             k_wfi_probe_stage<<<g.stream_blocks, kStageThreads, 0, st>>>(m, S, q, (int)(it & 1u), q.ctl + kCtlWords * (it + 1u));
         }
         k_wfi_probe_fold<<<(m.units + 127) / 128, 128, 0, st>>>(m, ctx->d_counters);
@@ -1947,7 +1992,7 @@ int launch_trace_probes_wavefront(NanContext* ctx, float* values, uint32_t* coun
     a.reset = reset;
     unsigned long long* counters = ctx->d_counters;
     return wf_run(
-        ctx, st, begin, end, rounds, cap, lr.ray_t_max,
+        ctx, st, begin, end, rounds, cap, lr.ray_t_max, false,
         [&](const WfState& S, const WfQueues& q, uint32_t first, uint32_t count) {
             k_wf_probe_generate<<<(count + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(s, lr, a, S, q, first, count, counters);
         },

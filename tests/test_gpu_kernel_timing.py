@@ -1,18 +1,21 @@
 """Kernel timing on: a round's closest-hit and shadow rays then run as a launch
-each, of kernels that nothing else launches over binary nodes in their default
-form. Pixels, texel slots, probe fields and the ray counts equal those without
-timing bit for bit (no tolerance: the same arithmetic in the same order), at
-sizes from one path to a queue that fills the grid's warps unevenly, and the
-times say that both kinds of launches ran."""
+each, of kernels that nothing else launches (but for the forms that refill
+lanes, 1 to 4). Pixels, texel slots, probe fields and the ray counts of every
+form, with timing and without, equal the default's bit for bit (no tolerance:
+the same arithmetic in the same order), at sizes from one path to a queue that
+fills the grid's warps unevenly, and the times say that both kinds of launches
+ran."""
 
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("builder", ["sah", "lbvh"])
+@pytest.mark.parametrize("builder,option", [("sah", {}), ("lbvh", {}), ("sah", {"traversal": 2}),
+                                            ("lbvh", {"traversal": 5}), ("sah", {"traversal": 6}),
+                                            ("sah", {"bvh_width": 8})])
 @pytest.mark.parametrize("width,height,sites", [(1, 1, 1), (33, 1, 33), (130, 131, 300), (641, 480, 3000)])
-def test_timing_does_not_change_results(device, width, height, sites, builder):
+def test_timing_does_not_change_results(device, width, height, sites, builder, option):
     import torch
 
     import nan_b200
@@ -28,8 +31,8 @@ def test_timing_does_not_change_results(device, width, height, sites, builder):
     texels = (begin, min(layout.total_surface_texels, begin + width * height))
     node.camera.begin_frame(width, height)  # one jitter for both
     results = []
-    for timing in (False, True):
-        scene.configure(kernel_timing=timing)
+    for form, timing in (({}, False), (option, False), (option, True)):
+        scene.configure(kernel_timing=timing, **form)
         scene.context.read_kernel_times(reset=True)
         scene.context.read_counters(reset=True)
         out = torch.zeros((height, width, 4), dtype=torch.float32, device="cuda")
@@ -53,8 +56,9 @@ def test_timing_does_not_change_results(device, width, height, sites, builder):
         results.append(([out, slots, rt.field.values.clone(), rt.attachments.radial_moments.clone()],
                         (c["extend_rays"], c["shadow_rays"], c["units"], c["paths"])))
     scene.configure()
-    (a, ca), (b, cb) = results
-    for x, y in zip(a, b):
-        torch.testing.assert_close(x.view(torch.int32), y.view(torch.int32), rtol=0, atol=0)
-    assert ca == cb and ca[0] > 0
+    a, ca = results[0]
+    for b, cb in results[1:]:
+        for x, y in zip(a, b):
+            torch.testing.assert_close(x.view(torch.int32), y.view(torch.int32), rtol=0, atol=0)
+        assert ca == cb and ca[0] > 0
     device.check()
