@@ -749,7 +749,9 @@ __device__ __forceinline__ bool filter_texel(const McView& mc, uint32_t u0, uint
     }
     hint.known = false;
     if (u >= total) return false;
+    // 32 texels lie in the next 32 instances, unless some of those are empty
     uint32_t hi = mc.instance_count - 1u;
+    if (i + 32u < mc.instance_count && __ldg(mc.surface_prefix + i + 32u) > last) hi = i + 31u;
     while (i < hi) {
         const uint32_t mid = (i + hi + 1u) >> 1;
         if (__ldg(mc.surface_prefix + mid) <= u) i = mid; else hi = mid - 1u;
