@@ -423,6 +423,17 @@ __device__ __forceinline__ bool walk_down(const SceneView& s, Stk& stack, const 
     return any;
 }
 
+// A walk's report when its overflow entry was overwritten: one predicated
+// reduction, by a global address. An atomic by a generic one could reach the
+// local stack, and the walks of a kernel then no longer share one (the batch
+// kernel with one sample a lane: 484 bytes of spills instead of 280 in 80
+// registers, 16-sample batch of 8 scenes 4.52 ms instead of 4.23).
+__device__ __forceinline__ void report_overflow(const SceneView& s, int overflow_entry) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %1, %2;\n\t@p red.global.or.b32 [%0], %3;\n\t}" ::"l"(
+                     __cvta_generic_to_global(s.status)),
+                 "r"(overflow_entry), "r"(kWalkEnd), "r"(kStatusStackOverflow));
+}
+
 // Closest hit in [tmin, tmax]; ties in t go to the lower flat triangle index
 // (lexicographic (instance, primitive)), so the result does not depend on
 // the traversal order. Binary-node traversal.
@@ -467,7 +478,7 @@ __device__ __forceinline__ HitInfo trace_closest_binary_s(const SceneView& s, St
         }
         node = stack.get(--sp);
     }
-    if (stack.get(kDepth + 1) != kWalkEnd) atomicOr(s.status, kStatusStackOverflow);
+    report_overflow(s, stack.get(kDepth + 1));
     if (best_key != 0xffffffffu) {
         hit.valid = true;
         hit.flat = best_key;
@@ -514,7 +525,7 @@ __device__ __forceinline__ bool trace_any_binary_s(const SceneView& s, Stk& stac
         if (blocked) break;
         node = stack.get(--sp);
     }
-    if (stack.get(kDepth + 1) != kWalkEnd) atomicOr(s.status, kStatusStackOverflow);
+    report_overflow(s, stack.get(kDepth + 1));
     return blocked;
 }
 
