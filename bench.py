@@ -6,12 +6,14 @@ seeded 200,688-triangle scene (313x313-vertex displaced terrain + 500 boxes
 with sides U[0.2, 3] and random yaw, albedo U[0.1, 0.9]); 16 texels/unit,
 per-triangle lattice resolution 4..64, 1 hemisphere sample per texel, 3
 bounces, sun at 45 deg with irradiance 3, constant sky 0.5. One step = one
-iteration (the wavefront integrator's generate, extend, shadow and stage
-launches; without kernel timing one launch traces a round's extend and shadow
-rays). Metric: Mrays/s, every closest-hit (extend) and any-hit (shadow)
-ray counted on the device. The roofline is that of the traversal kernels
-(k_wf_extend + k_wf_shadow), timed by CUDA events the library records on the
-launching stream inside the timed region.
+iteration as every caller gets it: the wavefront integrator's generate launch,
+then per round one trace launch (closest-hit and shadow rays) and one stage
+launch. Metric: Mrays/s, every closest-hit (extend) and any-hit (shadow) ray
+counted on the device. The split by kernel comes from a further pass with
+kernel timing on, outside the timed region, since timing runs the two kinds of
+rays as a launch each. The roofline is the L1 data pipe's, which bounds the
+trace launch; the bytes that a model of node visits charges per ray are given
+apart.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl nan|reference]
 
@@ -237,14 +239,15 @@ def measured_peak_gbs():
         return 6650.0, "fallback"
 
 
-def ncu_traffic(integrator: str):
-    """DRAM bytes (read + write) per step of the kernels the roofline covers,
-    from the committed ncu summary."""
+def trace_profile(args):
+    """What ncu counted per ray in k_wf_trace on the default workload (the
+    committed summary), or None where another kernel or workload runs."""
+    if (args.integrator, args.grid, args.boxes, args.bvh, args.width, args.traversal, args.ray_order) != (
+            "wavefront", 313, 500, "sah", 2, 0, 0):
+        return None
     try:
-        data = json.loads((ROOT / "profiles" / "traffic.json").read_text())
-        key = "traversal_bytes_per_step" if integrator == "wavefront" else "k_trace_texels_bytes_per_launch"
-        return data.get(key)
-    except Exception:
+        return json.loads((ROOT / "profiles" / "traffic.json").read_text())["k_wf_trace"]
+    except (OSError, ValueError, KeyError):
         return None
 
 
@@ -323,12 +326,6 @@ def run_nan(args):
     device.check()
     scene.context.read_counters(reset=True)
     launches0 = scene.context.launch_count
-    # stage timing on inside the timed region: an event pair around each
-    # wavefront launch, on the launching stream
-    scene.configure(args.integrator, trace_blocks_per_sm=args.blocks_per_sm, bvh_width=args.width,
-                    kernel_timing=True, ray_order=args.ray_order, traversal=args.traversal)
-    scene.context.read_kernel_times(reset=True)
-
     clocks = ClockSampler(local)
     events = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
     barrier()
@@ -350,11 +347,21 @@ def run_nan(args):
     launch_ms = [a.elapsed_time(b) for a, b in events]
     launches = scene.context.launch_count - launches0
     counters = scene.context.read_counters(reset=True)
-    ktimes = scene.context.read_kernel_times(reset=True)
-    scene.configure(args.integrator, trace_blocks_per_sm=args.blocks_per_sm, bvh_width=args.width,
-                    ray_order=args.ray_order, traversal=args.traversal)
     device.check()
     rays_local = counters["extend_rays"] + counters["shadow_rays"]
+
+    # split by kernel: the same iteration with an event pair around each launch
+    # on the launching stream, closest-hit and shadow rays apart
+    split_steps = max(1, min(args.steps, 5))
+    scene.configure(args.integrator, trace_blocks_per_sm=args.blocks_per_sm, bvh_width=args.width,
+                    kernel_timing=True, ray_order=args.ray_order, traversal=args.traversal)
+    scene.context.read_kernel_times(reset=True)
+    for _ in range(split_steps):
+        tracer.execute(stream, slots, it, texel_range=(begin, end))
+        it += 1
+    ktimes = {k: v / split_steps for k, v in scene.context.read_kernel_times(reset=True).items()}
+    scene.configure(args.integrator, trace_blocks_per_sm=args.blocks_per_sm, bvh_width=args.width,
+                    ray_order=args.ray_order, traversal=args.traversal)
 
     # e2e through the public API with host buffers: every step the slot
     # buffer goes H2D from pinned memory, the iteration runs, and the updated
@@ -383,13 +390,12 @@ def run_nan(args):
     e2e_counters = scene.context.read_counters(reset=True)
     e2e_rays_local = e2e_counters["extend_rays"] + e2e_counters["shadow_rays"]
 
-    trav_ms = ktimes["extend_ms"] + ktimes["shadow_ms"]
-    stats = torch.tensor([elapsed_ms, e2e_ms, trav_ms], dtype=torch.float64, device=device.torch_device)
+    stats = torch.tensor([elapsed_ms, e2e_ms], dtype=torch.float64, device=device.torch_device)
     sums = torch.tensor([float(rays_local), float(e2e_rays_local)], dtype=torch.float64, device=device.torch_device)
     if world > 1:
         dist.all_reduce(stats, op=dist.ReduceOp.MAX)
         dist.all_reduce(sums, op=dist.ReduceOp.SUM)
-    elapsed_ms, e2e_ms, trav_ms = float(stats[0]), float(stats[1]), float(stats[2])
+    elapsed_ms, e2e_ms = float(stats[0]), float(stats[1])
     rays_total, e2e_rays = float(sums[0]), float(sums[1])
     if world > 1:
         dist.destroy_process_group()
@@ -398,18 +404,27 @@ def run_nan(args):
 
     value = rays_total / (elapsed_ms * 1e3)
     bytes_per_ray, n_node, n_tri = roofline_bytes_per_ray(node, layout, scene.lighting)
-    avg_step_s = statistics.mean(launch_ms) * 1e-3
+    step_ms = statistics.mean(launch_ms)
     rays_per_step = rays_local / args.steps
-    step_achieved = rays_per_step * bytes_per_ray / avg_step_s / 1e9
-    if trav_ms > 0.0:
-        # traversal kernels: all rays' algorithmic bytes over their own device time
-        scope = "k_wf_extend + k_wf_shadow (per step: all extend and shadow launches)"
-        achieved = rays_per_step * bytes_per_ray / (trav_ms / args.steps * 1e-3) / 1e9
-    else:
-        scope = "k_trace_texels (one launch per step)"
-        achieved = step_achieved
     peak, peak_kind = measured_peak_gbs()
-    traffic = ncu_traffic(args.integrator)
+    # the step less its generate and stage kernels: the trace launches
+    trace_ms = step_ms - ktimes["stage_ms"] if ktimes["stage_ms"] > 0.0 else step_ms
+    visit_gbs = rays_per_step * bytes_per_ray / (trace_ms * 1e-3) / 1e9
+    roofline = None
+    profile = trace_profile(args)
+    if profile and clock_info.get("sm_mhz"):
+        sms = torch.cuda.get_device_properties(local).multi_processor_count
+        wavefronts = rays_per_step * profile["l1_wavefronts_per_ray"] / (trace_ms * 1e-3) / 1e9
+        wavefront_peak = sms * clock_info["sm_mhz"] * 1e-3  # one a cycle and SM
+        traffic = rays_per_step * profile["dram_bytes_per_ray"]
+        roofline = {"bound": "l1 data pipe", "achieved": wavefronts, "peak": wavefront_peak,
+                    "unit": "Gwavefronts/s", "frac": wavefronts / wavefront_peak,
+                    "scope": "k_wf_trace: the step less its generate and stage kernels",
+                    "l1_wavefronts_per_ray": profile["l1_wavefronts_per_ray"], "source": profile["source"],
+                    "peak_source": f"1 wavefront a cycle on {sms} SMs at the sampled clock",
+                    "traffic": traffic, "dram_gbs": traffic / (trace_ms * 1e-3) / 1e9,
+                    "dram_frac": traffic / (trace_ms * 1e-3) / 1e9 / peak,
+                    "dram_peak_source": f"{peak_kind} hbm_gbs {peak:g}"}
     line = {
         "metric": "Mrays/s", "value": value, "unit": "Mrays/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": elapsed_ms / args.steps, "higher_is_better": True,
@@ -430,14 +445,13 @@ def run_nan(args):
         "bvh_build_ms": scene.info()["build_ms"],
         "bvh_sah_cost": scene.info()["sah_cost"],
         "reference_sah_cost": getattr(roofline_bytes_per_ray, "sah_cost", None),
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": traffic, "scope": scope,
-                     "bytes_per_ray": bytes_per_ray, "nodes_per_ray": n_node, "tris_per_ray": n_tri,
-                     "step_achieved": step_achieved, "step_frac": step_achieved / peak,
-                     "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
-                     else peak_kind},
-        "kernel_ms_per_step": {"extend": ktimes["extend_ms"] / args.steps, "shadow": ktimes["shadow_ms"] / args.steps,
-                               "generate_shade_finalize": ktimes["stage_ms"] / args.steps},
+        "roofline": roofline,
+        # 32 + 16 + 32 N_node + 36 N_tri bytes a ray, as if every visit went to
+        # memory: the nodes come from the L1 and the L2, so this passes the HBM rate
+        "visit_model": {"bytes_per_ray": bytes_per_ray, "nodes_per_ray": n_node, "tris_per_ray": n_tri,
+                        "gbs": visit_gbs, "times_hbm_rate": visit_gbs / peak},
+        "kernel_ms_per_step": {"trace": trace_ms, "generate_and_stages": ktimes["stage_ms"],
+                               "extend_apart": ktimes["extend_ms"], "shadow_apart": ktimes["shadow_ms"]},
         "e2e": {"value": e2e_rays / (e2e_ms * 1e3), "unit": "Mrays/s",
                 "h2d_bytes_per_step": int(slots.numel() * 4), "d2h_bytes_per_step": int(slots.numel() * 4)},
         "gpu_launches": int(launches),
