@@ -1797,9 +1797,9 @@ int finish_binary(NanContext* ctx, uint32_t n, const float4* tris_sorted, const 
                   const int* root_dev, cudaStream_t s);
 
 // Binned-SAH hierarchy over the leaves (kernels k_sah_*): large nodes level by
-// level, one host readback of the next level's node count per level, then
-// the mid nodes and the small nodes in one launch each; the root is interior
-// node 0.
+// level, one host readback of the next level's node count per kSahBatch
+// levels, then the mid nodes and the small nodes in one launch each; the root
+// is interior node 0.
 int build_binned(NanContext* ctx, uint32_t n, const float4* tris_sorted, const float4* leaf_lo,
                  const float4* leaf_hi, int2* children, int* node_parent, int* leaf_parent, float4* node_lo,
                  float4* node_hi, uint32_t* arrivals, uint32_t* depth, double* sah, const Bounds* bounds,

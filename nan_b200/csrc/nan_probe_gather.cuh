@@ -123,7 +123,10 @@ struct ProbeWalk {
 // nodes, and so its candidates, in the order of a walk of its own. With one
 // copy of the gather for both radii, loops left rolled and a selection that
 // shrinks its scan (the kernel stalled on instruction fetches before, 3.1 an
-// issue), 1920x1080 pixels over 20,480 probes resolve in 1.81 ms (3.39).
+// issue), 1920x1080 pixels over 20,480 probes resolve in 1.81 ms (3.39). A warp
+// whose pixels hit several instances walks them one after the other, which
+// still gains where instances are many and small: a city of 20,000 boxes 2.38
+// -> 1.24 ms, a terrain under 20,000 boxes 4.17 -> 3.53 ms.
 __device__ __noinline__ void probe_gather(const ProbeLayoutView& v, const ProbeInstance& ins, uint32_t instance,
                                           f3 q, f3 qn, float radius_scale, bool want, Candidates& out,
                                           ProbeWalk& walk, uint32_t* status) {

@@ -125,7 +125,9 @@ __device__ __forceinline__ uint32_t visibility_cell(float x, float y, float z) {
 }
 
 // The table's rays in the order of their cells (any order within one), by the
-// whole block: a counting sort.
+// whole block: a counting sort, in each block of a launch. It costs a call of
+// few rays nothing that shows (one site x 1 ray 20.2 us without it, 20.5 with;
+// 100 sites x 64 rays 95.7 -> 77.0, 5,000 x 16 72.9 -> 62.6).
 __device__ __forceinline__ void visibility_order(const float* __restrict__ table, uint32_t rays, uint32_t* cells,
                                                  uint16_t* order) {
     for (uint32_t k = threadIdx.x; k < kVisCellCount; k += blockDim.x) cells[k] = 0u;

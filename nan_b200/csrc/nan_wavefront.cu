@@ -1871,8 +1871,8 @@ size_t probe_sample_bytes() { return sizeof(ProbeSample); }
 const void* wavefront_extend_kernel() { return reinterpret_cast<const void*>(&k_wf_trace<2, ManyScenes>); }
 
 // The multi-scene probe batch on the wavefront: generate every (set, probe)
-// unit as one path, then n * max_bounces rounds of extend / shade / shadow /
-// finalize over all sets, with no host synchronisation (capturable). The
+// unit as one path, then n * (max_bounces + 1) rounds of a trace and a stage
+// launch over all sets, with no host synchronisation (capturable). The
 // context's scratch must hold `total` paths.
 int launch_batch_wavefront(NanContext* ctx, const void* sets, const uint32_t* prefix, const void* batch_ctl,
                            uint32_t set_count, uint32_t total, uint32_t* set_of, uint32_t spp, uint32_t max_bounces,
